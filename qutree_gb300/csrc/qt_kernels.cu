@@ -13,6 +13,7 @@
 // processes tile b.  The planner (qt_plan.cpp) builds both once per tree.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <mutex>
 #include <type_traits>
 
@@ -27,7 +28,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kMpTile = kThreads;  // slots (up to four outputs each) per mode-product tile, as in the planner
 constexpr int kHpMaxDim = 112;  // largest bond the planner admits
-constexpr int kHpK = 16;
 constexpr int kAccRows = 64;
 constexpr int kCvtPerThread = 8;  // 2048 elements per tile, as in the planner
 
@@ -108,99 +108,125 @@ __global__ void __launch_bounds__(kThreads) k_mp(const MPTask* __restrict__ task
   mp_tile<P>(t, tl.y);
 }
 
+// One mode product passed by value (the primitive C ABI calls): one thread
+// per output, in memory order, so that the stores and, for before > 1, the
+// loads of `in` are coalesced and h is shared by the warp (before == 1: the
+// other way round).  Bound: the FP64 pipe.  A complex multiply-add holds a
+// sub-partition's FP64 unit for 256 cycles, far longer than its two operand
+// loads, so four outputs per thread (as in mp_tile) save nothing here and cost
+// parallelism: 32 x 32 x 32 along any mode ran in 38.5 us on 32 blocks.
 __global__ void __launch_bounds__(kThreads) k_mp_single(MPTask t) {
-  mp_tile<F64>(t, (int64_t)blockIdx.x * kMpTile);
+  const int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const int64_t before = t.before;
+  if (e >= before * t.a_out * t.after) return;
+  const int64_t b = e % before, r = e / before;
+  const int64_t j = r % t.a_out, c = r / t.a_out;
+  const double2* __restrict__ ip = t.in + b + before * t.a_in * c;
+  const double2* __restrict__ hp = t.h + j;
+  double2 acc = cz();
+#pragma unroll 4
+  for (int a = 0; a < t.a_in; ++a) cfma(acc, __ldg(hp + (int64_t)t.a_out * a), __ldg(ip + before * a));
+  t.out[e] = t.add ? cadd(t.out[e], acc) : acc;
 }
 
 // ---------------------------------------------------------------------------
-// Hole product (rhomat / contraction): S(i, j) = sum_k conj(A[k; i]) B[k; j]
-// with k = (b, c).  A 32 x 32 output tile per block, 2 x 2 outputs per
-// thread; A and B are staged through shared memory 16 k-rows at a time with
-// coalesced loads (along b when before > 1, along i when before == 1).
+// Hole product (rhomat / contraction) of the primitive C ABI call:
+// S(i, j) = sum_k conj(A[k; i]) B[k; j], k = (b, c).  A cluster of CTAs owns
+// one output tile of up to 16 x 16 and splits the reduction: every CTA takes
+// a contiguous range of k, its `groups` sets of ti x tj threads every
+// groups-th row of it, one output per thread.  Rows are staged through
+// shared memory 32 at a time (coalesced along b when before > 1, along the
+// columns when before == 1).  The partial sums of the groups, then those of
+// the CTAs (read through distributed shared memory) are added in a fixed
+// order: no workspace, no atomics.  Bound: the FP64 pipe, one complex
+// multiply-add per 256 cycles and sub-partition; so one output per thread
+// and as many SMs as the shape gives.  64 x 64 outputs over 3712 rows ran in
+// 4.4 ms on the four blocks of the former 32 x 32 tiles without a split.
 // ---------------------------------------------------------------------------
-template <class P>
-__device__ __forceinline__ void hp_tile(const HPTask& t, int mt0) {
-  // Output S is split into 2 x 2 micro-tiles {i, i + mi} x {j, j + mj}
-  // (mi = ceil(aA/2), mj = ceil(aB/2)), numbered column-major over the
-  // mi x mj grid; thread x of the block owns micro-tile mt0 + x.  Adjacent
-  // threads read adjacent rows of the staged operands (conflict-free shared
-  // loads).  Threads past the last micro-tile form whole idle warps (they
-  // only help stage operands), so no lanes idle inside a warp.
-  typedef typename P::S S;
-  typedef typename P::A A;
-  extern __shared__ __align__(16) unsigned char hp_smem[];
-  const S* __restrict__ Ap = reinterpret_cast<const S*>(t.A);
-  const S* __restrict__ Bp = reinterpret_cast<const S*>(t.B);
-  S* Sp = reinterpret_cast<S*>(t.S);
-  const int before = t.before;
+constexpr int kHcTile = 16;   // outputs of a tile per side
+constexpr int kHcRows = 32;   // staged rows
+constexpr int kHcMaxCl = 8;   // CTAs of a cluster (portable size)
+struct HcGeo {
+  int ti, tj, nti, groups, cl;  // tile sides, tiles along i, thread groups, CTAs per tile
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+// all threads of the cluster; orders shared-memory accesses across its CTAs
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+// element of the same shared-memory variable in CTA `rank` of the cluster
+__device__ __forceinline__ double2 ld_cluster(const double2* p, uint32_t rank) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(a), "r"(rank));
+  double2 v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(ra) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(kThreads) k_hp_single(HPTask t, HcGeo g) {
+  __shared__ double2 sA[kHcRows][kHcTile + 1], sB[kHcRows][kHcTile + 1];
+  __shared__ double2 red[kThreads], part[kThreads];
   const int aA = t.a, aB = t.aB > 0 ? t.aB : t.a;
-  S* sA = reinterpret_cast<S*>(hp_smem);   // [kHpK][aA]
-  S* sB = sA + kHpK * aA;                  // [kHpK][aB]
-  const int64_t K = (int64_t)before * t.after;
-  const int64_t sliceA = (int64_t)before * aA, sliceB = (int64_t)before * aB;
-  const int mi = (aA + 1) / 2, mj = (aB + 1) / 2;
-  const int mt = mt0 + threadIdx.x;
-  const bool active = mt < mi * mj;
-  const int i = active ? mt % mi : 0;
-  const int j = active ? mt / mi : 0;
-  const bool has_i1 = i + mi < aA, has_j1 = j + mj < aB;
-  const int i1 = has_i1 ? i + mi : i, j1 = has_j1 ? j + mj : j;
-  A acc00 = P::zero(), acc01 = P::zero(), acc10 = P::zero(), acc11 = P::zero();
-  const int nA = kHpK * aA, nAB = kHpK * (aA + aB);
-  for (int64_t k0 = 0; k0 < K; k0 += kHpK) {
-    for (int e = threadIdx.x; e < nAB; e += kThreads) {
-      const bool isA = e < nA;
-      const int ee = isA ? e : e - nA;
-      const int ncol = isA ? aA : aB;
-      int kk, ii;
-      if (before == 1) {
-        ii = ee % ncol;
-        kk = ee / ncol;
-      } else {
-        kk = ee % kHpK;
-        ii = ee / kHpK;
+  const uint32_t rank = g.cl > 1 ? cluster_rank() : 0;
+  const int tile = (int)(blockIdx.x / g.cl);
+  const int i0 = (tile % g.nti) * g.ti, j0 = (tile / g.nti) * g.tj;
+  const int mi = min(g.ti, aA - i0), mj = min(g.tj, aB - j0);
+  // at most 2^31 rows (the operands have at most 2^31 elements)
+  const uint32_t before = (uint32_t)t.before, K = before * (uint32_t)t.after;
+  const uint32_t per = (K + g.cl - 1) / g.cl;
+  const uint32_t kb = min(K, rank * per), ke = min(K, kb + per);
+  const int nout = g.ti * g.tj, grp = threadIdx.x / nout, o = threadIdx.x - grp * nout;
+  const int i = o % g.ti, j = o / g.ti;
+  const bool active = grp < g.groups;
+  double2 acc = cz();
+  for (uint32_t k0 = kb; k0 < ke; k0 += kHcRows) {
+    for (int e = threadIdx.x; e < 2 * kHcRows * kHcTile; e += kThreads) {
+      const bool isA = e < kHcRows * kHcTile;
+      const int ee = e & (kHcRows * kHcTile - 1);
+      const int kk = before == 1 ? ee / kHcTile : ee % kHcRows;
+      const int ii = before == 1 ? ee % kHcTile : ee / kHcRows;
+      const uint32_t k = k0 + kk;
+      double2 v = cz();
+      if (k < ke && ii < (isA ? mi : mj)) {
+        const uint32_t c = k / before, b = k - c * before;
+        const int64_t col = (isA ? i0 : j0) + ii;
+        v = __ldg((isA ? t.A : t.B) + b + (int64_t)before * (col + (int64_t)(isA ? aA : aB) * c));
       }
-      const int64_t k = k0 + kk;
-      S v = P::zero();
-      if (k < K) {
-        const int64_t b = k % before, c = k / before;
-        v = isA ? P::ld(Ap + b + (int64_t)before * ii + sliceA * c)
-                : P::ld(Bp + b + (int64_t)before * ii + sliceB * c);
-      }
-      (isA ? sA : sB)[kk * ncol + ii] = v;
+      (isA ? sA : sB)[kk][ii] = v;
     }
     __syncthreads();
     if (active) {
-#pragma unroll 4
-      for (int kk = 0; kk < kHpK; ++kk) {
-        const S a0 = sA[kk * aA + i], a1 = sA[kk * aA + i1];
-        const S b0 = sB[kk * aB + j], b1 = sB[kk * aB + j1];
-        P::macc(acc00, a0, b0);
-        P::macc(acc10, a1, b0);
-        P::macc(acc01, a0, b1);
-        P::macc(acc11, a1, b1);
-        if (kk & 1) {
-          P::norm(acc00);
-          P::norm(acc10);
-          P::norm(acc01);
-          P::norm(acc11);
-        }
-      }
+      const int nk = (int)min((uint32_t)kHcRows, ke - k0);
+      for (int kk = grp; kk < nk; kk += g.groups) cfmac(acc, sA[kk][i], sB[kk][j]);
     }
     __syncthreads();
   }
-  if (!active) return;
-  Sp[i + (int64_t)aA * j] = P::fin(acc00);
-  if (has_i1) Sp[i1 + (int64_t)aA * j] = P::fin(acc10);
-  if (has_j1) Sp[i + (int64_t)aA * j1] = P::fin(acc01);
-  if (has_i1 && has_j1) Sp[i1 + (int64_t)aA * j1] = P::fin(acc11);
+  if (g.groups > 1) {
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    if (grp == 0)
+      for (int q = 1; q < g.groups; ++q) acc = cadd(acc, red[q * nout + o]);
+  }
+  if (g.cl == 1) {
+    if (grp == 0 && i < mi && j < mj) t.S[(i0 + i) + (int64_t)aA * (j0 + j)] = acc;
+    return;
+  }
+  if (grp == 0) part[o] = acc;
+  cluster_sync();
+  for (int e = (int)rank + g.cl * (int)threadIdx.x; e < nout; e += g.cl * kThreads) {
+    double2 s = ld_cluster(part + e, 0);
+    for (int q = 1; q < g.cl; ++q) s = cadd(s, ld_cluster(part + e, (uint32_t)q));
+    const int ie = e % g.ti, je = e / g.ti;
+    if (ie < mi && je < mj) t.S[(i0 + ie) + (int64_t)aA * (j0 + je)] = s;
+  }
+  cluster_sync();  // no CTA leaves while its partial sums are being read
 }
-
-__global__ void __launch_bounds__(kThreads) k_hp_single(HPTask t) {
-  hp_tile<F64>(t, blockIdx.x * kThreads);
-}
-
-inline int hp_smem_bytes(int aA, int aB) { return kHpK * (aA + aB) * 16; }
 
 // ---------------------------------------------------------------------------
 // Hole products of the sweep, split over the reduction index k.  A block owns
@@ -339,27 +365,6 @@ __global__ void __launch_bounds__(kThreads, R * C > 9 ? 2 : 3)
   const int4 tl = tiles[tile0 + blockIdx.x];
   const HPTask t = tasks[tl.x];
   hp_split_tile<P, R, C>(t, tl, ws);
-}
-
-// one task passed by value: block b covers output tile b % ntiles, range b / ntiles
-template <class P, int R, int C>
-__global__ void __launch_bounds__(kThreads, R * C > 9 ? 2 : 3)
-    k_hp_one(HPTask t, int ntiles, typename P::S* __restrict__ ws) {
-  hp_split_tile<P, R, C>(t, make_int4(0, (int)(blockIdx.x % ntiles), (int)(blockIdx.x / ntiles), 0), ws);
-}
-
-template <class P>
-__global__ void __launch_bounds__(kThreads) k_hp_sum_one(HPTask t, const typename P::S* __restrict__ ws) {
-  typedef typename P::S S;
-  typedef typename P::A A;
-  const int aB = t.aB > 0 ? t.aB : t.a;
-  const int64_t n = (int64_t)t.a * aB;
-  S* Sp = reinterpret_cast<S*>(t.S);
-  for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kThreads) {
-    A acc = P::zero();
-    for (int z = 0; z < t.splits; ++z) P::add(acc, ws[t.ws + z * n + e]);
-    Sp[e] = P::fin(acc);
-  }
 }
 
 // S = sum over the k ranges of the partial tiles, in range order; kHpSumChunks
@@ -1099,33 +1104,6 @@ cudaError_t launch_dot(const double2* a, const double2* b, int64_t n, double2* o
   return cudaGetLastError();
 }
 
-cudaError_t launch_hp_one_shape(const HPTask& t, int ntiles, double2* ws, cudaStream_t s);
-
-cudaError_t launch_hp_split(const HPTask& task, double2* ws, int64_t ws_elems, cudaStream_t s) {
-  HPTask t = task;
-  const int aB = t.aB > 0 ? t.aB : t.a;
-  if (t.a > kHpMaxDim || aB > kHpMaxDim || t.a < 1 || aB < 1) return cudaErrorInvalidValue;
-  hp_shape(std::min(std::max(t.a, aB), kHpTile), &t.rows, &t.cols);
-  const int ntiles = ((t.a + kHpTile - 1) / kHpTile) * ((aB + kHpTile - 1) / kHpTile);
-  const int64_t K = (int64_t)t.before * t.after;
-  int64_t kc = std::max<int64_t>(256, (K * ntiles + 4 * 152 - 1) / (4 * 152));
-  kc = (kc + kHpRows - 1) / kHpRows * kHpRows;
-  int64_t splits = (K + kc - 1) / kc;
-  const int64_t per = (int64_t)t.a * aB;
-  if (splits > 1 && splits * per > ws_elems) {  // fewer, longer ranges to fit the workspace
-    splits = std::max<int64_t>(1, ws_elems / per);
-    kc = (K + splits - 1) / splits;
-    splits = (K + kc - 1) / kc;
-  }
-  t.splits = (int)splits;
-  t.kchunk = (int)std::min<int64_t>(K, kc);
-  t.ws = 0;
-  cudaError_t e = launch_hp_one_shape(t, ntiles, ws, s);
-  if (e != cudaSuccess) return e;
-  if (t.splits > 1) k_hp_sum_one<F64><<<(unsigned)std::min<int64_t>(64, (per + kThreads - 1) / kThreads), kThreads, 0, s>>>(t, ws);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_lincomb(double2* out, const LinComb& lc, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (lc.count < 0 || lc.count > kLinCombMax) return cudaErrorInvalidValue;
@@ -1231,30 +1209,6 @@ cudaError_t launch_hp_shape(int rows, int cols, const HPTask* tasks, const int4*
     default: return cudaErrorInvalidValue;
   }
 }
-
-template <int R, int C>
-cudaError_t launch_hp_one_rc(const HPTask& t, int ntiles, double2* ws, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_hp_one<F64, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHpSmem);
-  if (e != cudaSuccess) return e;
-  k_hp_one<F64, R, C><<<(unsigned)((int64_t)ntiles * t.splits), kThreads, kHpSmem, s>>>(t, ntiles, ws);
-  return cudaSuccess;
-}
-
-cudaError_t launch_hp_one_shape(const HPTask& t, int ntiles, double2* ws, cudaStream_t s) {
-  switch (t.rows * 8 + t.cols) {
-    case 1 * 8 + 1: return launch_hp_one_rc<1, 1>(t, ntiles, ws, s);
-    case 1 * 8 + 2: return launch_hp_one_rc<1, 2>(t, ntiles, ws, s);
-    case 1 * 8 + 3: return launch_hp_one_rc<1, 3>(t, ntiles, ws, s);
-    case 1 * 8 + 4: return launch_hp_one_rc<1, 4>(t, ntiles, ws, s);
-    case 2 * 8 + 3: return launch_hp_one_rc<2, 3>(t, ntiles, ws, s);
-    case 2 * 8 + 4: return launch_hp_one_rc<2, 4>(t, ntiles, ws, s);
-    case 3 * 8 + 3: return launch_hp_one_rc<3, 3>(t, ntiles, ws, s);
-    case 3 * 8 + 4: return launch_hp_one_rc<3, 4>(t, ntiles, ws, s);
-    case 4 * 8 + 4: return launch_hp_one_rc<4, 4>(t, ntiles, ws, s);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
 
 // ---------------------------------------------------------------------------
 // CDVR kernels (complex128)
@@ -1677,24 +1631,37 @@ cudaError_t launch_set_identity(double2* m, int d, int prec, cudaStream_t s) {
 }
 
 cudaError_t launch_single_mp(const MPTask& task, cudaStream_t s, void*) {
-  const int64_t slots = (int64_t)task.before * ((task.a_out + 3) / 4) * task.after;
-  const int64_t blocks = (slots + kMpTile - 1) / kMpTile;
+  const int64_t n = (int64_t)task.before * task.a_out * task.after;
+  const int64_t blocks = (n + kThreads - 1) / kThreads;
   if (blocks == 0) return cudaSuccess;
   k_mp_single<<<(unsigned)blocks, kThreads, 0, s>>>(task);
   return cudaGetLastError();
 }
 
 cudaError_t launch_single_hp(const HPTask& task, cudaStream_t s, void*) {
-  const int aB = task.aB > 0 ? task.aB : task.a;
-  const int64_t micro = (int64_t)((task.a + 1) / 2) * ((aB + 1) / 2);
-  const int64_t blocks = (micro + kThreads - 1) / kThreads;
-  if (blocks == 0) return cudaSuccess;
-  const int sm = hp_smem_bytes(task.a, aB);
-  if (sm > 200 * 1024) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_hp_single, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  if (e != cudaSuccess) return e;
-  k_hp_single<<<(unsigned)blocks, kThreads, sm, s>>>(task);
-  return cudaGetLastError();
+  const int aA = task.a, aB = task.aB > 0 ? task.aB : task.a;
+  if (aA < 1 || aB < 1) return cudaSuccess;
+  HcGeo g;
+  g.nti = (aA + kHcTile - 1) / kHcTile;
+  const int ntj = (aB + kHcTile - 1) / kHcTile;
+  g.ti = (aA + g.nti - 1) / g.nti;  // tiles of equal sides
+  g.tj = (aB + ntj - 1) / ntj;
+  g.groups = std::min(kThreads / (g.ti * g.tj), kHcRows);
+  const int64_t tiles = (int64_t)g.nti * ntj, K = (int64_t)task.before * task.after;
+  // more CTAs per tile while they find SMs (152) and at least 16 rows each
+  g.cl = 1;
+  while (g.cl < kHcMaxCl && tiles * g.cl < 152 && K >= 32 * g.cl) g.cl *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * g.cl));
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)g.cl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_hp_single, task, g);
 }
 
 // ---------------------------------------------------------------------------
