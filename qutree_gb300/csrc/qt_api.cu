@@ -1677,8 +1677,9 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
     for (int x : g.shape) maxd = std::max(maxd, x);
   }
   const int64_t vstride = (maxN + 15) / 16 * 16, mstride = (int64_t)maxd * maxd;
-  // vectors V_0..V_{K-1}, W, Y, T, U; matrices S, H, R; dot scratch
-  const int64_t total = (n_krylov + 4) * vstride + 3 * mstride + 512;
+  // vectors V_0..V_{K-1}, W, Y, T, U; matrices S, H, R; dot scratch; hole-product partial tiles
+  const int64_t ws_elems = 64 * mstride;
+  const int64_t total = (n_krylov + 4) * vstride + 3 * mstride + 512 + ws_elems;
   DevFree work;
   {
     cudaError_t e = dev_malloc(&work.p, total * sizeof(cd));
@@ -1694,6 +1695,7 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
   cd* dH = dS + mstride;
   cd* dR = dH + mstride;
   cd* dscal = dR + mstride;
+  cd* hpws = dscal + 512;
   // the driver works on the complex128 wavefunction; with double-float
   // arithmetic the plan's stages read B_PSI, refreshed node by node
   const bool df = c->prec >= 1;
@@ -1742,7 +1744,9 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
     t.kchunk = 0;
     t.ws = 0;
     t.rows = t.cols = 4;
-    cudaError_t e = qt::launch_single_hp(t, c->stream, nullptr);
+    // the split by fixed ranges of the reduction, whose order of additions the
+    // Krylov sweep's results are sensitive to
+    cudaError_t e = qt::launch_hp_split(t, hpws, ws_elems, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "qt_scf hole product");
     c->launches += 1;
     return QT_OK;

@@ -687,6 +687,9 @@ inline void hp_shape(int m, int* rows, int* cols) {
       }
     }
 }
+// One complex128 hole product split over its reduction index (partial tiles
+// in ws, at most ws_elems elements); S written in full.
+cudaError_t launch_hp_split(const HPTask& task, double2* ws, int64_t ws_elems, cudaStream_t s);
 // SCF Krylov helpers (complex128): out[0] = sum conj(a) b (out needs 257
 // elements of workspace); out = sum_t c_t v_t
 constexpr int kLinCombMax = 32;

@@ -367,6 +367,27 @@ __global__ void __launch_bounds__(kThreads, R * C > 9 ? 2 : 3)
   hp_split_tile<P, R, C>(t, tl, ws);
 }
 
+// one task passed by value: block b covers output tile b % ntiles, range b / ntiles
+template <class P, int R, int C>
+__global__ void __launch_bounds__(kThreads, R * C > 9 ? 2 : 3)
+    k_hp_one(HPTask t, int ntiles, typename P::S* __restrict__ ws) {
+  hp_split_tile<P, R, C>(t, make_int4(0, (int)(blockIdx.x % ntiles), (int)(blockIdx.x / ntiles), 0), ws);
+}
+
+template <class P>
+__global__ void __launch_bounds__(kThreads) k_hp_sum_one(HPTask t, const typename P::S* __restrict__ ws) {
+  typedef typename P::S S;
+  typedef typename P::A A;
+  const int aB = t.aB > 0 ? t.aB : t.a;
+  const int64_t n = (int64_t)t.a * aB;
+  S* Sp = reinterpret_cast<S*>(t.S);
+  for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kThreads) {
+    A acc = P::zero();
+    for (int z = 0; z < t.splits; ++z) P::add(acc, ws[t.ws + z * n + e]);
+    Sp[e] = P::fin(acc);
+  }
+}
+
 // S = sum over the k ranges of the partial tiles, in range order; kHpSumChunks
 // blocks of 256 outputs per task (the loads of four ranges in flight)
 constexpr int kHpSumChunks = 16;
@@ -1104,6 +1125,33 @@ cudaError_t launch_dot(const double2* a, const double2* b, int64_t n, double2* o
   return cudaGetLastError();
 }
 
+cudaError_t launch_hp_one_shape(const HPTask& t, int ntiles, double2* ws, cudaStream_t s);
+
+cudaError_t launch_hp_split(const HPTask& task, double2* ws, int64_t ws_elems, cudaStream_t s) {
+  HPTask t = task;
+  const int aB = t.aB > 0 ? t.aB : t.a;
+  if (t.a > kHpMaxDim || aB > kHpMaxDim || t.a < 1 || aB < 1) return cudaErrorInvalidValue;
+  hp_shape(std::min(std::max(t.a, aB), kHpTile), &t.rows, &t.cols);
+  const int ntiles = ((t.a + kHpTile - 1) / kHpTile) * ((aB + kHpTile - 1) / kHpTile);
+  const int64_t K = (int64_t)t.before * t.after;
+  int64_t kc = std::max<int64_t>(256, (K * ntiles + 4 * 152 - 1) / (4 * 152));
+  kc = (kc + kHpRows - 1) / kHpRows * kHpRows;
+  int64_t splits = (K + kc - 1) / kc;
+  const int64_t per = (int64_t)t.a * aB;
+  if (splits > 1 && splits * per > ws_elems) {  // fewer, longer ranges to fit the workspace
+    splits = std::max<int64_t>(1, ws_elems / per);
+    kc = (K + splits - 1) / splits;
+    splits = (K + kc - 1) / kc;
+  }
+  t.splits = (int)splits;
+  t.kchunk = (int)std::min<int64_t>(K, kc);
+  t.ws = 0;
+  cudaError_t e = launch_hp_one_shape(t, ntiles, ws, s);
+  if (e != cudaSuccess) return e;
+  if (t.splits > 1) k_hp_sum_one<F64><<<(unsigned)std::min<int64_t>(64, (per + kThreads - 1) / kThreads), kThreads, 0, s>>>(t, ws);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_lincomb(double2* out, const LinComb& lc, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (lc.count < 0 || lc.count > kLinCombMax) return cudaErrorInvalidValue;
@@ -1209,6 +1257,30 @@ cudaError_t launch_hp_shape(int rows, int cols, const HPTask* tasks, const int4*
     default: return cudaErrorInvalidValue;
   }
 }
+
+template <int R, int C>
+cudaError_t launch_hp_one_rc(const HPTask& t, int ntiles, double2* ws, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(k_hp_one<F64, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHpSmem);
+  if (e != cudaSuccess) return e;
+  k_hp_one<F64, R, C><<<(unsigned)((int64_t)ntiles * t.splits), kThreads, kHpSmem, s>>>(t, ntiles, ws);
+  return cudaSuccess;
+}
+
+cudaError_t launch_hp_one_shape(const HPTask& t, int ntiles, double2* ws, cudaStream_t s) {
+  switch (t.rows * 8 + t.cols) {
+    case 1 * 8 + 1: return launch_hp_one_rc<1, 1>(t, ntiles, ws, s);
+    case 1 * 8 + 2: return launch_hp_one_rc<1, 2>(t, ntiles, ws, s);
+    case 1 * 8 + 3: return launch_hp_one_rc<1, 3>(t, ntiles, ws, s);
+    case 1 * 8 + 4: return launch_hp_one_rc<1, 4>(t, ntiles, ws, s);
+    case 2 * 8 + 3: return launch_hp_one_rc<2, 3>(t, ntiles, ws, s);
+    case 2 * 8 + 4: return launch_hp_one_rc<2, 4>(t, ntiles, ws, s);
+    case 3 * 8 + 3: return launch_hp_one_rc<3, 3>(t, ntiles, ws, s);
+    case 3 * 8 + 4: return launch_hp_one_rc<3, 4>(t, ntiles, ws, s);
+    case 4 * 8 + 4: return launch_hp_one_rc<4, 4>(t, ntiles, ws, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 
 // ---------------------------------------------------------------------------
 // CDVR kernels (complex128)
