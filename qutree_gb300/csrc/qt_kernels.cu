@@ -38,61 +38,90 @@ __device__ __forceinline__ void cfmac(double2& acc, double2 a, double2 b) { cfma
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return cadd64(a, b); }
 
 // ---------------------------------------------------------------------------
-// Mode-k product (matvec / matrixTensor): one thread per slot (b, j0..j0+3, c)
-// of up to four outputs that share the input fiber in[b, :, c]: per a one
-// input load and four h loads feed four products.  Slots run b fastest:
+// Mode-k product (matvec / matrixTensor).  A slot is (b, j0..j0+3, c): up to
+// four outputs that share the input fiber in[b, :, c].  A thread takes NJ of
+// a slot's outputs (block (tile, part): outputs j0 + NJ part ..): with NJ = 4
+// one input load and four h loads feed four products per a; with NJ = 1 four
+// times as many warps run a chain a quarter as long.  Slots run b fastest:
 // along higher modes consecutive threads read consecutive input elements
 // (coalesced) and share h; along mode 0 (before = 1) they read consecutive
-// groups of h's rows and share the input fiber.
+// groups of h's rows and share the input fiber.  Every output is summed in
+// the same order whatever NJ is.
 // ---------------------------------------------------------------------------
-template <class P>
-__device__ __forceinline__ void mp_tile(const MPTask& t, int64_t slot0) {
+template <class P, int NJ>
+__global__ void __launch_bounds__(kThreads) k_mp(const MPTask* __restrict__ tasks,
+                                                 const int2* __restrict__ tiles, int64_t tile0) {
   typedef typename P::S S;
   typedef typename P::A A;
+  constexpr int U = 4 / NJ;  // steps of a whose loads are in flight together
+  const int2 tl = tiles[tile0 + blockIdx.x];
+  const MPTask t = tasks[tl.x];
   const S* __restrict__ in = reinterpret_cast<const S*>(t.in);
   const S* __restrict__ h = reinterpret_cast<const S*>(t.h);
   S* out = reinterpret_cast<S*>(t.out);
   const int nq = (t.a_out + 3) / 4;
   const int64_t before = t.before;
-  const int64_t slot = slot0 + threadIdx.x;
+  const int64_t slot = (int64_t)tl.y + threadIdx.x;
   if (slot >= before * nq * t.after) return;
   const int64_t b = slot % before;
   const int64_t r = slot / before;
-  const int j0 = 4 * (int)(r % nq);
+  const int j0 = 4 * (int)(r % nq) + NJ * (int)blockIdx.y;
   const int64_t c = r / nq;
-  const int nj = t.a_out - j0 < 4 ? t.a_out - j0 : 4;
+  const int nj = t.a_out - j0 < NJ ? t.a_out - j0 : NJ;
+  if (nj <= 0) return;
   const S* ip = in + b + before * t.a_in * c;  // in[b, a, c] = ip[before a]
   const bool unit = t.alpha.x == 1.0 && t.alpha.y == 0.0;
   const typename P::C alpha = P::coef(t.alpha);
-  S res[4];
+  S res[NJ];
   if (t.diag) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < NJ; ++q) {
       const int j = j0 + (q < nj ? q : 0);
       res[q] = P::mul(P::ld(h + j), P::ld(ip + before * j));
     }
   } else {
-    A acc[4] = {P::zero(), P::zero(), P::zero(), P::zero()};
+    A acc[NJ];
+#pragma unroll
+    for (int q = 0; q < NJ; ++q) acc[q] = P::zero();
     const S* hp = h + j0;  // h(j, a) = h[j + a_out a]
     const int64_t hs = t.a_out;
-    for (int a = 0; a < t.a_in; ++a) {
-      const S x = P::ld(ip);
-      S h0[4];
+    int a = 0;
+    for (; a + U <= t.a_in; a += U) {
+      S x[U], h0[U][NJ];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) h0[q] = P::ld(hp + (q < nj ? q : 0));
+      for (int u = 0; u < U; ++u) {
+        x[u] = P::ld(ip + before * u);
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) h0[u][q] = P::ld(hp + hs * u + (q < nj ? q : 0));
+      }
+      ip += before * U;
+      hp += hs * U;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) {
+          P::mac(acc[q], h0[u][q], x[u]);
+          if ((a + u) & 1) P::norm(acc[q]);
+        }
+    }
+    for (; a < t.a_in; ++a) {
+      const S x = P::ld(ip);
+      S h0[NJ];
+#pragma unroll
+      for (int q = 0; q < NJ; ++q) h0[q] = P::ld(hp + (q < nj ? q : 0));
       ip += before;
       hp += hs;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < NJ; ++q) {
         P::mac(acc[q], h0[q], x);
         if (a & 1) P::norm(acc[q]);
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) res[q] = P::fin(acc[q]);
+    for (int q = 0; q < NJ; ++q) res[q] = P::fin(acc[q]);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < NJ; ++q)
     if (q < nj) {
       const int64_t o = b + before * ((j0 + q) + (int64_t)t.a_out * c);
       const S v = unit ? res[q] : P::scale(alpha, res[q]);
@@ -100,20 +129,12 @@ __device__ __forceinline__ void mp_tile(const MPTask& t, int64_t slot0) {
     }
 }
 
-template <class P>
-__global__ void __launch_bounds__(kThreads) k_mp(const MPTask* __restrict__ tasks,
-                                                 const int2* __restrict__ tiles, int64_t tile0) {
-  const int2 tl = tiles[tile0 + blockIdx.x];
-  const MPTask t = tasks[tl.x];
-  mp_tile<P>(t, tl.y);
-}
-
 // One mode product passed by value (the primitive C ABI calls): one thread
 // per output, in memory order, so that the stores and, for before > 1, the
 // loads of `in` are coalesced and h is shared by the warp (before == 1: the
 // other way round).  Bound: the FP64 pipe.  A complex multiply-add holds a
 // sub-partition's FP64 unit for 256 cycles, far longer than its two operand
-// loads, so four outputs per thread (as in mp_tile) save nothing here and cost
+// loads, so four outputs per thread (as in k_mp) save nothing here and cost
 // parallelism: 32 x 32 x 32 along any mode ran in 38.5 us on 32 blocks.
 __global__ void __launch_bounds__(kThreads) k_mp_single(MPTask t) {
   const int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -475,6 +496,90 @@ __global__ void __launch_bounds__(kThreads) k_acc(const AccTask* __restrict__ ta
   S* out = reinterpret_cast<S*>(t.out);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
+    const int j = jb + q;
+    if (rv && j < d) {
+      const S v = P::scale(alpha, P::fin(acc[q]));
+      S* p = out + r + rows * j;
+      *p = t.add ? P::plus(*p, v) : v;
+    }
+  }
+}
+
+// The same with NQ = 1 or 2 of a thread's four columns (block (tile, part)),
+// for stages that would leave SMs idle.  A thread sums all terms of a node,
+// a chain of count x d steps: with one column a step is a quarter as long,
+// four times as many warps run, and the loads of four steps are in flight
+// together.  Every output is summed in the order of k_acc.
+template <class P, int NQ>
+__global__ void __launch_bounds__(kThreads) k_acc_few(const AccTask* __restrict__ tasks,
+                                                      const AccTerm* __restrict__ terms,
+                                                      const int4* __restrict__ tiles, int64_t tile0) {
+  typedef typename P::S S;
+  typedef typename P::A A;
+  constexpr int U = 4 / NQ;  // steps whose loads are in flight together
+  const int4 tl = tiles[tile0 + blockIdx.x];
+  const AccTask t = tasks[tl.x];
+  const int r = tl.y + threadIdx.x % kAccRows;
+  const int jb = tl.z + (threadIdx.x / kAccRows) * 4 + NQ * (int)blockIdx.y;
+  const bool rv = r < t.rows;
+  const int d = t.d;
+  if (jb >= d) return;  // the whole warp lies past the last column
+  const int nq = d - jb < NQ ? d - jb : NQ;  // uniform across the warp
+  const int64_t rows = t.rows;
+  A acc[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) acc[q] = P::zero();
+  for (int s = 0; s < t.count; ++s) {
+    const AccTerm T = terms[t.first + s];
+    const S* X = reinterpret_cast<const S*>(T.X) + r;
+    const S* H = reinterpret_cast<const S*>(T.H);
+    if (H == nullptr) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int j = jb + q;
+        if (rv && j < d) P::add(acc[q], P::ld(X + rows * j));
+      }
+      continue;
+    }
+    const S* hrow[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) hrow[q] = H + (q < nq ? jb + q : 0);
+    int jp = 0;
+    for (; jp + U <= d; jp += U) {
+      S x[U], hv[U][NQ];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        x[u] = rv ? P::ld(X + rows * (jp + u)) : P::zero();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) hv[u][q] = P::ld(hrow[q] + (int64_t)d * (jp + u));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+          if (q < nq) P::mac(acc[q], hv[u][q], x[u]);
+        if ((jp + u) & 1) {
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) P::norm(acc[q]);
+        }
+      }
+    }
+    for (; jp < d; ++jp) {
+      const S x = rv ? P::ld(X + rows * jp) : P::zero();
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (q < nq) P::mac(acc[q], P::ld(hrow[q] + (int64_t)d * jp), x);
+      if (jp & 1) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) P::norm(acc[q]);
+      }
+    }
+  }
+  const double2 alpha64 = t.alpha_ptr ? *t.alpha_ptr : t.alpha;
+  const typename P::C alpha = P::coef(alpha64);
+  S* out = reinterpret_cast<S*>(t.out);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
     const int j = jb + q;
     if (rv && j < d) {
       const S v = P::scale(alpha, P::fin(acc[q]));
@@ -1586,12 +1691,28 @@ __global__ void __launch_bounds__(kThreads) k_ew(const EWTask* __restrict__ task
   }
 }
 
+// outputs per thread of a mode-product or accumulation stage of `tiles` tiles:
+// one (four blocks per tile) while four per thread would leave SMs with fewer
+// than two blocks, two up to twice that.  Stages of an 8-mode complex128
+// sweep: mode products 151 -> 115 us, accumulations 110 -> 57; of a 12-mode
+// double-float one (bonds 13..19): 282 -> 207 and 195 -> 133.  Beyond, one
+// output per thread costs loads: the mode products of 64 uneven trees 2.93 -> 3.81 ms,
+// accumulations at bonds 58..96 34 -> 45 ms.
+inline int outputs_per_thread(int64_t tiles) { return tiles <= 2 * 152 ? 1 : tiles <= 4 * 152 ? 2 : 4; }
+
 template <class P>
 cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int max_eig_d,
                            cudaStream_t s) {
   switch (st.kind) {
     case ST_MP:
-      if (st.n_tiles > 0) k_mp<P><<<(unsigned)st.n_tiles, kThreads, 0, s>>>(t.mp, t.mp_tiles, st.first_tile);
+      if (st.n_tiles > 0) {
+        const unsigned n = (unsigned)st.n_tiles;
+        switch (outputs_per_thread(st.n_tiles)) {
+          case 1: k_mp<P, 1><<<dim3(n, 4), kThreads, 0, s>>>(t.mp, t.mp_tiles, st.first_tile); break;
+          case 2: k_mp<P, 2><<<dim3(n, 2), kThreads, 0, s>>>(t.mp, t.mp_tiles, st.first_tile); break;
+          default: k_mp<P, 4><<<n, kThreads, 0, s>>>(t.mp, t.mp_tiles, st.first_tile);
+        }
+      }
       if (st.noz > 0) {
         cudaError_t e = launch_mp_tc(std::is_same<P, DF64>::value, t.mp, t.mp_oz_tiles, st.oz0, st.noz,
                                      t.mp_oz_tasks, st.ozt0, st.nozt, t.status, s);
@@ -1617,8 +1738,14 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       break;
     }
     case ST_ACC:
-      if (st.n_tiles > 0)
-        k_acc<P><<<(unsigned)st.n_tiles, kThreads, 0, s>>>(t.acc, t.acc_terms, t.acc_tiles, st.first_tile);
+      if (st.n_tiles > 0) {
+        const unsigned n = (unsigned)st.n_tiles;
+        switch (outputs_per_thread(st.n_tiles)) {
+          case 1: k_acc_few<P, 1><<<dim3(n, 4), kThreads, 0, s>>>(t.acc, t.acc_terms, t.acc_tiles, st.first_tile); break;
+          case 2: k_acc_few<P, 2><<<dim3(n, 2), kThreads, 0, s>>>(t.acc, t.acc_terms, t.acc_tiles, st.first_tile); break;
+          default: k_acc<P><<<n, kThreads, 0, s>>>(t.acc, t.acc_terms, t.acc_tiles, st.first_tile);
+        }
+      }
       if (st.nati > 0) {
         if (!std::is_same<P, DF64>::value) return cudaErrorInvalidValue;  // the planner emits none
         cudaError_t e = launch_acc_tc(t.acc, t.acc_terms, t.acc_tc_items, st.ati0, st.nati, st.atc_units,
