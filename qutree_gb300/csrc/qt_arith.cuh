@@ -66,6 +66,13 @@ struct F64 {
     const double den = x.x * x.x + x.y * x.y;
     return make_double2(x.x / den, -x.y / den);
   }
+  // real scalars of the Hermitian inversion: Re x > 0, 1 / Re x, conj(x) r, real diagonal
+  typedef double R;
+  static __device__ __forceinline__ bool positive(const S& x) { return x.x > 0.0; }
+  static __device__ __forceinline__ R rrecip(const S& x) { return 1.0 / x.x; }
+  static __device__ __forceinline__ S conj_scale(const S& x, R r) { return make_double2(x.x * r, -x.y * r); }
+  static __device__ __forceinline__ S real(R r) { return make_double2(r, 0.0); }
+  static __device__ __forceinline__ S conj(const S& x) { return make_double2(x.x, -x.y); }
 };
 
 // ---- double-float helpers --------------------------------------------------
@@ -172,6 +179,27 @@ struct DF64 {
     const float2 r = df_split(re / den), i = df_split(-im / den);
     return make_float4(r.x, r.y, i.x, i.y);
   }
+  typedef float2 R;
+  static __device__ __forceinline__ bool positive(const S& x) { return x.x > 0.f; }
+  // 1 / (hi + lo) on the FP32 pipe: r0 = fl(1 / hi), e = 1 - (hi + lo) r0
+  // (about 2^-24, its own rounding 2^-48), r = r0 + r0 (e + e^2)
+  static __device__ __forceinline__ R rrecip(const S& x) {
+    const float r0 = __frcp_rn(x.x);
+    float e = __fmaf_rn(-x.x, r0, 1.f);
+    e = __fmaf_rn(-x.y, r0, e);
+    const float c = __fmul_rn(r0, __fmaf_rn(e, e, e));
+    R r;
+    df_quick_two_sum(r0, c, r.x, r.y);
+    return r;
+  }
+  static __device__ __forceinline__ S conj_scale(const S& x, R r) {
+    S v = zero();
+    df_mac(v.x, v.y, x.x, x.y, r.x, r.y);
+    df_mac(v.z, v.w, -x.z, -x.w, r.x, r.y);
+    return fin(v);
+  }
+  static __device__ __forceinline__ S real(R r) { return make_float4(r.x, r.y, 0.f, 0.f); }
+  static __device__ __forceinline__ S conj(const S& x) { return make_float4(x.x, x.y, -x.z, -x.w); }
 };
 
 // ---- complex64 arithmetic ---------------------------------------------------
@@ -223,6 +251,14 @@ struct C32 {
     const double den = re * re + im * im;
     return make_float4((float)(re / den), 0.f, (float)(-im / den), 0.f);
   }
+  typedef float R;
+  static __device__ __forceinline__ bool positive(const S& x) { return x.x > 0.f; }
+  static __device__ __forceinline__ R rrecip(const S& x) { return __frcp_rn(x.x); }
+  static __device__ __forceinline__ S conj_scale(const S& x, R r) {
+    return make_float4(__fmul_rn(x.x, r), 0.f, __fmul_rn(-x.z, r), 0.f);
+  }
+  static __device__ __forceinline__ S real(R r) { return make_float4(r, 0.f, 0.f, 0.f); }
+  static __device__ __forceinline__ S conj(const S& x) { return make_float4(x.x, 0.f, -x.z, 0.f); }
 };
 
 }  // namespace qt

@@ -708,6 +708,64 @@ __global__ void __launch_bounds__(kThreads) k_cvt(const CvtTask* __restrict__ ta
 }
 
 // ---------------------------------------------------------------------------
+// Inverse of a Hermitian positive definite d x d matrix by the symmetric sweep
+// operator, in place: A (shared memory, column-major, lower triangle) becomes
+// -A^-1 (lower triangle).  Step k takes column c of the current matrix and
+// p = 1 / c_k: A_ij -= c_i conj(c_j) p, A_ik = c_i p, A_kk = -p.  The pivots
+// are those of the Cholesky factorisation; the first that is not positive
+// ends the sweep (false, uniform over the block, A void).  d^3 / 2 complex
+// multiply-adds (Gauss-Jordan on [A | I] without the symmetry: 2 d^3) and one
+// barrier per step: the threads that update column k + 1 also write it to
+// the other column buffer.  256 threads as 16 x 16 (i, j); c: 2 d elements.
+// Bound: FP64 issue for d >= 32 (complex128), the barrier and the pivot's
+// reciprocal below.
+// ---------------------------------------------------------------------------
+template <class P>
+__device__ bool herm_sweep_inverse(typename P::S* A, int d, typename P::S* c) {
+  typedef typename P::S S;
+  __shared__ typename P::R pr[2];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  for (int i = threadIdx.x; i < d; i += kThreads) c[i] = A[i];
+  if (threadIdx.x == 0) pr[0] = P::rrecip(A[0]);
+  for (int k = 0; k < d; ++k) {
+    __syncthreads();
+    const S* cur = c + (k & 1) * d;
+    S* nxt = c + ((k + 1) & 1) * d;
+    if (!P::positive(cur[k])) return false;
+    const typename P::R p = pr[k & 1];
+    if (k + 1 < d && tx == ((k + 1) & 15) && ty == tx) {
+      // the owner of the next pivot first: its reciprocal runs under the others' updates
+      typename P::A a = A[k + 1 + d * (k + 1)];
+      P::mac(a, cur[k + 1], P::neg(P::conj_scale(cur[k + 1], p)));
+      pr[(k + 1) & 1] = P::rrecip(P::fin(a));
+    }
+    for (int j = ty; j < d; j += 16) {
+      const S cj = cur[j];
+      const S w = P::conj_scale(cj, p);
+      const S nw = P::neg(w);
+      const int i0 = j - ((j - tx) & 15);  // the thread's rows i >= j: first multiple step at or above j
+      for (int i = i0 < j ? i0 + 16 : i0; i < d; i += 16) {
+        S v;
+        if (j == k) {
+          v = i == k ? P::neg(P::real(p)) : P::conj(P::conj_scale(cur[i], p));
+        } else if (i == k) {
+          v = w;
+        } else {
+          typename P::A a = A[i + d * j];
+          P::mac(a, cur[i], nw);
+          v = P::fin(a);
+        }
+        A[i + d * j] = v;
+        if (j == k + 1) nxt[i] = v;
+        else if (i == k + 1) nxt[j] = P::conj(v);
+      }
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // Regularised inverse of a Hermitian matrix (SpectralDecompositionTree::
 // calculate + invert): parallel cyclic Jacobi with a round-robin pairing
 // (every round rotates d/2 disjoint index pairs at once), then
@@ -859,17 +917,52 @@ __device__ __forceinline__ void eig_body(const EigTask& t, double eps) {
   int* pq = (int*)(fw + m);               // 2*np
   __shared__ double red_off[kThreads], red_diag[kThreads];
   double2* U = t.U;
-  for (int e = threadIdx.x; e < d * d; e += kThreads) {
-    const int i = e % d, j = e / d;
-    const double2 aij = t.rho[i + (int64_t)d * j], aji = t.rho[j + (int64_t)d * i];
-    // Hermitian part
-    A[e] = (i == j) ? make_double2(aij.x, 0.0)
-                    : make_double2(0.5 * (aij.x + aji.x), 0.5 * (aij.y - aji.y));
-    // shifted copy for the positive-definiteness certificate below
-    U[e] = (i == j) ? make_double2(A[e].x - 100.0 * eps, 0.0) : A[e];
+  auto load = [&](double2* dst) {  // the Hermitian part
+    for (int e = threadIdx.x; e < d * d; e += kThreads) {
+      const int i = e % d, j = e / d;
+      const double2 aij = t.rho[i + (int64_t)d * j], aji = t.rho[j + (int64_t)d * i];
+      dst[e] = (i == j) ? make_double2(aij.x, 0.0)
+                        : make_double2(0.5 * (aij.x + aji.x), 0.5 * (aij.y - aji.y));
+    }
+    __syncthreads();
+  };
+  load(A);
+  // First path.  The smallest eigenvalue is at least 1 / |rho^-1|_F; if that
+  // exceeds 40 eps, eps*exp(-w/eps) changes 1/w by less than 2e-19 relative and
+  // the regularised inverse is the plain inverse.
+  __shared__ double2 col_s[2 * kHpMaxDim];
+  if (herm_sweep_inverse<F64>(A, d, col_s)) {
+    double n2 = 0.0;
+    for (int e = threadIdx.x; e < d * d; e += kThreads) {
+      const int i = e % d, j = e / d;
+      if (i < j) continue;
+      const double2 x = A[e];
+      n2 += (i == j ? 1.0 : 2.0) * (x.x * x.x + x.y * x.y);
+    }
+    red_off[threadIdx.x] = n2;
+    __syncthreads();
+    for (int s = kThreads / 2; s > 0; s >>= 1) {
+      if (threadIdx.x < s) red_off[threadIdx.x] += red_off[threadIdx.x + s];
+      __syncthreads();
+    }
+    const double lim = 1.0 / (40.0 * eps);
+    if (red_off[0] <= lim * lim) {
+      for (int e = threadIdx.x; e < d * d; e += kThreads) {
+        const int i = e % d, j = e / d;
+        const double2 x = i >= j ? A[e] : A[j + d * i];
+        t.rhoinv[e] = i == j ? make_double2(-x.x, 0.0) : make_double2(-x.x, i > j ? -x.y : x.y);
+      }
+      return;
+    }
   }
   __syncthreads();
-  // Fast path.  If every eigenvalue exceeds 50*eps, eps*exp(-w/eps) changes
+  load(A);
+  for (int e = threadIdx.x; e < d * d; e += kThreads) {
+    // shifted copy for the positive-definiteness certificate below
+    U[e] = (e % d == e / d) ? make_double2(A[e].x - 100.0 * eps, 0.0) : A[e];
+  }
+  __syncthreads();
+  // Second path.  If every eigenvalue exceeds 50*eps, eps*exp(-w/eps) changes
   // 1/w by less than 4e-24 relative, so the regularised inverse is the plain
   // inverse.  A Cholesky factorisation of rho - 100*eps*I that succeeds
   // certifies that bound (its backward error, ~d*2^-53*|rho|, is far below
@@ -968,29 +1061,27 @@ __global__ void __launch_bounds__(kThreads) k_eig(const EigTask* __restrict__ ta
 }
 
 // ---------------------------------------------------------------------------
-// Projector pieces of LayerDerivative (projectOut + rho^-1), per node:
-//   Sinv = S^-1 (Gauss-Jordan, partial pivoting; S is overwritten)
-//   P    = Sinv D
-//   M2   = -(rhoinv P^T)
+// Projector pieces of LayerDerivative (projectOut + rho^-1), per node, in the
+// arithmetic of the plan:
+//   X  = S^-1
+//   P  = X D
+//   M2 = -(rhoinv P^T)
 // so that the derivative is dPsi = alpha ((H Phi) rhoinv^T + Phi M2^T).
+// S = Phi^dagger Phi is Hermitian positive definite: X comes from the sweep
+// operator; a pivot that is not positive (linearly dependent columns) sends
+// the node to Gauss-Jordan with partial pivoting.  Row m of P gives column m
+// of M2, so the blocks (node, part) of a node share the rows of P: each
+// inverts S itself (no exchange) and takes every parts-th row.
 // ---------------------------------------------------------------------------
-// Projector of one node in the arithmetic of the plan: X = S^-1 by
-// Gauss-Jordan with partial pivoting (warp-parallel pivot search), then
-// P = X D and M2 = -rhoinv P^T.  S and X live in shared memory when
-// 2 d^2 elements fit (smem != 0), else in the task's Sinv / P slots.
+// X = S^-1 by Gauss-Jordan with partial pivoting (warp-parallel pivot
+// search); W (d x d) is scratch
 template <class P>
-__global__ void __launch_bounds__(kThreads) k_proj2(const ProjTask* __restrict__ tasks, int64_t task0, int smem) {
+__device__ void pivoted_inverse(const typename P::S* Sin, typename P::S* W, typename P::S* X, int d) {
   typedef typename P::S S;
   typedef typename P::A A;
-  extern __shared__ __align__(16) unsigned char proj_smem[];
-  const ProjTask t = tasks[task0 + blockIdx.x];
-  const int d = t.d;
-  S* W = smem ? reinterpret_cast<S*>(proj_smem) : reinterpret_cast<S*>(t.P);      // working S
-  S* X = smem ? W + d * d : reinterpret_cast<S*>(t.Sinv);                          // becomes S^-1
   __shared__ S fcol[kHpMaxDim];
   __shared__ int piv;
   __shared__ S pinv;
-  const S* Sin = reinterpret_cast<const S*>(t.S);
   for (int e = threadIdx.x; e < d * d; e += kThreads) {
     W[e] = Sin[e];
     S z = P::zero();
@@ -1051,29 +1142,66 @@ __global__ void __launch_bounds__(kThreads) k_proj2(const ProjTask* __restrict__
     }
     __syncthreads();
   }
-  // P = X D into W (S is no longer needed)
-  const S* D = reinterpret_cast<const S*>(t.D);
-  for (int e = threadIdx.x; e < d * d; e += kThreads) {
-    const int i = e % d, j = e / d;
-    A acc = P::zero();
-    for (int k = 0; k < d; ++k) {
-      P::mac(acc, X[i + d * k], D[k + d * j]);
-      if (k & 1) P::norm(acc);
+}
+
+template <class P>
+__global__ void __launch_bounds__(kThreads) k_proj(const ProjTask* __restrict__ tasks, int64_t task0) {
+  typedef typename P::S S;
+  typedef typename P::A A;
+  extern __shared__ __align__(16) unsigned char proj_smem[];
+  const ProjTask t = tasks[task0 + blockIdx.x];
+  const int d = t.d;
+  S* X = reinterpret_cast<S*>(proj_smem);
+  __shared__ __align__(16) unsigned char col_raw[2 * kHpMaxDim * sizeof(S)];
+  const S* Sin = reinterpret_cast<const S*>(t.S);
+  S* Pm = reinterpret_cast<S*>(t.P);
+  int part = blockIdx.y, parts = gridDim.y;
+  for (int e = threadIdx.x; e < d * d; e += kThreads) X[e] = Sin[e];
+  __syncthreads();
+  if (herm_sweep_inverse<P>(X, d, reinterpret_cast<S*>(col_raw))) {
+    for (int e = threadIdx.x; e < d * d; e += kThreads) {  // X = -(lower triangle), mirrored
+      const int i = e % d, j = e / d;
+      if (i < j) continue;
+      const S x = P::neg(X[e]);
+      X[e] = x;
+      if (i > j) X[j + d * i] = P::conj(x);
     }
-    W[e] = P::fin(acc);
+  } else {
+    if (part > 0) return;  // one block of the node (the outcome is the same in all): the scratch is the node's
+    parts = 1;
+    S* W = Pm;
+    S* Xg = reinterpret_cast<S*>(t.Sinv);
+    __syncthreads();
+    pivoted_inverse<P>(Sin, W, Xg, d);
+    for (int e = threadIdx.x; e < d * d; e += kThreads) X[e] = Xg[e];
   }
   __syncthreads();
-  // M2 = -rhoinv P^T
-  const S* Ri = reinterpret_cast<const S*>(t.rhoinv);
-  S* M2 = reinterpret_cast<S*>(t.M2);
-  for (int e = threadIdx.x; e < d * d; e += kThreads) {
-    const int j = e % d, m = e / d;
+  // this block's rows of P = X D: rows part, part + parts, ...
+  const S* __restrict__ D = reinterpret_cast<const S*>(t.D);
+  const int mine = (d - part + parts - 1) / parts;
+  for (int e = threadIdx.x; e < mine * d; e += kThreads) {
+    const int i = part + parts * (e % mine), j = e / mine;
     A acc = P::zero();
+#pragma unroll 4
     for (int k = 0; k < d; ++k) {
-      P::mac(acc, Ri[j + d * k], W[m + d * k]);
+      P::mac(acc, X[i + d * k], P::ld(D + k + d * j));
       if (k & 1) P::norm(acc);
     }
-    M2[e] = P::neg(P::fin(acc));
+    Pm[i + d * j] = P::fin(acc);
+  }
+  __syncthreads();
+  // M2 = -rhoinv P^T, the columns m that these rows give
+  const S* __restrict__ Ri = reinterpret_cast<const S*>(t.rhoinv);
+  S* M2 = reinterpret_cast<S*>(t.M2);
+  for (int e = threadIdx.x; e < mine * d; e += kThreads) {
+    const int j = e % d, m = part + parts * (e / d);
+    A acc = P::zero();
+#pragma unroll 4
+    for (int k = 0; k < d; ++k) {
+      P::mac(acc, P::ld(Ri + j + d * k), Pm[m + d * k]);
+      if (k & 1) P::norm(acc);
+    }
+    M2[j + d * m] = P::neg(P::fin(acc));
   }
 }
 
@@ -1768,14 +1896,15 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       break;
     }
     case ST_PROJ: {
-      // max_eig_d bounds every node's bond
-      const int64_t need = 2 * (int64_t)max_eig_d * max_eig_d * 16;
-      const int sm = need <= 200 * 1024 ? (int)need : 0;
-      if (sm) {
-        cudaError_t e = cudaFuncSetAttribute(k_proj2<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        if (e != cudaSuccess) return e;
-      }
-      k_proj2<P><<<(unsigned)st.n_tasks, kThreads, sm, s>>>(t.proj, st.first_task, sm);
+      // max_eig_d (<= kHpMaxDim) bounds every node's bond.  Up to four blocks
+      // per node while the stage leaves SMs idle: the rows of P are shared
+      // out, the inversion is repeated (64-mode sweep, bonds 32..64: 510 us with
+      // one block per node, 387 with two; 16 modes: 76 -> 57 with four).
+      const int sm = max_eig_d * max_eig_d * 16;
+      cudaError_t e = cudaFuncSetAttribute(k_proj<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      if (e != cudaSuccess) return e;
+      const unsigned parts = (unsigned)std::max<int64_t>(1, std::min<int64_t>(4, 2 * 152 / st.n_tasks));
+      k_proj<P><<<dim3((unsigned)st.n_tasks, parts), kThreads, sm, s>>>(t.proj, st.first_task);
       break;
     }
     case ST_CVT:
