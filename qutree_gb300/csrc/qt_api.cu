@@ -1271,57 +1271,118 @@ int qt_qr_orthogonal(qt_ctx* c) {
   const int64_t cap = c->buf_elems[qt::B_SCR];
   int max_h = 0;
   for (const auto& g : nd) max_h = std::max(max_h, g.height);
-  // per height: Q scratch, R, the task records and the parent's temporary copy
+  // task records: the host copies live until the stream has been waited for
+  std::vector<std::vector<qt::QRTask>> qr_keep;
+  std::vector<std::vector<qt::MPTask>> mp_keep;
+  std::vector<std::vector<int>> by_height(max_h + 1);
+  for (int a = 0; a < (int)nd.size(); ++a)
+    if (!nd[a].top()) by_height[nd[a].height].push_back(a);
+  std::vector<int> slot(nd.size(), -1);  // a parent's place in the height's list
   for (int h = 0; h <= max_h; ++h) {
-    std::vector<int> ids;
-    for (int a = 0; a < (int)nd.size(); ++a)
-      if (!nd[a].top() && nd[a].height == h) ids.push_back(a);
+    const std::vector<int>& ids = by_height[h];
     if (ids.empty()) continue;
-    std::vector<qt::QRTask> tasks;
-    int64_t off = 0, tmp = 0;
+    // the chain scratch of a height: per node M (min(m, n) x n) and R, the
+    // records, then the parents' other copies
+    qr_keep.emplace_back();
+    std::vector<qt::QRTask>& tasks = qr_keep.back();
+    int64_t off = 0;
+    int max_m = 0, max_n = 0;
+    std::vector<int> parents;
+    std::vector<std::vector<size_t>> kids;  // per parent: its children of this height
     for (int a : ids) {
       const int64_t n = nd[a].dup(), m = nd[a].N / n;
       qt::QRTask t;
       t.A = psi + nd[a].off;
       t.Qs = scr + off;
-      off += m * n;
+      off += std::min(m, n) * n;
       t.R = scr + off;
       off += n * n;
       t.m = (int)m;
       t.n = (int)n;
       tasks.push_back(t);
-      tmp = std::max(tmp, nd[nd[a].parent].N);
+      max_m = std::max(max_m, t.m);
+      max_n = std::max(max_n, t.n);
+      const int pa = nd[a].parent;
+      if (slot[pa] < 0) {
+        slot[pa] = (int)parents.size();
+        parents.push_back(pa);
+        kids.emplace_back();
+      }
+      kids[slot[pa]].push_back(tasks.size() - 1);
     }
-    const int64_t task_elems = ((int64_t)(tasks.size() * sizeof(qt::QRTask)) + 15) / 16;
-    if (off + tmp + task_elems > cap)
+    for (int p : parents) slot[p] = -1;
+    auto room = [](size_t bytes) { return ((int64_t)bytes + 15) / 16; };
+    void* dtasks = scr + off;
+    off += room(tasks.size() * sizeof(qt::QRTask));
+    int64_t largest = 0;
+    for (int p : parents) largest = std::max(largest, nd[p].N);
+    // records of the mode products, where they fit (else one launch each)
+    qt::MPTask* dmp = nullptr;
+    const int64_t mp_room = room(ids.size() * sizeof(qt::MPTask));
+    if (off + mp_room + largest <= cap) {
+      dmp = reinterpret_cast<qt::MPTask*>(scr + off);
+      off += mp_room;
+    }
+    if (off + largest > cap)
       return fail(c, QT_ERR_ALLOC, "qt_qr_orthogonal: the chain scratch is too small for one height");
-    double2* ptmp = scr + off;
-    void* dtasks = scr + off + tmp;
     QT_CUDA(c, cudaMemcpyAsync(dtasks, tasks.data(), tasks.size() * sizeof(qt::QRTask), cudaMemcpyHostToDevice,
                                c->stream));
-    QT_CUDA(c, qt::launch_house_qr(dtasks, (int)tasks.size(), c->stream));
+    QT_CUDA(c, qt::launch_house_qr(dtasks, (int)tasks.size(), max_m, max_n, c->stream));
     c->launches += 1;
-    // R into the parents along the child index (siblings of one parent in turn)
-    for (size_t i = 0; i < ids.size(); ++i) {
-      const qt::NodeGeo& g = nd[ids[i]];
-      const qt::NodeGeo& pg = nd[g.parent];
-      qt::MPTask t;
-      t.in = psi + pg.off;
-      t.out = ptmp;
-      t.h = tasks[i].R;
-      t.alpha = make_double2(1.0, 0.0);
-      t.before = (int)pg.before(g.child_idx);
-      t.a_in = t.a_out = g.dup();
-      t.after = (int)pg.after(g.child_idx);
-      t.diag = 0;
-      t.add = 0;
-      QT_CUDA(c, qt::launch_single_mp(t, c->stream, nullptr));
-      QT_CUDA(c, cudaMemcpyAsync(psi + pg.off, ptmp, pg.N * 16, cudaMemcpyDeviceToDevice, c->stream));
-      c->launches += 1;
+    // R into the parents along the child index: as many parents together as
+    // the scratch holds, their children in turn, from one copy to the other
+    for (size_t p0 = 0; p0 < parents.size();) {
+      int64_t used = off;
+      size_t p1 = p0;
+      std::vector<double2*> cur, other;
+      size_t rounds = 0;
+      for (; p1 < parents.size() && p1 - p0 < 32768 && used + nd[parents[p1]].N <= cap; ++p1) {
+        cur.push_back(psi + nd[parents[p1]].off);
+        other.push_back(scr + used);
+        used += nd[parents[p1]].N;
+        rounds = std::max(rounds, kids[p1].size());
+      }
+      for (size_t r = 0; r < rounds; ++r) {
+        mp_keep.emplace_back();
+        std::vector<qt::MPTask>& mt = mp_keep.back();
+        int64_t outputs = 0;
+        for (size_t q = 0; q < cur.size(); ++q) {
+          const std::vector<size_t>& k = kids[p0 + q];
+          if (r >= k.size()) continue;
+          const qt::NodeGeo& g = nd[ids[k[r]]];
+          const qt::NodeGeo& pg = nd[g.parent];
+          qt::MPTask t;
+          t.in = cur[q];
+          t.out = other[q];
+          t.h = tasks[k[r]].R;
+          t.alpha = make_double2(1.0, 0.0);
+          t.before = (int)pg.before(g.child_idx);
+          t.a_in = t.a_out = g.dup();
+          t.after = (int)pg.after(g.child_idx);
+          t.diag = 0;
+          t.add = 0;
+          mt.push_back(t);
+          std::swap(cur[q], other[q]);
+          outputs = std::max(outputs, pg.N);
+        }
+        if (dmp) {
+          QT_CUDA(c, cudaMemcpyAsync(dmp, mt.data(), mt.size() * sizeof(qt::MPTask), cudaMemcpyHostToDevice, c->stream));
+          QT_CUDA(c, qt::launch_mp_each(dmp, (int)mt.size(), outputs, c->stream));
+          c->launches += 1;
+        } else {
+          for (const qt::MPTask& t : mt) QT_CUDA(c, qt::launch_single_mp(t, c->stream, nullptr));
+          c->launches += (int64_t)mt.size();
+        }
+      }
+      for (size_t q = 0; q < cur.size(); ++q) {
+        const qt::NodeGeo& pg = nd[parents[p0 + q]];
+        if (cur[q] != psi + pg.off)
+          QT_CUDA(c, cudaMemcpyAsync(psi + pg.off, cur[q], pg.N * 16, cudaMemcpyDeviceToDevice, c->stream));
+      }
+      p0 = p1;
     }
-    // the task records must outlive their copy
-    QT_CUDA(c, cudaStreamSynchronize(c->stream));
   }
+  QT_CUDA(c, cudaStreamSynchronize(c->stream));
   c->swept = false;
   return QT_OK;
 }

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads) k_mp(const MPTask* __restrict__ task
 // sub-partition's FP64 unit for 256 cycles, far longer than its two operand
 // loads, so four outputs per thread (as in k_mp) save nothing here and cost
 // parallelism: 32 x 32 x 32 along any mode ran in 38.5 us on 32 blocks.
-__global__ void __launch_bounds__(kThreads) k_mp_single(MPTask t) {
+__device__ __forceinline__ void mp_single(const MPTask& t) {
   const int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   const int64_t before = t.before;
   if (e >= before * t.a_out * t.after) return;
@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kThreads) k_mp_single(MPTask t) {
   for (int a = 0; a < t.a_in; ++a) cfma(acc, __ldg(hp + (int64_t)t.a_out * a), __ldg(ip + before * a));
   t.out[e] = t.add ? cadd(t.out[e], acc) : acc;
 }
+__global__ void __launch_bounds__(kThreads) k_mp_single(MPTask t) { mp_single(t); }
 
 // ---------------------------------------------------------------------------
 // Hole product (rhomat / contraction) of the primitive C ABI call:
@@ -2120,118 +2121,273 @@ cudaError_t launch_rho_inverse_static(const double2* rho, double2* rhoinv, int n
 
 // ---------------------------------------------------------------------------
 // Householder QR of node tensors (qrOrthogonal, complex128 on the FP64 pipe).
-// One block per node: A (m x n, column-major: the node tensor as a
-// (lastBefore x d_up) matrix) is factored in place by n reflectors
-// H_j = I - tau_j v_j v_j^H (v_j in A[j:m, j], the diagonal of R aside);
-// then the thin Q = H_0 ... H_{n-1} [I; 0] is formed in the scratch Qs and
-// copied over A, and R (n x n, column-major, upper triangular) is written to R.
-// Reflector j maps x = A[j:m, j] to alpha e_1 with alpha = -e^{i arg x_0} |x|
-// (the LAPACK / Eigen choice).  Warps take columns (k = j + 1 + warp,
-// j + 1 + warp + 8, ...), each column's dot product a warp reduction.
+// A (m x n, column-major: the node tensor as a (lastBefore x d_up) matrix) is
+// replaced by its thin Q = H_0 ... H_{s-1} [I; 0], s = min(m, n), and R (n x n,
+// column-major, upper triangular) is written.  Reflector j,
+// H_j = I - tau_j v_j v_j^H, maps x = A[j:m, j] to alpha e_1 with
+// alpha = -e^{i arg x_0} |x| (the Eigen choice).
+//
+// A cluster of CTAs owns a node, each CTA a contiguous block of its rows (in
+// shared memory when they fit, else in place).  Step j is one pass over the
+// rows for all dot products with x = A[j:m, j] (columns k > j: to update
+// them; k < j: the Gram matrix of the reflectors), one exchange of the CTAs'
+// partial sums through distributed shared memory, and the update:
+//   w_k = v^H a_k = x^H a_k - conj(alpha) a_jk,   a_k -= tau v w_k,
+// where |x|^2 is the sum for k = j, and row j comes from its CTA.  Then
+// Q = [I; 0] - V M with the compact form M = T V_top^H, (T^-1)_il = v_i^H v_l
+// for i < l and 1 / tau_i on the diagonal, solved by back substitution
+// (columns shared out over the CTAs), and one product per row.  No atomics,
+// fixed orders of addition.
+//
+// Bound: the FP64 pipe, 10 m n^2 DFMA over the cluster's SMs, and per step a
+// chain of about 3 us (sums, exchange, square root, divisions).  One block per
+// node ran the 31 nodes of a 16-mode tree (bonds 32) in 13.5 ms.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
+constexpr int kQrBuf = 16;  // rows of V staged at a time when the block is in global memory
+__device__ __forceinline__ void qr_sync(int cl) {
+  if (cl > 1)
+    cluster_sync();
+  else
+    __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) k_house_qr(const QRTask* __restrict__ tasks) {
-  const QRTask t = tasks[blockIdx.x];
-  double2* __restrict__ A = t.A;
+__global__ void __launch_bounds__(kThreads) k_house_qr(const QRTask* __restrict__ tasks, int cl, int slab_smem) {
+  extern __shared__ __align__(16) unsigned char qr_raw[];
+  const QRTask t = tasks[blockIdx.x / cl];
   const int m = t.m, n = t.n, steps = min(m, n);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = kThreads / 32;
-  __shared__ double s_tau[112];
-  __shared__ double2 s_alpha[112];
-  __shared__ double s_nrm[kThreads / 32];
+  const int tid = threadIdx.x;
+  const int rank = cl > 1 ? (int)cluster_rank() : 0;
+  const int rp = (m + cl - 1) / cl;                       // rows per CTA
+  const int r0 = min(m, rank * rp), nr = min(m, r0 + rp) - r0;
+  double2* sh = reinterpret_cast<double2*>(qr_raw);
+  double2* part = sh;             // [2][n] this CTA's sums (read by the cluster)
+  double2* rowj = part + 2 * n;   // [2][n] row j, in its CTA (read by the cluster)
+  double2* tw = rowj + 2 * n;     // [n] tau w_k
+  double2* red = tw + n;          // [kThreads]
+  double2* slab = red + kThreads; // the CTA's rows, or kQrBuf rows of V
+  __shared__ double s_tau[kHpMaxDim];
+  __shared__ double2 s_alpha[kHpMaxDim];
+  double2* X = slab_smem ? slab : t.A + r0;  // element (i, k) of the block at X[i + ld k]
+  const int64_t ld = slab_smem ? (rp | 1) : m;
+  if (slab_smem)
+    for (int e = tid; e < nr * n; e += kThreads) {
+      const int i = e % nr, k = e / nr;
+      X[i + ld * k] = t.A[r0 + i + (int64_t)m * k];
+    }
+  int ch = 1;  // dot products: n column slots x ch row lanes (a power of two)
+  while (2 * ch * n <= kThreads) ch *= 2;
+  __syncthreads();
   for (int j = 0; j < steps; ++j) {
-    double2* x = A + (int64_t)m * j;
-    // |x|^2 over rows j..m-1
-    double q = 0.0;
-    for (int i = j + tid; i < m; i += kThreads) q += x[i].x * x[i].x + x[i].y * x[i].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    if (lane == 0) s_nrm[warp] = q;
+    const int par = j & 1, lo = max(0, j - r0);  // first row of the block at or below row j
+    // partial x^H a_k over the block's rows >= j
+    {
+      const int k = tid % n, c = tid / n;
+      double2 acc = cz();
+      if (c < ch) {
+        const double2* x = X + ld * j;
+        const double2* a = X + ld * k;
+        for (int i = lo + c; i < nr; i += ch) cfmac(acc, x[i], a[i]);
+        red[tid] = acc;
+      }
+      for (int h = ch / 2; h > 0; h /= 2) {
+        __syncthreads();
+        if (c < h) red[tid] = cadd(red[tid], red[tid + h * n]);
+      }
+      __syncthreads();
+      if (tid < n) part[par * n + tid] = red[tid];
+      if (j >= r0 && j < r0 + nr && tid < n) rowj[par * n + tid] = X[(j - r0) + ld * tid];
+    }
+    qr_sync(cl);
+    // total sums (CTAs in a fixed tree) and row j
+    double2 row = cz();
+    {
+      const int k = tid % n, c = tid / n;
+      if (cl > 1) {
+        int q = 1;  // threads per column, a power of two
+        while (2 * q * n <= kThreads && 2 * q <= cl) q *= 2;
+        if (c < q) {
+          double2 v = cz();
+          for (int r = c; r < cl; r += q) v = cadd(v, ld_cluster(part + par * n + k, (uint32_t)r));
+          red[tid] = v;
+        }
+        for (int h = q / 2; h > 0; h /= 2) {
+          __syncthreads();
+          if (c < h) red[tid] = cadd(red[tid], red[tid + h * n]);
+        }
+        if (tid < n) row = ld_cluster(rowj + par * n + tid, (uint32_t)(j / rp));
+      } else if (tid < n) {
+        red[tid] = part[par * n + tid];
+        row = rowj[par * n + tid];
+      }
+    }
+    if (tid == j) red[kThreads - 1] = red[j];  // |x|^2 (the slot is free: n <= kHpMaxDim)
+    if (tid == j) tw[j] = row;                     // x_0
     __syncthreads();
-    if (tid == 0) {
-      double nrm2 = 0.0;
-      for (int w = 0; w < nw; ++w) nrm2 += s_nrm[w];
-      const double2 x0 = x[j];
-      const double ax0 = sqrt(x0.x * x0.x + x0.y * x0.y), nrm = sqrt(nrm2);
-      const double2 ph = ax0 > 0.0 ? make_double2(x0.x / ax0, x0.y / ax0) : make_double2(1.0, 0.0);
-      const double2 alpha = make_double2(-ph.x * nrm, -ph.y * nrm);
-      const double2 v0 = make_double2(x0.x - alpha.x, x0.y - alpha.y);
-      const double vn2 = nrm2 - ax0 * ax0 + v0.x * v0.x + v0.y * v0.y;
-      s_tau[j] = vn2 > 0.0 ? 2.0 / vn2 : 0.0;
-      s_alpha[j] = nrm2 > 0.0 ? alpha : make_double2(0.0, 0.0);
-      x[j] = v0;  // v_j = x - alpha e_1 (rows j..m-1 of column j)
+    if (tid < 32) {  // the scalars, roots and divisions in separate lanes
+      const double nrm2 = red[kThreads - 1].x;
+      const double2 x0 = tw[j];
+      const double a2 = x0.x * x0.x + x0.y * x0.y;
+      const double rt = sqrt(tid == 0 ? nrm2 : a2);
+      const double nrm = __shfl_sync(0xffffffffu, rt, 0), ax0 = __shfl_sync(0xffffffffu, rt, 1);
+      const double den = nrm2 + ax0 * nrm;  // |v|^2 / 2
+      const double q = tid == 0 ? 1.0 / den : x0.x / ax0;
+      const double qy = x0.y / ax0;
+      if (tid == 0) s_tau[j] = den > 0.0 ? q : 0.0;
+      if (tid == 1) {
+        const double2 ph = ax0 > 0.0 ? make_double2(q, qy) : make_double2(1.0, 0.0);
+        s_alpha[j] = make_double2(-ph.x * nrm, -ph.y * nrm);
+      }
     }
     __syncthreads();
     const double tau = s_tau[j];
-    // columns k > j: a -= tau v (v^H a)
-    for (int k = j + 1 + warp; k < n; k += nw) {
-      double2* a = A + (int64_t)m * k;
-      double2 w = make_double2(0.0, 0.0);
-      for (int i = j + lane; i < m; i += 32) {
-        const double2 vi = x[i], ai = a[i];
-        w.x += vi.x * ai.x + vi.y * ai.y;  // conj(v) a
-        w.y += vi.x * ai.y - vi.y * ai.x;
-      }
-      w = warp_sum2(w);
-      const double2 tw = make_double2(tau * w.x, tau * w.y);
-      for (int i = j + lane; i < m; i += 32) {
-        const double2 vi = x[i];
-        a[i].x -= vi.x * tw.x - vi.y * tw.y;
-        a[i].y -= vi.x * tw.y + vi.y * tw.x;
+    const double2 al = s_alpha[j];
+    if (tid < n && tid != j) {
+      double2 w = red[tid];  // - conj(alpha) a_jk
+      w.x = fma(-al.x, row.x, fma(-al.y, row.y, w.x));
+      w.y = fma(-al.x, row.y, fma(al.y, row.x, w.y));
+      if (tid > j)
+        tw[tid] = make_double2(tau * w.x, tau * w.y);
+      else if (rank == 0)
+        t.R[j + (int64_t)n * tid] = make_double2(w.x, -w.y);  // v_k^H v_j, parked below R's diagonal
+    }
+    if (j >= r0 && j < r0 + nr && tid == j) X[(j - r0) + ld * j] = make_double2(row.x - al.x, row.y - al.y);
+    __syncthreads();
+    const int nk = n - 1 - j;
+    if (nk > 0) {
+      const int rows = kThreads / nk;  // row lanes per column
+      const int k = j + 1 + tid % nk, c = tid / nk;
+      if (c < rows) {
+        const double2* v = X + ld * j;
+        double2* a = X + ld * k;
+        const double2 f = make_double2(-tw[k].x, -tw[k].y);
+        for (int i = lo + c; i < nr; i += rows) cfma(a[i], v[i], f);
       }
     }
     __syncthreads();
   }
-  // R: the upper triangle above the diagonal is final in A, the diagonal is alpha
+  // R's upper triangle (final in the rows above the diagonal; the diagonal is alpha)
   for (int e = tid; e < n * n; e += kThreads) {
     const int i = e % n, k = e / n;
-    double2 r = make_double2(0.0, 0.0);
-    if (i < k && i < m) r = A[i + (int64_t)m * k];
-    else if (i == k && i < steps) r = s_alpha[i];
-    t.R[e] = r;
+    if (i > k) continue;
+    if (i >= r0 && i < r0 + nr)
+      t.R[e] = i < k ? X[(i - r0) + ld * k] : s_alpha[i];
+    else if (i >= m && rank == 0)
+      t.R[e] = cz();
   }
-  // thin Q = H_0 ... H_{n-1} [I; 0], accumulated backwards in Qs
-  double2* __restrict__ Q = t.Qs;
-  for (int64_t e = tid; e < (int64_t)m * n; e += kThreads) {
-    const int i = (int)(e % m), k = (int)(e / m);
-    Q[e] = make_double2(i == k ? 1.0 : 0.0, 0.0);
+  // the reflectors' top rows for the other CTAs
+  if (slab_smem)
+    for (int e = tid; e < min(nr, max(0, n - r0)) * steps; e += kThreads) {
+      const int w = min(nr, n - r0), i = e % w, k = e / w;
+      t.A[r0 + i + (int64_t)m * k] = X[i + ld * k];
+    }
+  qr_sync(cl);
+  // M = T V_top^H (steps x n) into Qs, columns rank, rank + cl, ...
+  {
+    const int cb = min(kThreads / steps, kThreads / 2), i = tid % steps, c = tid / steps;
+    for (int c0 = 0; rank + cl * c0 < n; c0 += cb) {
+      const int k = rank + cl * (c0 + c);
+      const bool act = c < cb && k < n;
+      double2 acc = cz();
+      if (act && i <= k && k < m) {
+        acc = t.A[k + (int64_t)m * i];
+        acc.y = -acc.y;
+      }
+      for (int l = steps - 1; l >= 0; --l) {
+        double2* mr = red + (l & 1) * (kThreads / 2);
+        if (act && i == l) {
+          const double2 v = make_double2(s_tau[l] * acc.x, s_tau[l] * acc.y);
+          mr[c] = v;
+          t.Qs[l + (int64_t)steps * k] = v;
+        }
+        __syncthreads();
+        if (act && i < l) {
+          const double2 g = t.R[l + (int64_t)n * i];
+          cfma(acc, make_double2(-g.x, -g.y), mr[c]);
+        }
+      }
+      __syncthreads();
+    }
   }
-  __syncthreads();
-  for (int j = steps - 1; j >= 0; --j) {
-    const double2* v = A + (int64_t)m * j;
-    const double tau = s_tau[j];
-    for (int k = j + warp; k < n; k += nw) {
-      double2* qk = Q + (int64_t)m * k;
-      double2 w = make_double2(0.0, 0.0);
-      for (int i = j + lane; i < m; i += 32) {
-        const double2 vi = v[i], ai = qk[i];
-        w.x += vi.x * ai.x + vi.y * ai.y;
-        w.y += vi.x * ai.y - vi.y * ai.x;
+  qr_sync(cl);
+  if (rank == 0)
+    for (int e = tid; e < n * n; e += kThreads)
+      if (e % n > e / n) t.R[e] = cz();
+  // Q = [I; 0] - V M, row by row
+  const int span = slab_smem ? nr : kQrBuf;
+  for (int b0 = 0; b0 < nr; b0 += span) {
+    const int nb = min(span, nr - b0);
+    const double2* v = X;
+    int64_t lv = ld;
+    if (!slab_smem) {
+      for (int e = tid; e < nb * steps; e += kThreads) slab[e] = X[b0 + e % nb + ld * (e / nb)];
+      __syncthreads();
+      v = slab;
+      lv = nb;
+    }
+    for (int e = tid; e < nb * n; e += kThreads) {
+      const int i = e % nb, k = e / nb, row = r0 + b0 + i;
+      double2 acc = make_double2(row == k ? 1.0 : 0.0, 0.0);
+      const int last = min(row, steps - 1);  // v_l is zero above row l
+#pragma unroll 4
+      for (int l = 0; l <= last; ++l) {
+        const double2 x = v[i + lv * l];
+        cfma(acc, make_double2(-x.x, -x.y), t.Qs[l + (int64_t)steps * k]);
       }
-      w = warp_sum2(w);
-      const double2 tw = make_double2(tau * w.x, tau * w.y);
-      for (int i = j + lane; i < m; i += 32) {
-        const double2 vi = v[i];
-        qk[i].x -= vi.x * tw.x - vi.y * tw.y;
-        qk[i].y -= vi.x * tw.y + vi.y * tw.x;
-      }
+      t.A[row + (int64_t)m * k] = acc;
     }
     __syncthreads();
   }
-  for (int64_t e = tid; e < (int64_t)m * n; e += kThreads) A[e] = Q[e];
 }
 
-cudaError_t launch_house_qr(const void* tasks, int n_tasks, cudaStream_t s) {
-  if (n_tasks <= 0) return cudaSuccess;
-  k_house_qr<<<(unsigned)n_tasks, kThreads, 0, s>>>(static_cast<const QRTask*>(tasks));
+// mode products of several tensors, one thread per output as k_mp_single;
+// blockIdx.y is the task
+__global__ void __launch_bounds__(kThreads) k_mp_each(const MPTask* __restrict__ tasks) {
+  mp_single(tasks[blockIdx.y]);
+}
+
+cudaError_t launch_mp_each(const MPTask* tasks, int n_tasks, int64_t max_outputs, cudaStream_t s) {
+  if (n_tasks <= 0 || max_outputs <= 0) return cudaSuccess;
+  k_mp_each<<<dim3((unsigned)((max_outputs + kThreads - 1) / kThreads), (unsigned)n_tasks), kThreads, 0, s>>>(tasks);
   return cudaGetLastError();
+}
+
+// CTAs per node: the most (a power of two, at most 16, or 8 where clusters of
+// 16 do not fit) that leave every CTA at least 32 rows and the launch at most
+// 152 CTAs.
+cudaError_t launch_house_qr(const void* tasks, int n_tasks, int max_m, int max_n, cudaStream_t s) {
+  if (n_tasks <= 0) return cudaSuccess;
+  const int fixed = 5 * max_n + kThreads;  // shared elements beside the rows
+  constexpr int kMaxSmem = 227 * 1024 - 4096;  // the static arrays take the rest
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaFuncSetAttribute(k_house_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_house_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  int cl = 1;
+  while (cl < 16 && (int64_t)2 * cl * n_tasks <= 152 && max_m >= 64 * cl) cl *= 2;
+  for (;; cl /= 2) {
+    const int64_t rp = (max_m + cl - 1) / cl;
+    const int64_t in_smem = 16 * (fixed + (rp | 1) * max_n);
+    const int slab = in_smem <= kMaxSmem;
+    cfg.dynamicSmemBytes = (size_t)(slab ? in_smem : 16 * (fixed + (int64_t)kQrBuf * max_n));
+    cfg.gridDim = dim3((unsigned)(n_tasks * cl));
+    at[0].val.clusterDim.x = (unsigned)cl;
+    int fit = 1;
+    if (cl > 8) {
+      if (cudaOccupancyMaxActiveClusters(&fit, k_house_qr, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        fit = 0;
+      }
+    }
+    if (fit < 1) continue;
+    return cudaLaunchKernelEx(&cfg, k_house_qr, static_cast<const QRTask*>(tasks), cl, slab);
+  }
 }
 
 }  // namespace qt
