@@ -26,7 +26,6 @@ namespace qt {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMpTile = kThreads;  // slots (up to four outputs each) per mode-product tile, as in the planner
 constexpr int kHpMaxDim = 112;  // largest bond the planner admits
 constexpr int kAccRows = 64;
 constexpr int kCvtPerThread = 8;  // 2048 elements per tile, as in the planner

@@ -58,7 +58,6 @@ struct TfSmem {
 };
 static_assert(sizeof(TfSmem) <= 232448, "shared memory of the split-TF32 kernel exceeds 227 KB");
 
-__device__ __forceinline__ int fexp(float v) { return (__float_as_int(v) >> 23) & 0xff; }
 __device__ __forceinline__ float pow2f(int k) { return __int_as_float((k + 127) << 23); }
 __device__ __forceinline__ float scale2(float v, int k) {
   if (k > 127) return (v * pow2f(127)) * pow2f(k - 127);
@@ -83,14 +82,20 @@ __device__ __forceinline__ float dsplit(float& r, float sigma) {
   return x;
 }
 __device__ __forceinline__ float digit_sigma(int s) { return __int_as_float(((127 + 16 - 7 * s) << 23) | 0x400000); }
-// v 2^k exactly (row scaling)
-__device__ __forceinline__ float row_scale(float v, int k) {
-  return (k >= -126 && k <= 127) ? v * pow2f(k) : scale2(v, k);
+// 2^(126 - eb), eb in 1..255 (subnormal from eb = 253 on): the row's scaling
+__device__ __forceinline__ float row_factor(int eb) {
+  const int k = 126 - eb;
+  return __int_as_float(k >= -126 ? (k + 127) << 23 : 0x00800000 >> (-126 - k));
 }
+// |x| as an ordered integer; the biased exponent of a row whose largest one
+// is m.  A row of zeros gets 126 (scale 1): its digits are zero whatever the
+// scale, and the epilogue's common path keeps its rows.
+__device__ __forceinline__ int fmag(float v) { return __float_as_int(v) & 0x7fffffff; }
+__device__ __forceinline__ int row_exponent(int m) { return m == 0 ? 126 : max(1, m >> 23); }
 // the seven digits x_s of hi + lo as floats (exact in bf16: their upper
-// 16 bits are the bf16)
-__device__ __forceinline__ void digits_f32(float hi, float lo, int eb, float d[kDig]) {
-  float rh = row_scale(hi, 126 - eb), rl = row_scale(lo, 126 - eb);
+// 16 bits are the bf16); f = row_factor of the row
+__device__ __forceinline__ void digits_f32(float hi, float lo, float f, float d[kDig]) {
+  float rh = __fmul_rn(hi, f), rl = __fmul_rn(lo, f);
 #pragma unroll
   for (int s = 0; s < kDig; ++s) {
     float x = dsplit(rh, digit_sigma(s));
@@ -658,20 +663,20 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
     img = static_cast<unsigned char*>(T.tc_img) + (size_t)u.y * hp_tc_chunk_bytes(np, steps);
   }
   (void)ncols;
-  __shared__ int fx[64];
-  if (threadIdx.x < 64) fx[threadIdx.x] = 1;
+  __shared__ int fx[64];  // largest |W| of a row as an integer, then its exponent
+  if (threadIdx.x < 64) fx[threadIdx.x] = 0;
   __syncthreads();
-  int m = 1;
+  int m = 0;
   for (int ks = q; ks < steps; ks += 4) {
     float4 v[16];
     load16(ks, v);
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) m = max(m, max(fexp(v[kk].x), fexp(v[kk].z)));
+    for (int kk = 0; kk < 16; ++kk) m = max(m, max(fmag(v[kk].x), fmag(v[kk].z)));
   }
   atomicMax(&fx[n], m);
   __syncthreads();
   if (n < np) {
-    const int f = fx[n];
+    const float f = row_factor(row_exponent(fx[n]));
     const int rows = 3 * np, plane = rows * 32;
     for (int ks = q; ks < steps; ks += 4) {
       float4 v[16];
@@ -707,7 +712,8 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
       }
     }
   }
-  if (threadIdx.x < 64) reinterpret_cast<int*>(img + (size_t)steps * kDig * 3 * np * 32)[threadIdx.x] = fx[threadIdx.x];
+  if (threadIdx.x < 64)
+    reinterpret_cast<int*>(img + (size_t)steps * kDig * 3 * np * 32)[threadIdx.x] = row_exponent(fx[threadIdx.x]);
 }
 
 // pre-pass of the hole products: the biased row exponents E of the M side
@@ -730,7 +736,7 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int m = m0 + warp + 8 * r;
-      e[r] = 1;
+      e[r] = 0;
       if (m < rows) {
         const int mi = m / a, j = m - mi * a;
         const float4* __restrict__ B = reinterpret_cast<const float4*>(g.hp[G.member[mi]].B);
@@ -740,7 +746,7 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
           if (k < k1) {
             const int c = k / before, b = k - c * before;
             const float4 x = __ldg(B + b + (int64_t)before * j + (int64_t)before * a * c);
-            e[r] = max(e[r], max(fexp(x.x), fexp(x.z)));
+            e[r] = max(e[r], max(fmag(x.x), fmag(x.z)));
           }
         }
       }
@@ -750,12 +756,12 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
       int v = e[r];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (lane == 0) ex[m0 + warp + 8 * r] = (uint8_t)v;
+      if (lane == 0) ex[m0 + warp + 8 * r] = (uint8_t)row_exponent(v);
     }
   } else {
     __shared__ int part[8][32];
     const int m = m0 + lane;
-    int e = 1;
+    int e = 0;
     if (m < rows) {
       const int mi = m / a, j = m - mi * a;
       const float4* __restrict__ B = reinterpret_cast<const float4*>(g.hp[G.member[mi]].B);
@@ -763,7 +769,7 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
       const int ka = k0 + warp * span, kb = min(k1, ka + span);
       for (int k = ka; k < kb; ++k) {
         const float4 x = __ldg(B + j + (int64_t)a * k);
-        e = max(e, max(fexp(x.x), fexp(x.z)));
+        e = max(e, max(fmag(x.x), fmag(x.z)));
       }
     }
     part[warp][lane] = e;
@@ -772,9 +778,64 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
       int v = part[0][lane];
 #pragma unroll
       for (int w = 1; w < 8; ++w) v = max(v, part[w][lane]);
-      ex[m] = (uint8_t)v;
+      ex[m] = (uint8_t)row_exponent(v);
     }
   }
+}
+
+// Four columns of the accumulators (real parts from column 0 of `addr`, the
+// imaginary parts np columns on), their levels added in double-float: levels
+// 0..2 by two-sums, the others (at least one) into the low word.  All threads
+// of the warp.
+__device__ __forceinline__ void tcs_levels(uint32_t addr, int np, int NL, float (&v)[2][4], float (&l)[2][4]) {
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    float lv[kDig][4];
+    const uint32_t a = addr + (uint32_t)(part * np);
+#pragma unroll
+    for (int L = 0; L < kDig; ++L)
+      if (L < 4 || L < NL) tmem_ld4(a + (uint32_t)(L * 2 * np), lv[L]);
+    tmem_wait_ld();
+    if (NL > 4) {
+#pragma unroll
+      for (int L = 4; L < kDig; ++L)
+        if (L < NL) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) lv[3][i] = __fadd_rn(lv[3][i], lv[L][i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float s, e1, e2;
+      df_two_sum(lv[0][i], lv[1][i], s, e1);
+      df_two_sum(s, lv[2][i], v[part][i], e2);
+      l[part][i] = __fadd_rn(__fadd_rn(e2, e1), lv[3][i]);
+    }
+  }
+}
+
+// 4 x 4 transpose of o among the four lanes of a quad: afterwards o[i] is what
+// lane (lane & ~3) + i held in o[lane & 3]
+__device__ __forceinline__ void quad_transpose(float4 (&o)[4], int lane) {
+#pragma unroll
+  for (int bit = 1; bit <= 2; bit <<= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i & bit) continue;  // the pair (i, i | bit)
+      const float4 send = up ? o[i] : o[i | bit];
+      float4 got;
+      got.x = __shfl_xor_sync(0xffffffffu, send.x, bit);
+      got.y = __shfl_xor_sync(0xffffffffu, send.y, bit);
+      got.z = __shfl_xor_sync(0xffffffffu, send.z, bit);
+      got.w = __shfl_xor_sync(0xffffffffu, send.w, bit);
+      if (up) o[i] = got;
+      else o[i | bit] = got;
+    }
+  }
+}
+__device__ __forceinline__ float4* shfl_ptr(float4* p, int src) {
+  return reinterpret_cast<float4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), src));
 }
 
 // the producers' view of row r of an item: its source of X and validity
@@ -890,16 +951,21 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         };
         // the row's largest exponent over the unit's k (hole products: from
         // the pre-pass), eight loads in flight
-        int eb = 1;
-        if (OP == TCS_HP)
+        int eb;
+        if (OP == TCS_HP) {
           eb = g.groups[itm.x].ex[(size_t)(itm.z + u) * kRows + r];
-        else if (R.valid)
-          for (int h8 = 0; h8 < 2 * I.nks; ++h8) {
-            float4 x[8];
-            load8(x, h8 >> 1, h8 & 1);
+        } else {
+          int mx = 0;
+          if (R.valid)
+            for (int h8 = 0; h8 < 2 * I.nks; ++h8) {
+              float4 x[8];
+              load8(x, h8 >> 1, h8 & 1);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) eb = max(eb, max(fexp(x[i].x), fexp(x[i].z)));
-          }
+              for (int i = 0; i < 8; ++i) mx = max(mx, max(fmag(x[i].x), fmag(x[i].z)));
+            }
+          eb = row_exponent(mx);
+        }
+        const float rowf = row_factor(eb);
         // the epilogue of the unit two back has read ex of this buffer
         if (!mbar_wait(&sm.bar.exfree[buf], use_par ^ 1, kSpin)) {
           set_status(status, 18);
@@ -936,10 +1002,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float d0[kDig], d1[kDig], e0[kDig], e1[kDig];
-              digits_f32(x[2 * i].x, x[2 * i].y, eb, d0);
-              digits_f32(x[2 * i + 1].x, x[2 * i + 1].y, eb, d1);
-              digits_f32(x[2 * i].z, x[2 * i].w, eb, e0);
-              digits_f32(x[2 * i + 1].z, x[2 * i + 1].w, eb, e1);
+              digits_f32(x[2 * i].x, x[2 * i].y, rowf, d0);
+              digits_f32(x[2 * i + 1].x, x[2 * i + 1].y, rowf, d1);
+              digits_f32(x[2 * i].z, x[2 * i].w, rowf, e0);
+              digits_f32(x[2 * i + 1].z, x[2 * i + 1].w, rowf, e1);
 #pragma unroll
               for (int d = 0; d < kDig; ++d) {
                 wr[d][i] = pack_bf16(d0[d], d1[d]);
@@ -1054,7 +1120,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
       for (int u = 0; u < I.nunits; ++u, ++un) {
         const int buf = (int)(un & 1);
         const bool store = u == 0 && !add_first;
-        if (!mbar_wait(&sm.bar.exready[buf], (un >> 1) & 1, kSpin) || !mbar_wait(&sm.bar.tfull, un & 1, kSpin)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sm.bar.exready[buf], (un >> 1) & 1, kSpin) &&
+                                         mbar_wait(&sm.bar.tfull, un & 1, kSpin))) {
           set_status(status, 17);
           ok = false;
           break;
@@ -1064,65 +1131,96 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         mbar_arrive(&sm.bar.exfree[buf]);
         const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, u, np) +
                                                       (size_t)tcs_img_steps<OP>(np) * kDig * 3 * np * 32);
+        const int f0 = __ldg(fxg + lane), f1 = __ldg(fxg + 32 + lane);
         __syncwarp();
-        for (int i = lane; i < 64; i += 32) fxw[i] = __ldg(fxg + i);
+        fxw[lane] = f0 << 23;
+        fxw[32 + lane] = f1 << 23;
         __syncwarp();
-        for (int n0 = c0; n0 < c1; n0 += 4) {
+        // the common case: every scale 2^(E + F) of the warp's rows and the
+        // unit's columns is a normal number and no operand is infinite or NaN
+        const int fmax = max(__reduce_max_sync(0xffffffffu, f0), __reduce_max_sync(0xffffffffu, f1));
+        const int fmin = min(__reduce_min_sync(0xffffffffu, f0), __reduce_min_sync(0xffffffffu, f1));
+        const bool normal = __all_sync(
+            0xffffffffu, !base || (er + fmin >= 126 && er + fmax <= 379 && er < 255 && fmax < 255));
+        const int erow = (er - 125) << 23;  // + (F << 23): the bits of 2^(E - 126 + F - 126)
+        float4* p = base + stride * c0;
+        // outputs contiguous along the columns (stride 1): a lane's 16-byte
+        // stores would touch 32 lines; the quads transpose 4 x 4 blocks so
+        // that a store covers eight rows of 64 bytes
+        const bool along = stride == 1 && store && normal;  // uniform
+        float4* qp[4];
+        if (along) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) qp[i] = shfl_ptr(base, (lane & ~3) + i);
+        }
+        for (int n0 = c0; n0 < c1; n0 += 4, p += 4 * stride) {
+          const int nc = min(4, I.ncols - n0);  // columns of the block that exist (uniform)
+          if (nc <= 0) break;
           // the old outputs of these four columns: their loads in flight
           // together, under the tensor-memory reads
           float4 old[4];
+          if (!store) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            old[e] = (base && !store && n0 + e < I.ncols) ? base[stride * (n0 + e)] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int e = 0; e < 4; ++e)
+              old[e] = (base && e < nc) ? p[stride * e] : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
           __syncwarp();
-          float vre[4], vim[4], lre[4], lim[4];
-#pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            float lv[kDig][4];
-#pragma unroll
-            for (int L = 0; L < kDig; ++L)
-              if (L < NL) tmem_ld4(lane_addr + (uint32_t)(L * 2 * np + part * np + n0), lv[L]);
-            tmem_wait_ld();
-            float* v = part ? vim : vre;
-            float* l = part ? lim : lre;
+          float v[2][4], l[2][4];  // recombined levels: re and im of the four columns
+          tcs_levels(lane_addr + (uint32_t)n0, np, NL, v, l);
+          if (along) {
+            float4 o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              v[i] = lv[0][i];
-              l[i] = 0.f;
-              if (NL > 1) df_add(v[i], l[i], lv[1][i], 0.f);
-              if (NL > 2) df_add(v[i], l[i], lv[2][i], 0.f);
-              float t3 = 0.f;
-#pragma unroll
-              for (int L = 3; L < kDig; ++L)
-                if (L < NL) t3 = __fadd_rn(t3, lv[L][i]);
-              l[i] = __fadd_rn(l[i], t3);
+              const float f = __int_as_float(erow + fxw[n0 + i]);
+              o[i] = make_float4(__fmul_rn(v[0][i], f), __fmul_rn(l[0][i], f), __fmul_rn(v[1][i], f),
+                                 __fmul_rn(l[1][i], f));
+              df_norm(o[i].x, o[i].y);
+              df_norm(o[i].z, o[i].w);
             }
+            quad_transpose(o, lane);
+            const int col = n0 + (lane & 3);
+            if (col < I.ncols) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (qp[i]) qp[i][col] = o[i];
+            }
+            continue;
           }
           if (!base) continue;
+          if (normal) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = n0 + i;
-            if (col >= I.ncols) continue;
-            const int fn = fxw[col];
-            const int sh = (er - 126) + (fn - 126);
-            float4 v;
-            if (sh >= -126 && sh <= 127) {
-              const float f = pow2f(sh);
-              v = make_float4(vre[i] * f, lre[i] * f, vim[i] * f, lim[i] * f);
-            } else {
-              v = make_float4(scale2(vre[i], sh), scale2(lre[i], sh), scale2(vim[i], sh), scale2(lim[i], sh));
+            for (int i = 0; i < 4; ++i) {
+              const float f = __int_as_float(erow + fxw[n0 + i]);
+              float4 o = make_float4(__fmul_rn(v[0][i], f), __fmul_rn(l[0][i], f), __fmul_rn(v[1][i], f),
+                                     __fmul_rn(l[1][i], f));
+              if (!store) {
+                df_add(o.x, o.y, old[i].x, old[i].y);
+                df_add(o.z, o.w, old[i].z, old[i].w);
+              }
+              df_norm(o.x, o.y);
+              df_norm(o.z, o.w);
+              if (i < nc) p[stride * i] = o;
             }
-            if (!store) {
-              df_add(v.x, v.y, old[i].x, old[i].y);
-              df_add(v.z, v.w, old[i].z, old[i].w);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (i >= nc) continue;
+              const int fn = fxw[n0 + i] >> 23;
+              const int sh = (er - 126) + (fn - 126);
+              float4 o = make_float4(scale2(v[0][i], sh), scale2(l[0][i], sh), scale2(v[1][i], sh),
+                                     scale2(l[1][i], sh));
+              if (!store) {
+                df_add(o.x, o.y, old[i].x, old[i].y);
+                df_add(o.z, o.w, old[i].z, old[i].w);
+              }
+              df_norm(o.x, o.y);
+              df_norm(o.z, o.w);
+              if (er == 255 || fn == 255) {  // an Inf or NaN among the operands: propagate it
+                const float nan = __int_as_float(0x7fffffff);
+                o = make_float4(nan, nan, nan, nan);
+              }
+              p[stride * i] = o;
             }
-            df_norm(v.x, v.y);
-            df_norm(v.z, v.w);
-            if (er == 255 || fn == 255) {  // an Inf or NaN among the operands: propagate it
-              const float nan = __int_as_float(0x7fffffff);
-              v = make_float4(nan, nan, nan, nan);
-            }
-            base[stride * col] = v;
           }
         }
         fence_before_sync();
