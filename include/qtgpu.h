@@ -79,15 +79,17 @@ extern "C" {
  * and outputs of the C ABI are complex128 in both cases. */
 #define QT_PREC_F64 0x000
 #define QT_PREC_DF64 0x100
-/* Double-float arithmetic as QT_PREC_DF64, with the mode products (k <= 64
- * indices in and out) on the fifth-generation tensor cores (tcgen05.mma,
- * accumulators in tensor memory); hole products and last-index
- * accumulations stay on the FP32 pipe.  Every operand row is scaled by a
+/* Double-float arithmetic as QT_PREC_DF64, with the mode products, hole
+ * products and last-index accumulations of shapes from 32 to 112 on the
+ * fifth-generation tensor cores (tcgen05.mma, accumulators in tensor memory;
+ * beyond 64 output columns in column blocks of at most 48, accumulations
+ * only in the compressed plan's sweep).  Every operand row is scaled by a
  * power of two and cut into seven signed digits of at most eight bits by
  * error-free splits, digit products are exact in bf16, each level of digit
  * pairs sums exactly in fp32 as far as tensor memory holds separate level
  * accumulators (all seven for outputs padded to <= 32 columns, five for 48,
- * four for 64, the last taking the remaining levels), and the levels are
+ * four for 64, at most five beyond 64 reduction indices or output columns,
+ * the last taking the remaining levels), and the levels are
  * recombined in double-float.  The error is relative to the row maxima of
  * the operands: 2^-49 of the row scale per value, plus the fp32 rounding of
  * the last level accumulator.  Parity tolerance 1e-10 per contraction and
@@ -386,10 +388,10 @@ int qt_rho_inverse_noalloc(qt_ctx* ctx, void* rhoinv, const void* rho, int n_mat
                            double eps);
 
 /* Lower bounds of the shapes the next qt_prepare puts on the tensor cores
- * (QT_PREC_DF64_TC; QT_PREC_TF32X3 uses the mode-product bound): mode
- * products with mp_min <= a_in, a_out <= 64, hole products with
- * hp_min <= a <= 64, accumulations with acc_min <= d <= 64; 65 keeps a kind
- * on the FP32 pipe.  Defaults 32, 32, 32 (measured on GB300); the autotuner
+ * (QT_PREC_DF64_TC; QT_PREC_TF32X3 uses the mode-product bound, up to 64):
+ * mode products with mp_min <= a_in, a_out <= 112, hole products with
+ * hp_min <= a <= 112, accumulations with acc_min <= d <= 112; 65 keeps a
+ * kind on the FP32 pipe.  Defaults 32, 32, 32 (measured on GB300); the autotuner
  * (qutree_gb300/autotune.py) times probe problems per size on the device
  * and caches the bounds per device.  QT_ERR_ARG outside 1..65. */
 int qt_set_tc_thresholds(qt_ctx* ctx, int mp_min, int hp_min, int acc_min);

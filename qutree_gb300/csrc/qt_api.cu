@@ -518,7 +518,9 @@ int qt_prepare(qt_ctx* c, int flavour) {
     g.before = s.before;
     g.a = s.a;
     g.after = s.after;
-    g.ap = (s.a + 7) & ~7;
+    g.c0 = s.c0;
+    g.nc = s.nc;
+    g.ap = s.ap;
     g.n = s.n;
     g.nchunks = s.nchunks;
     for (int m = 0; m < qt::kHpTcMembers; ++m) g.member[m] = s.member[m];

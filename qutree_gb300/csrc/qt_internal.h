@@ -52,34 +52,47 @@ struct HPTask {
 // all have the same a, before and after.
 constexpr int kHpTcChunk = 64;     // k of the shorter chunks
 constexpr int kHpTcMembers = 8;    // tasks per group (a >= 16)
+// column block of a mode product in its tile and pre-pass records
+constexpr int kMpTcBlockShift = 26, kMpTcTaskShift = 28;
 struct HpTcGroup {
   const double2* A;
   unsigned char* img;  // A's operand images, one per chunk of hp_tc_kc(ap) k
   unsigned char* ex;   // biased row exponents of the members' B, 128 rows per chunk
   int before, a, after;
-  int ap;              // a padded to a multiple of 8
+  int c0, nc;          // the group's columns i: nc of them from c0 (all a of them up to 64)
+  int ap;              // nc padded to a multiple of 8
   int n, nchunks;
   int member[kHpTcMembers];
 };
 // Which contractions the planner puts on the tensor cores: shapes from a
-// lower bound per kind to 64 (padded to at most 64 output columns).  Below
-// the bound the fixed costs of a tile (row exponents, the level
-// recombination, the 128-row tile itself) outweigh the products.  The
-// default bounds, 32, were measured on a forest of uneven trees with bonds
-// 4..24: the double-float sweep took 82.7 ms with every shape up to 64 on the
-// tensor cores, 57.2 ms with the bounds (as on the FP32 pipe alone);
-// qt_set_tc_thresholds takes bounds found by the autotuner
+// lower bound per kind up to kTcMaxDim.  Below the bound the fixed costs of a
+// tile (row exponents, the level recombination, the 128-row tile itself)
+// outweigh the products.  The default bounds, 32, were measured on a forest
+// of uneven trees with bonds 4..24: the double-float sweep took 82.7 ms with
+// every shape up to 64 on the tensor cores, 57.2 ms with the bounds (as on the
+// FP32 pipe alone); qt_set_tc_thresholds takes bounds found by the autotuner
 // (qutree_gb300/autotune.py).  65 keeps a kind off the tensor cores.
+// Shapes beyond 64 output columns (the accumulator tile's most) are cut into
+// column blocks, each an item of its own that produces the row digits again:
+// the 64-mode tree with bonds 32..96 runs its sweep in 36.5 ms this way,
+// 157 ms with the shapes from 65 on the FP32 pipe.
+constexpr int kTcCols = 64;     // output columns of one accumulator tile
+constexpr int kTcMaxDim = 112;  // seven 16-k steps; the planner's largest bond
 struct TcTune {
   int mp = 32, hp = 32, acc = 32;
 };
-// hole product: lo <= a <= 64 and at least two 64-k chunks of reduction
+// hole product: lo <= a and at least two 64-k chunks of reduction
 inline bool hp_tc_eligible(int before, int a, int after, int lo = 32) {
-  return a >= lo && a <= 64 && (int64_t)before * after >= 2 * kHpTcChunk;
+  return a >= lo && lo <= kTcCols && a <= kTcMaxDim && (int64_t)before * after >= 2 * kHpTcChunk;
 }
 // mode product (not diagonal): lo <= a_in, a_out <= 64
 inline bool mp_tc_eligible(int a_in, int a_out, int lo = 32) {
   return a_in >= lo && a_in <= 64 && a_out >= lo && a_out <= 64;
+}
+// mode product beyond 64 (double-float plans): at least one full 128-row tile
+inline bool mp_tc_wide(int a_in, int a_out, int64_t rows, int lo = 32) {
+  return a_in >= lo && a_out >= lo && lo <= kTcCols && (a_in > 64 || a_out > 64) && a_in <= kTcMaxDim &&
+         a_out <= kTcMaxDim && rows >= 128;
 }
 #ifdef __CUDACC__
 #define QT_HD __host__ __device__
@@ -90,6 +103,14 @@ inline bool mp_tc_eligible(int a_in, int a_out, int lo = 32) {
 // accumulators keep the levels 0..2 exact up to 170 k, else 64 k (seven
 // exact levels up to 73 k)
 QT_HD constexpr int hp_tc_kc(int ap) { return ap > 32 ? 2 * kHpTcChunk : kHpTcChunk; }
+// column blocks of n output columns, and the columns of a full one (a multiple
+// of 8; the last block has the rest).  Beyond kTcCols a block has at most 48:
+// five level accumulators, whose last one holds levels 4..6 only (2^-52 of
+// the row scales), below the digits' truncation.
+QT_HD constexpr int tc_blocks(int n) { return n <= kTcCols ? 1 : (n + 47) / 48; }
+QT_HD constexpr int tc_width(int n) { return ((n + tc_blocks(n) - 1) / tc_blocks(n) + 7) & ~7; }
+// 16-k steps of the operand image of a mode product or accumulation over k
+QT_HD constexpr int tc_steps(int k) { return k <= 64 ? 4 : (k + 15) / 16; }
 // bytes of one unit's operand image: steps of 16 k x 7 digits x rows
 // [-Wi | Wr | Wi] (3 ap) x 16 bf16, then the column exponents (int, 64 slots)
 QT_HD constexpr int64_t hp_tc_chunk_bytes(int ap, int steps) {
@@ -109,11 +130,13 @@ struct AccTask {
   int rows, d;
   int first, count;
   int add, pad;
-  void* tc_img = nullptr;  // tensor-core path: images of alpha H_t, one per term (hp_tc_chunk_bytes(., 4))
+  void* tc_img = nullptr;  // tensor-core path: images of alpha H_t, one per column block and term
 };
 // an accumulation the planner puts on the tensor cores (double-float plans):
-// lo <= d <= 64 and at least 64 rows
-inline bool acc_tc_eligible(int rows, int d, int lo = 32) { return d >= lo && d <= 64 && rows >= 64; }
+// lo <= d <= kTcMaxDim and at least 64 rows
+inline bool acc_tc_eligible(int rows, int d, int lo = 32) {
+  return d >= lo && lo <= kTcCols && d <= kTcMaxDim && rows >= 64;
+}
 
 // out = sum_t c_t * M_t for d x d matrices (grouped mean fields).
 struct LinTerm {
@@ -541,8 +564,8 @@ struct Plan {
   std::vector<int4> hp_segs;  // (rows, cols, first tile, tile count) per hole-product launch
   // double-float plans with tensor-core mode products: (task, block of 32 rows)
   bool mp_tensor = false;
-  std::vector<int2> mp_oz_tiles;
-  std::vector<int> mp_oz_tasks;
+  std::vector<int2> mp_oz_tiles;  // (task, 128-row block | column block << kMpTcBlockShift)
+  std::vector<int> mp_oz_tasks;   // task | column block << kMpTcTaskShift
   int64_t oz_bytes = 0;  // B_OZ: operand images of the tensor-core tasks of one stage (reused by every stage)
   // double-float plans with tensor-core hole products (groups bound to HpTcGroup)
   bool hp_tensor = false;
@@ -550,6 +573,7 @@ struct Plan {
   struct SHpTcGroup {
     Ref A;
     int before = 0, a = 0, after = 0, n = 0, nchunks = 0;
+    int c0 = 0, nc = 0, ap = 0;  // columns of the group
     int member[kHpTcMembers] = {0, 0, 0, 0, 0, 0, 0, 0};
     int64_t img = 0;  // byte offset of the images in B_OZ
     int64_t ex = 0;   // byte offset of the row exponents in B_OZ (128 per chunk)
@@ -557,8 +581,8 @@ struct Plan {
   std::vector<SHpTcGroup> hp_tc_groups;
   std::vector<int4> hp_tc_items;  // (group, z, first chunk, end chunk)
   std::vector<int2> hp_tc_imgs;   // (group, chunk) of the image pre-pass
-  std::vector<int4> acc_tc_items;  // (task, 128-row block, units before the item in its stage, 0)
-  std::vector<int2> acc_tc_imgs;   // (task, term) of the image pre-pass
+  std::vector<int4> acc_tc_items;  // (task, 128-row block, units before the item in its stage, column block)
+  std::vector<int2> acc_tc_imgs;   // (task, term + terms x column block) of the image pre-pass
   std::vector<int4> acc_tiles;
   std::vector<int2> cvt_tiles;
   // constant matrices written once at prepare: (offset, d) identity

@@ -102,6 +102,7 @@ class Builder {
     stage_inverse();
     if (scf && !compressed) throw std::runtime_error("the SCF sweep needs the compressed plan");
     if (compressed) {
+      wide_acc = true;
       comp_layout();
       comp_represent();
       comp_meanfield();
@@ -113,7 +114,9 @@ class Builder {
       P.main_end = (int64_t)P.stages.size();
       const double sweep_flops = P.stats.exec_flops;
       const PlanStats counts = P.stats;
+      wide_acc = false;
       comp_frozen_apply();
+      wide = false;
       if (scf) scf_segments();
       P.stats = counts;
       P.stats.exec_flops = sweep_flops;
@@ -143,6 +146,15 @@ class Builder {
 
  private:
   Plan& P;
+  // Contractions of more than 64 columns on the tensor cores.  The digits'
+  // error is relative to a row's largest operand, a double-float
+  // multiply-add's to each product.  The sweep's error does not tell them apart
+  // (bonds 66..96 against the oracle: 2.9e-13, double-float 2.6e-13), but
+  // accumulations that cancel do: (H Phi) rhoinv^T + Phi M2^T with H Phi formed
+  // (the frozen-matrix derivative; reference and grouped plans) gives 2.3e-12
+  // instead of 3.3e-13.  Those, and the SCF segments, whose Krylov vectors
+  // amplify any change of rounding, keep the FP32 pipe beyond 64.
+  bool wide = true, wide_acc = false;
   std::vector<NodeGeo>& nd;
   const OpTable& ops;
   const SopDesc& sop;
@@ -470,7 +482,8 @@ class Builder {
     std::vector<char> tc(t1 - t0, 0);
     if (P.hp_tensor)
       for (int64_t t = t0; t < t1; ++t)
-        tc[t - t0] = hp_tc_eligible(P.hp[t].before, P.hp[t].a, P.hp[t].after, P.tune.hp);
+        tc[t - t0] = hp_tc_eligible(P.hp[t].before, P.hp[t].a, P.hp[t].after, P.tune.hp) &&
+                     (wide || P.hp[t].a <= kTcCols);
     double work = 0;
     for (int64_t t = t0; t < t1; ++t)
       if (!tc[t - t0]) work += (double)ntiles(P.hp[t]) * P.hp[t].before * P.hp[t].after;
@@ -521,38 +534,44 @@ class Builder {
   // Returns whether any task was cut.
   bool hp_tensor_items(int64_t t0, int64_t t1, const std::vector<char>& tc, int64_t& ws) {
     const int64_t g0 = (int64_t)P.hp_tc_groups.size();
-    std::map<std::tuple<int, int64_t, int, int, int>, int64_t> open, img;
+    std::map<std::tuple<int, int64_t, int, int, int, int>, int64_t> open, img;
     for (int64_t t = t0; t < t1; ++t) {
       if (!tc[t - t0]) continue;
       const Plan::SHP& h = P.hp[t];
-      const auto key = std::make_tuple(h.A.buf, h.A.off, h.before, h.a, h.after);
-      auto it = open.find(key);
-      if (it == open.end() || P.hp_tc_groups[it->second].n >= std::min(kHpTcMembers, 128 / h.a)) {
-        Plan::SHpTcGroup g;
-        g.A = h.A;
-        g.before = h.before;
-        g.a = h.a;
-        g.after = h.after;
-        const int ap = (h.a + 7) & ~7, kc = hp_tc_kc(ap);
-        g.nchunks = (int)(((int64_t)h.before * h.after + kc - 1) / kc);
-        const int64_t gi = (int64_t)P.hp_tc_groups.size();
-        auto im = img.find(key);
-        if (im == img.end()) {  // this group's pre-pass writes A's images
-          g.img = stage_oz_;
-          stage_oz_ += g.nchunks * hp_tc_chunk_bytes(ap, kc / 16);
-          img[key] = g.img;
-          for (int c = 0; c < g.nchunks; ++c) P.hp_tc_imgs.push_back(make_int2((int)gi, c));
-        } else {
-          g.img = im->second;
+      // one group per column block (a > 64: two, with one member each)
+      for (int cb = 0; cb < tc_blocks(h.a); ++cb) {
+        const auto key = std::make_tuple(h.A.buf, h.A.off, h.before, h.a, h.after, cb);
+        auto it = open.find(key);
+        if (it == open.end() || P.hp_tc_groups[it->second].n >= std::min(kHpTcMembers, 128 / h.a)) {
+          Plan::SHpTcGroup g;
+          g.A = h.A;
+          g.before = h.before;
+          g.a = h.a;
+          g.after = h.after;
+          g.ap = tc_width(h.a);
+          g.c0 = cb * g.ap;
+          g.nc = std::min(g.ap, h.a - g.c0);
+          const int kc = hp_tc_kc(g.ap);
+          g.nchunks = (int)(((int64_t)h.before * h.after + kc - 1) / kc);
+          const int64_t gi = (int64_t)P.hp_tc_groups.size();
+          auto im = img.find(key);
+          if (im == img.end()) {  // this group's pre-pass writes A's images
+            g.img = stage_oz_;
+            stage_oz_ += g.nchunks * hp_tc_chunk_bytes(g.ap, kc / 16);
+            img[key] = g.img;
+            for (int c = 0; c < g.nchunks; ++c) P.hp_tc_imgs.push_back(make_int2((int)gi, c));
+          } else {
+            g.img = im->second;
+          }
+          g.ex = stage_oz_;  // the row exponents of this group's B, written by the items' pre-pass
+          stage_oz_ += (int64_t)g.nchunks * 128;
+          P.hp_tc_groups.push_back(g);
+          open[key] = gi;
+          it = open.find(key);
         }
-        g.ex = stage_oz_;  // the row exponents of this group's B, written by the items' pre-pass
-        stage_oz_ += (int64_t)g.nchunks * 128;
-        P.hp_tc_groups.push_back(g);
-        open[key] = gi;
-        it = open.find(key);
+        Plan::SHpTcGroup& g = P.hp_tc_groups[it->second];
+        g.member[g.n++] = (int)t;
       }
-      Plan::SHpTcGroup& g = P.hp_tc_groups[it->second];
-      g.member[g.n++] = (int)t;
     }
     const int64_t g1 = (int64_t)P.hp_tc_groups.size();
     // one chunk per item: every unit stores its partial tiles (an item of
@@ -561,10 +580,10 @@ class Builder {
     bool split = false;
     for (int64_t g = g0; g < g1; ++g) {
       const Plan::SHpTcGroup& G = P.hp_tc_groups[g];
-      const int kc = hp_tc_kc((G.a + 7) & ~7);
+      const int kc = hp_tc_kc(G.ap);
       const int cpi = 1;
       const int splits = (G.nchunks + cpi - 1) / cpi;
-      for (int m = 0; m < G.n; ++m) {
+      for (int m = 0; m < G.n && G.c0 == 0; ++m) {  // the other column blocks share the partial tiles
         Plan::SHP& h = P.hp[G.member[m]];
         h.splits = splits;
         h.kchunk = cpi * kc;
@@ -591,15 +610,17 @@ class Builder {
     units = 0;
     for (int64_t t = t0; t < t1; ++t) {
       Plan::SAcc& a = P.acc[t];
-      if (a.count < 1 || !acc_tc_eligible(a.rows, a.d, P.tune.acc)) continue;
+      if (a.count < 1 || !acc_tc_eligible(a.rows, a.d, P.tune.acc) || (a.d > kTcCols && !wide_acc)) continue;
       tc[t - t0] = 1;
       a.tc_img = stage_oz_;
-      stage_oz_ += (int64_t)a.count * hp_tc_chunk_bytes((a.d + 7) & ~7, 4);
-      for (int s = 0; s < a.count; ++s) P.acc_tc_imgs.push_back(make_int2((int)t, s));
-      for (int64_t b = 0; b * 128 < a.rows; ++b) {
-        P.acc_tc_items.push_back(make_int4((int)t, (int)b, (int)units, 0));
-        units += a.count;
-      }
+      const int nb = tc_blocks(a.d);
+      stage_oz_ += (int64_t)a.count * nb * hp_tc_chunk_bytes(tc_width(a.d), tc_steps(a.d));
+      for (int s = 0; s < a.count * nb; ++s) P.acc_tc_imgs.push_back(make_int2((int)t, s));
+      for (int64_t b = 0; b * 128 < a.rows; ++b)
+        for (int cb = 0; cb < nb; ++cb) {
+          P.acc_tc_items.push_back(make_int4((int)t, (int)b, (int)units, cb));
+          units += a.count;
+        }
     }
     int64_t w = tile0;
     for (int64_t i = tile0; i < tile1; ++i) {
@@ -662,16 +683,18 @@ class Builder {
     std::vector<char> oz(t1 - t0, 0);
     for (int64_t t = t0; t < t1; ++t) {
       auto& m = P.mp[t];
-      if (m.diag || !mp_tc_eligible(m.a_in, m.a_out, P.tune.mp)) continue;
+      const int64_t rows = (int64_t)m.before * m.after;
+      const bool beyond = wide && P.hp_tensor && mp_tc_wide(m.a_in, m.a_out, rows, P.tune.mp);
+      if (m.diag || !(beyond || mp_tc_eligible(m.a_in, m.a_out, P.tune.mp))) continue;
       oz[t - t0] = 1;
       m.oz_h = stage_oz_;
       // double-float plans: the sum-of-products kernel's image of alpha h;
       // complex64 plans: the split-TF32 image
-      stage_oz_ += P.hp_tensor ? hp_tc_chunk_bytes((m.a_out + 7) & ~7, 4) : mp_oz_h_bytes();
-      P.mp_oz_tasks.push_back((int)t);
-      const int64_t rows = (int64_t)m.before * m.after;
+      const int nb = tc_blocks(m.a_out);
+      stage_oz_ += P.hp_tensor ? nb * hp_tc_chunk_bytes(tc_width(m.a_out), tc_steps(m.a_in)) : mp_oz_h_bytes();
+      for (int cb = 0; cb < nb; ++cb) P.mp_oz_tasks.push_back((int)t | cb << kMpTcTaskShift);
       for (int64_t r = 0; r * kMpOzRows * kMpOzSub < rows; ++r)
-        P.mp_oz_tiles.push_back(make_int2((int)t, (int)r));
+        for (int cb = 0; cb < nb; ++cb) P.mp_oz_tiles.push_back(make_int2((int)t, (int)r | cb << kMpTcBlockShift));
     }
     int64_t w = tile0;
     for (int64_t i = tile0; i < tile1; ++i) {

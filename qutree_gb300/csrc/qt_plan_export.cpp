@@ -429,7 +429,7 @@ static void table(const qt::Plan& P, int what, std::vector<int64_t>& v, std::vec
             v.push_back(P.cd.xhole[m][a]);
           }
       break;
-    case 40:  // tensor-core mode-product tiles: (task, tile of kMpOzSub x kMpOzRows rows)
+    case 40:  // tensor-core mode-product tiles: (task, tile of kMpOzSub x kMpOzRows rows | column block << kMpTcBlockShift)
       for (auto& t : P.mp_oz_tiles) {
         v.push_back(t.x);
         v.push_back(t.y);
@@ -443,10 +443,10 @@ static void table(const qt::Plan& P, int what, std::vector<int64_t>& v, std::vec
         v.push_back(st.nozt);
       }
       break;
-    case 42:  // tensor-core tasks: (task, byte offset of its digits of h in B_OZ)
+    case 42:  // tensor-core tasks: (task | column block << kMpTcTaskShift, byte offset of its digits of h in B_OZ)
       for (int t : P.mp_oz_tasks) {
         v.push_back(t);
-        v.push_back(P.mp[t].oz_h);
+        v.push_back(P.mp[t & ((1 << qt::kMpTcTaskShift) - 1)].oz_h);
       }
       break;
     case 43:  // classic mode-product tiles: (task, first slot)
@@ -546,7 +546,7 @@ static void table(const qt::Plan& P, int what, std::vector<int64_t>& v, std::vec
     case 56:  // B_OZ bytes
       v.push_back(P.oz_bytes);
       break;
-    case 57:  // tensor-core accumulation items: (task, 128-row block, units before the item, 0)
+    case 57:  // tensor-core accumulation items: (task, 128-row block, units before the item, column block)
       for (auto& t : P.acc_tc_items) {
         v.push_back(t.x);
         v.push_back(t.y);
@@ -554,7 +554,7 @@ static void table(const qt::Plan& P, int what, std::vector<int64_t>& v, std::vec
         v.push_back(t.w);
       }
       break;
-    case 58:  // image pre-pass units of the accumulations: (task, term)
+    case 58:  // image pre-pass units of the accumulations: (task, term + terms x column block)
       for (auto& t : P.acc_tc_imgs) {
         v.push_back(t.x);
         v.push_back(t.y);

@@ -485,12 +485,12 @@ struct TcsArgs {
   int* status;
 };
 
-// item `it` of the launch (mode products: (task, 128-row block, 0, 0))
+// item `it` of the launch (mode products: (task, 128-row block, 0, column block))
 template <int OP>
 __device__ __forceinline__ int4 tcs_fetch(const TcsArgs& g, int64_t it) {
   if (OP == TCS_MP) {
     const int2 t = g.mp_tiles[g.item0 + it];
-    return make_int4(t.x, t.y, 0, 0);
+    return make_int4(t.x, t.y & ((1 << kMpTcBlockShift) - 1), 0, t.y >> kMpTcBlockShift);
   }
   return g.items[g.item0 + it];
 }
@@ -534,9 +534,10 @@ __device__ __forceinline__ void tcs_range(const TcsArgs& g, int64_t& i0, int64_t
   i1 = first_at(g.units * (blockIdx.x + 1) / gridDim.x);
 }
 
-// per item: padded columns np, real columns, units, 16-k steps per unit
+// per item: its column block (padded columns np, real columns, first one),
+// units, 16-k steps per unit and of the operand image
 struct TcsItem {
-  int np, ncols, nunits, nks;
+  int np, ncols, c0, nunits, nks, isteps;
   int nl;  // level accumulators
 };
 template <int OP>
@@ -545,39 +546,41 @@ __device__ __forceinline__ TcsItem tcs_item(const TcsArgs& g, int4 itm) {
   if (OP == TCS_HP) {
     const HpTcGroup& G = g.groups[itm.x];
     v.np = G.ap;
-    v.ncols = G.a;
+    v.ncols = G.nc;
+    v.c0 = G.c0;
     v.nunits = itm.w - itm.z;
-    v.nks = hp_tc_kc(G.ap) / kChunkK;
-    // 128-k chunks keep four accumulators (levels 0..2 exact up to 170 k)
-    v.nl = v.nks > 4 ? min(4, levels_for(G.ap)) : levels_for(G.ap);
-  } else if (OP == TCS_ACC) {
+    v.nks = v.isteps = hp_tc_kc(G.ap) / kChunkK;
+    // 128-k chunks keep four accumulators (levels 0..2 exact up to 170 k);
+    // column blocks of wide bonds five (levels 0..3 exact up to 128 k)
+    v.nl = v.nks > 4 ? min(G.a > kTcCols ? 5 : 4, levels_for(G.ap)) : levels_for(G.ap);
+    return v;
+  }
+  int n, k;
+  if (OP == TCS_ACC) {
     const AccTask& T = g.acc[itm.x];
-    v.np = (T.d + 7) & ~7;
-    v.ncols = T.d;
+    n = k = T.d;
     v.nunits = T.count;
-    v.nks = (T.d + kChunkK - 1) / kChunkK;
-    v.nl = levels_for(v.np);
   } else {
     const MPTask& t = g.mp[itm.x];
-    v.np = (t.a_out + 7) & ~7;
-    v.ncols = t.a_out;
+    n = t.a_out;
+    k = t.a_in;
     v.nunits = 1;
-    v.nks = (t.a_in + kChunkK - 1) / kChunkK;
-    v.nl = levels_for(v.np);
   }
+  v.np = tc_width(n);
+  v.c0 = itm.w * v.np;
+  v.ncols = min(v.np, n - v.c0);
+  v.nks = (k + kChunkK - 1) / kChunkK;
+  v.isteps = tc_steps(k);
+  // beyond 64 k (up to 112) five accumulators at most (levels 0..3 exact up to 128 k)
+  v.nl = k > 64 ? min(5, levels_for(v.np)) : levels_for(v.np);
   return v;
 }
-// image steps of a unit (the image's layout; the unit may use fewer)
 template <int OP>
-__device__ __forceinline__ int tcs_img_steps(int np) {
-  return OP == TCS_HP ? hp_tc_kc(np) / kChunkK : 4;
-}
-template <int OP>
-__device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4 itm, int u, int np) {
-  const int64_t cb = hp_tc_chunk_bytes(np, tcs_img_steps<OP>(np));
+__device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4 itm, int u, const TcsItem& I) {
+  const int64_t cb = hp_tc_chunk_bytes(I.np, I.isteps);
   if (OP == TCS_HP) return g.groups[itm.x].img + (size_t)(itm.z + u) * cb;
-  if (OP == TCS_MP) return static_cast<const unsigned char*>(g.mp[itm.x].oz_h);
-  return static_cast<const unsigned char*>(g.acc[itm.x].tc_img) + (size_t)u * cb;
+  if (OP == TCS_MP) return static_cast<const unsigned char*>(g.mp[itm.x].oz_h) + (size_t)itm.w * cb;
+  return static_cast<const unsigned char*>(g.acc[itm.x].tc_img) + (size_t)(u + I.nunits * itm.w) * cb;
 }
 
 // pre-pass: the image of W for one unit -- per 16-k step and digit a plane of
@@ -588,10 +591,38 @@ __device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4
 // MP units (task): W(j, k) = alpha h(j, k).
 template <int OP>
 __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restrict__ units, int64_t first) {
-  const int2 u = OP == TCS_MP ? make_int2(g.mp_tasks[first + blockIdx.x], 0) : units[first + blockIdx.x];
+  int2 u = OP == TCS_MP ? make_int2(g.mp_tasks[first + blockIdx.x], 0) : units[first + blockIdx.x];
   const int n = threadIdx.x & 63, q = threadIdx.x >> 6;
-  int np, ncols, steps;
+  int np, ncols, c0, steps;  // the unit's column block and image
   unsigned char* img;
+  if (OP == TCS_HP) {
+    const HpTcGroup& G = g.groups[u.x];
+    np = G.ap;
+    ncols = G.nc;
+    c0 = G.c0;
+    steps = hp_tc_kc(np) / kChunkK;
+    img = G.img + (size_t)u.y * hp_tc_chunk_bytes(np, steps);
+  } else {
+    int cb, cols, k;
+    if (OP == TCS_MP) {
+      cb = u.x >> kMpTcTaskShift;
+      u.x &= (1 << kMpTcTaskShift) - 1;
+      const MPTask& t = g.mp[u.x];
+      cols = t.a_out;
+      k = t.a_in;
+      img = static_cast<unsigned char*>(t.oz_h);
+    } else {
+      const AccTask& T = g.acc[u.x];
+      cb = u.y / T.count;
+      cols = k = T.d;
+      img = static_cast<unsigned char*>(T.tc_img);
+    }
+    np = tc_width(cols);
+    c0 = cb * np;
+    ncols = min(np, cols - c0);
+    steps = tc_steps(k);
+    img += (size_t)(OP == TCS_MP ? cb : u.y) * hp_tc_chunk_bytes(np, steps);
+  }
   // the 16 values of row n at step ks
   auto load16 = [&](int ks, float4 (&v)[16]) {
     if (OP == TCS_HP) {
@@ -602,8 +633,8 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
 #pragma unroll
       for (int kk = 0; kk < 16; ++kk) {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < G.a && k0 + kk < K) {
-          x = __ldg(A + w.off(n, G.before, G.a));
+        if (n < ncols && k0 + kk < K) {
+          x = __ldg(A + w.off(c0 + n, G.before, G.a));
           x.z = -x.z;
           x.w = -x.w;
         }
@@ -619,15 +650,15 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
       for (int kk = 0; kk < 16; ++kk) {
         const int k = ks * kChunkK + kk;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < t.a_out && k < t.a_in) {
-          x = __ldg(H + n + (int64_t)t.a_out * k);
+        if (n < ncols && k < t.a_in) {
+          x = __ldg(H + c0 + n + (int64_t)t.a_out * k);
           if (!one) x = DF64::mul(cf, x);
         }
         v[kk] = x;
       }
     } else {
       const AccTask& T = g.acc[u.x];
-      const AccTerm tm = g.terms[T.first + u.y];
+      const AccTerm tm = g.terms[T.first + u.y % T.count];
       const double2 alpha = T.alpha_ptr ? *T.alpha_ptr : T.alpha;
       const float4 cf = DF64::coef(alpha);
       const float4* __restrict__ H = reinterpret_cast<const float4*>(tm.H);
@@ -635,34 +666,14 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
       for (int kk = 0; kk < 16; ++kk) {
         const int k = ks * kChunkK + kk;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < T.d && k < T.d) {
-          if (H) x = DF64::mul(cf, __ldg(H + n + (int64_t)T.d * k));
-          else if (n == k) x = cf;
+        if (n < ncols && k < T.d) {
+          if (H) x = DF64::mul(cf, __ldg(H + c0 + n + (int64_t)T.d * k));
+          else if (c0 + n == k) x = cf;
         }
         v[kk] = x;
       }
     }
   };
-  if (OP == TCS_HP) {
-    const HpTcGroup& G = g.groups[u.x];
-    np = G.ap;
-    ncols = G.a;
-    steps = hp_tc_kc(np) / kChunkK;
-    img = G.img + (size_t)u.y * hp_tc_chunk_bytes(np, steps);
-  } else if (OP == TCS_MP) {
-    const MPTask& t = g.mp[u.x];
-    np = (t.a_out + 7) & ~7;
-    ncols = t.a_out;
-    steps = 4;
-    img = static_cast<unsigned char*>(t.oz_h);
-  } else {
-    const AccTask& T = g.acc[u.x];
-    np = (T.d + 7) & ~7;
-    ncols = T.d;
-    steps = 4;
-    img = static_cast<unsigned char*>(T.tc_img) + (size_t)u.y * hp_tc_chunk_bytes(np, steps);
-  }
-  (void)ncols;
   __shared__ int fx[64];  // largest |W| of a row as an integer, then its exponent
   if (threadIdx.x < 64) fx[threadIdx.x] = 0;
   __syncthreads();
@@ -974,7 +985,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         }
         sm.ex[buf][r] = (uint8_t)eb;
         mbar_arrive(&sm.bar.exready[buf]);
-        const unsigned char* img = tcs_image<OP>(g, itm, u, I.np);
+        const unsigned char* img = tcs_image<OP>(g, itm, u, I);
         float4 nx[8];
         load8(nx, 0, 0);
         for (int ks = 0; ks < I.nks; ++ks, ++q) {
@@ -1117,6 +1128,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         stride = t.before;
         add_first = t.add != 0;
       }
+      if (base) base += stride * I.c0;
       for (int u = 0; u < I.nunits; ++u, ++un) {
         const int buf = (int)(un & 1);
         const bool store = u == 0 && !add_first;
@@ -1129,8 +1141,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         fence_after_sync();
         const int er = (int)sm.ex[buf][r];
         mbar_arrive(&sm.bar.exfree[buf]);
-        const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, u, np) +
-                                                      (size_t)tcs_img_steps<OP>(np) * kDig * 3 * np * 32);
+        const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, u, I) +
+                                                      (size_t)I.isteps * kDig * 3 * np * 32);
         const int f0 = __ldg(fxg + lane), f1 = __ldg(fxg + 32 + lane);
         __syncwarp();
         fxw[lane] = f0 << 23;
