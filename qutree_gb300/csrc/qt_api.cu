@@ -1740,9 +1740,9 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
     for (int x : g.shape) maxd = std::max(maxd, x);
   }
   const int64_t vstride = (maxN + 15) / 16 * 16, mstride = (int64_t)maxd * maxd;
-  // vectors V_0..V_{K-1}, W, Y, T, U; matrices S, H, R; dot scratch; hole-product partial tiles
+  // vectors V_0..V_{K-1}, W, Y, T; matrices S, H, R; dot scratch; hole-product partial tiles
   const int64_t ws_elems = 64 * mstride;
-  const int64_t total = (n_krylov + 4) * vstride + 3 * mstride + 512 + ws_elems;
+  const int64_t total = (n_krylov + 3) * vstride + 3 * mstride + 512 + ws_elems;
   DevFree work;
   {
     cudaError_t e = dev_malloc(&work.p, total * sizeof(cd));
@@ -1753,8 +1753,7 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
   cd* W = V(n_krylov);
   cd* Y = V(n_krylov + 1);
   cd* T = V(n_krylov + 2);
-  cd* U = V(n_krylov + 3);  // complex128 copy of H v (double-float plans)
-  cd* dS = base + (n_krylov + 4) * vstride;
+  cd* dS = base + (n_krylov + 3) * vstride;
   cd* dH = dS + mstride;
   cd* dR = dH + mstride;
   cd* dscal = dR + mstride;
@@ -1766,7 +1765,6 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
   cd* psi_ar = c->buf[qt::B_PSI];
   cd* kin = c->buf[qt::B_KRY] + P.kry_in;
   cd* kout = c->buf[qt::B_KRY] + P.kry_out;
-  cd* hv = df ? U : kout;  // H v in complex128
   auto to_arith = [&](cd* dst, const cd* src, int64_t n) -> int {
     cudaError_t e = qt::launch_convert(dst, src, n, 0, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "qt_scf convert");
@@ -1844,48 +1842,46 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
       const int64_t N = g.N;
       cd* pa = psi + g.aoff;
       int size = (int)std::min<int64_t>(n_krylov, N);
-      // Lanczos on the effective Hamiltonian (solveKrylovSpace)
+      // Lanczos on the effective Hamiltonian (solveKrylovSpace): the whole
+      // recursion is enqueued, its scalars come back with one wait
       std::vector<double> al, be;
-      cd s;
-      if ((rc = dot(pa, pa, N, s)) != QT_OK) return rc;
-      if (!(s.x > 0.0) || !std::isfinite(s.x)) return fail(c, QT_ERR_NUMERIC, "qt_scf: zero or non-finite node tensor");
-      if ((rc = lincomb(V(0), {{pa, cmk(1.0 / std::sqrt(s.x), 0)}}, N)) != QT_OK) return rc;
-      for (int l = 0; l < size; ++l) {
-        if (df) {
-          if ((rc = to_arith(kin, V(l), N)) != QT_OK) return rc;
-        } else {
-          QT_CUDA(c, cudaMemcpyAsync(kin, V(l), N * sizeof(cd), cudaMemcpyDeviceToDevice, c->stream));
-        }
-        if ((rc = run_stages(c, P.scf_apply_b[a], P.scf_apply_e[a])) != QT_OK) return rc;
-        if (df) {
-          cudaError_t e = qt::launch_convert(U, kout, N, 1, c->stream);
-          if (e != cudaSuccess) return cuda_fail(c, e, "qt_scf convert");
-          c->launches += 1;
-        }
-        if ((rc = dot(V(l), hv, N, s)) != QT_OK) return rc;
-        if (!std::isfinite(s.x)) return fail(c, QT_ERR_NUMERIC, "qt_scf: non-finite <v|H|v>");
-        al.push_back(s.x);
-        if (l + 1 == size) break;
-        if (l == 0)
-          rc = lincomb(W, {{hv, cmk(1, 0)}, {V(0), cmk(-al[0], 0)}}, N);
-        else
-          rc = lincomb(W, {{hv, cmk(1, 0)}, {V(l), cmk(-al[l], 0)}, {V(l - 1), cmk(-be[l - 1], 0)}}, N);
-        if (rc != QT_OK) return rc;
-        if ((rc = dot(W, W, N, s)) != QT_OK) return rc;
-        const double nrm = std::sqrt(std::max(s.x, 0.0));
-        if (!std::isfinite(nrm)) return fail(c, QT_ERR_NUMERIC, "qt_scf: non-finite Lanczos residual");
-        // an invariant subspace: the residual is rounding noise (the reference
-        // divides by it); the Lanczos space ends here
-        double scale = 0.0;
-        for (double x : al) scale = std::max(scale, std::fabs(x));
-        for (double x : be) scale = std::max(scale, x);
-        if (nrm <= kLanczosBreakdown * scale) {
-          size = l + 1;
-          break;
-        }
-        be.push_back(nrm);
-        if ((rc = lincomb(V(l + 1), {{W, cmk(1.0 / nrm, 0)}}, N)) != QT_OK) return rc;
+      double* dres = reinterpret_cast<double*>(dscal);
+      qt::LanczosStep lz;
+      lz.df = df ? 1 : 0;
+      lz.n = N;
+      lz.w = W;
+      lz.kin = kin;
+      lz.kout = kout;
+      lz.res = dres;
+      lz.breakdown = kLanczosBreakdown;
+      for (int l = -1; l < size; ++l) {
+        lz.l = l;
+        lz.last = l + 1 == size ? 1 : 0;
+        lz.v = l < 0 ? pa : V(l);
+        lz.prev = l > 0 ? V(l - 1) : nullptr;
+        lz.next = l + 1 < size ? V(l + 1) : nullptr;
+        if (l >= 0 && (rc = run_stages(c, P.scf_apply_b[a], P.scf_apply_e[a])) != QT_OK) return rc;
+        cudaError_t e = qt::launch_lanczos(lz, c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "qt_scf Lanczos step");
+        c->launches += 1;
       }
+      double hres[qt::kLzScalars];
+      QT_CUDA(c, cudaMemcpyAsync(hres, dres, sizeof(hres), cudaMemcpyDeviceToHost, c->stream));
+      QT_CUDA(c, cudaStreamSynchronize(c->stream));
+      if (!(hres[qt::kLzNorm2] > 0.0) || !std::isfinite(hres[qt::kLzNorm2]))
+        return fail(c, QT_ERR_NUMERIC, "qt_scf: zero or non-finite node tensor");
+      // an invariant subspace: the residual is rounding noise (the reference
+      // divides by it); the Lanczos space ended there
+      if (hres[qt::kLzStop] != 0.0) size = (int)hres[qt::kLzStop];
+      for (int l = 0; l < size; ++l) {
+        if (!std::isfinite(hres[l])) return fail(c, QT_ERR_NUMERIC, "qt_scf: non-finite <v|H|v>");
+        al.push_back(hres[l]);
+        if (l + 1 == size) break;
+        if (!std::isfinite(hres[qt::kLzBeta + l]))
+          return fail(c, QT_ERR_NUMERIC, "qt_scf: non-finite Lanczos residual");
+        be.push_back(hres[qt::kLzBeta + l]);
+      }
+      cd s;
       std::vector<double> E, U;
       tridiag_eigh(al, be, size, E, U);
       if (ritz) ritz[nritz] = E[0];

@@ -726,6 +726,24 @@ struct LinComb {
   int count;
 };
 cudaError_t launch_dot(const double2* a, const double2* b, int64_t n, double2* out, cudaStream_t s);
+// one step of the Lanczos recursion (k_lanczos); the scalars in res:
+// al_l at l, be_l at kLzBeta + l, the size of an invariant space (0: none),
+// |psi|^2 of the start
+constexpr int kLzBeta = 32, kLzStop = 64, kLzNorm2 = 65, kLzScalars = 66;
+struct LanczosStep {
+  int l, last, df;      // l = -1: start; last: only al_l; df: kin and kout in the float4 layout
+  int parts;            // set by the launch
+  int64_t n, slice;
+  const double2* v;     // V_l (start: psi)
+  const double2* prev;  // V_{l-1}, or nullptr
+  double2* next;        // V_{l+1}
+  double2* w;           // work vector
+  void* kin;
+  const void* kout;
+  double* res;
+  double breakdown;
+};
+cudaError_t launch_lanczos(const LanczosStep& step, cudaStream_t s);
 // complex128 <-> double-float copy (dir 0: to double-float)
 cudaError_t launch_convert(void* dst, const void* src, int64_t n, int dir, cudaStream_t s);
 cudaError_t launch_lincomb(double2* out, const LinComb& lc, int64_t n, cudaStream_t s);

@@ -1340,6 +1340,152 @@ __global__ void __launch_bounds__(kThreads) k_convert(void* __restrict__ dst, co
   }
 }
 
+// One step of the Lanczos recursion of the SCF driver, its scalars on the
+// device: l < 0 starts it (V_0 = psi / |psi|), l >= 0 takes h = H V_l
+// (LanczosStep::kout, in the plan's arithmetic) and forms
+//   al_l = Re <V_l, h>,  w = h - al_l V_l - be_{l-1} V_{l-1},  be_l = |w|,
+//   V_{l+1} = w / be_l,
+// the last step (l + 1 == size) only al_l.  The new vector also goes to the
+// effective Hamiltonian's input kin.  A residual below `breakdown` times the
+// largest |al|, be ends the space (res[kLzStop] = l + 1; later steps return at
+// once).  A cluster of up to eight CTAs; every dot product is summed as
+// k_dot_part and k_dot do it (slices of 8192 or more by 512 threads and a
+// tree, then a tree over the slices), slices shared out over the CTAs, the
+// partial sums read through distributed shared memory.  One launch in place
+// of eight with two waits of the host between them; per step 80 us of an
+// 8-mode tree's ~110 went there.
+__device__ __forceinline__ double ld_cluster_d(const double* p, uint32_t rank) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(a), "r"(rank));
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];\n" : "=d"(v) : "r"(ra) : "memory");
+  return v;
+}
+__device__ __forceinline__ double lz_tree(double v, double* red) {
+  red[threadIdx.x] = v;
+  __syncthreads();
+  for (int w = kDotThreads / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  const double r = red[0];
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kDotThreads) k_lanczos(LanczosStep t, int cl) {
+  __shared__ double red[kDotThreads];
+  __shared__ double part[2][kDotParts];
+  if (t.l >= 0 && t.res[kLzStop] != 0.0) return;  // the same in every CTA
+  const int rank = cl > 1 ? (int)cluster_rank() : 0;
+  // the sum over all slices of each thread's running products (sum(i)), in two stages
+  auto dot = [&](int which, auto sum) {
+    for (int p = rank; p < t.parts; p += cl) {
+      const int64_t lo = p * t.slice, hi = min(t.n, lo + t.slice);
+      double acc = 0.0;
+      for (int64_t i = lo + threadIdx.x; i < hi; i += kDotThreads) sum(i, acc);
+      const double v = lz_tree(acc, red);
+      if (threadIdx.x == 0) part[which][p / cl] = v;
+    }
+    if (cl > 1) cluster_sync();
+    else __syncthreads();
+    const int p = threadIdx.x;
+    double v = 0.0;
+    if (p < t.parts) v = cl > 1 ? ld_cluster_d(&part[which][p / cl], (uint32_t)(p % cl)) : part[which][p];
+    return lz_tree(v, red);
+  };
+  auto each = [&](auto f) {
+    for (int p = rank; p < t.parts; p += cl) {
+      const int64_t lo = p * t.slice, hi = min(t.n, lo + t.slice);
+      for (int64_t i = lo + threadIdx.x; i < hi; i += kDotThreads) f(i);
+    }
+  };
+  auto emit = [&](int64_t i, double2 v) {  // the new Krylov vector, also as the input of the next product
+    t.next[i] = v;
+    if (t.df) {
+      const float2 r = df_split(v.x), m = df_split(v.y);
+      reinterpret_cast<float4*>(t.kin)[i] = make_float4(r.x, r.y, m.x, m.y);
+    } else {
+      reinterpret_cast<double2*>(t.kin)[i] = v;
+    }
+  };
+  auto add2 = [](double& acc, double2 a, double2 b) { acc = fma(a.y, b.y, fma(a.x, b.x, acc)); };
+  const bool writer = rank == 0 && threadIdx.x == 0;
+  if (t.l < 0) {
+    const double s = dot(0, [&](int64_t i, double& acc) { add2(acc, t.v[i], t.v[i]); });
+    const double c = 1.0 / sqrt(s);
+    each([&](int64_t i) { emit(i, make_double2(c * t.v[i].x, c * t.v[i].y)); });
+    if (writer) {
+      t.res[kLzStop] = 0.0;
+      t.res[kLzNorm2] = s;
+    }
+  } else {
+    const double al = dot(0, [&](int64_t i, double& acc) {
+      double2 h;
+      if (t.df) {
+        const float4 f = reinterpret_cast<const float4*>(t.kout)[i];
+        h = make_double2((double)f.x + (double)f.y, (double)f.z + (double)f.w);
+      } else {
+        h = reinterpret_cast<const double2*>(t.kout)[i];
+      }
+      t.w[i] = h;
+      add2(acc, t.v[i], h);
+    });
+    if (writer) t.res[t.l] = al;
+    if (!t.last) {
+      const double be = t.prev ? t.res[kLzBeta + t.l - 1] : 0.0;
+      const double s = dot(1, [&](int64_t i, double& acc) {
+        double2 w = t.w[i];
+        const double2 v = t.v[i];
+        w.x = fma(-al, v.x, w.x);
+        w.y = fma(-al, v.y, w.y);
+        if (t.prev) {
+          const double2 u = t.prev[i];
+          w.x = fma(-be, u.x, w.x);
+          w.y = fma(-be, u.y, w.y);
+        }
+        t.w[i] = w;
+        add2(acc, w, w);
+      });
+      const double nrm = sqrt(fmax(s, 0.0));
+      double scale = fabs(al);
+      for (int q = 0; q < t.l; ++q) scale = fmax(scale, fmax(fabs(t.res[q]), t.res[kLzBeta + q]));
+      const bool stop = nrm <= t.breakdown * scale;
+      if (writer) {
+        t.res[kLzBeta + t.l] = s == s ? nrm : s;  // fmax drops a NaN
+        if (stop) t.res[kLzStop] = t.l + 1;
+      }
+      if (!stop) {
+        const double c = 1.0 / nrm;
+        each([&](int64_t i) { emit(i, make_double2(c * t.w[i].x, c * t.w[i].y)); });
+      }
+    }
+  }
+  if (cl > 1) cluster_sync();  // no CTA leaves while its partial sums are being read
+}
+
+cudaError_t launch_lanczos(const LanczosStep& step, cudaStream_t s) {
+  LanczosStep t = step;
+  // the slices of launch_dot
+  int64_t parts = std::min<int64_t>(kDotParts, std::max<int64_t>(1, (t.n + 8191) / 8192));
+  t.slice = (t.n + parts - 1) / parts;
+  t.parts = (int)std::max<int64_t>(1, (t.n + t.slice - 1) / t.slice);
+  int cl = 1;
+  while (cl < 8 && cl < t.parts) cl *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cl);
+  cfg.blockDim = dim3(kDotThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_lanczos, t, cl);
+}
+
 cudaError_t launch_convert(void* dst, const void* src, int64_t n, int dir, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const int blocks = (int)std::min<int64_t>((n + kThreads - 1) / kThreads, 152 * 8);
