@@ -925,17 +925,19 @@ int qt_psi_load(qt_ctx* c, const char* path) {
 }
 
 namespace {
-// kernel launches of stages [b0, b1): a hole-product stage one per tile
-// shape, two for its tensor-core items (image pre-pass and products), one
+// kernel launches of stages [b0, b1): a hole-product stage one per class of
+// tile shapes, two for its tensor-core items (image pre-pass and products), one
 // for the partial sums of split tasks; a mode-product stage one for its
 // FP32-pipe tiles and two for its tensor-core tiles (pre-pass and products)
 int64_t kernels_in(const qt::Plan& P, int64_t b0, int64_t b1) {
   int64_t n = 0;
   for (int64_t i = b0; i < b1; ++i) {
     const qt::Stage& st = P.stages[i];
-    if (st.kind == qt::ST_HP)
-      n += st.nseg + (st.nhti > 0 ? (st.nhtu > 0 ? 3 : 2) : 0) + (st.aux ? 1 : 0);
-    else if (st.kind == qt::ST_MP)
+    if (st.kind == qt::ST_HP) {
+      bool cls[3] = {false, false, false};
+      for (int g = st.seg0; g < st.seg0 + st.nseg; ++g) cls[qt::hp_class(P.hp_segs[g].x, P.hp_segs[g].y)] = true;
+      n += cls[0] + cls[1] + cls[2] + (st.nhti > 0 ? (st.nhtu > 0 ? 3 : 2) : 0) + (st.aux ? 1 : 0);
+    } else if (st.kind == qt::ST_MP)
       n += (st.n_tiles > 0 ? 1 : 0) + (st.noz > 0 ? (st.nozt > 0 ? 2 : 1) : 0);
     else if (st.kind == qt::ST_ACC)
       n += (st.n_tiles > 0 ? 1 : 0) + (st.nati > 0 ? (st.natu > 0 ? 2 : 1) : 0);

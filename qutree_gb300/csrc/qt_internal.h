@@ -714,6 +714,8 @@ inline void hp_shape(int m, int* rows, int* cols) {
       }
     }
 }
+// launch class of a register-tile shape: the shapes of one class share a launch
+inline int hp_class(int rows, int cols) { return rows == 1 ? 0 : rows * cols <= 9 ? 1 : 2; }
 // One complex128 hole product split over its reduction index (partial tiles
 // in ws, at most ws_elems elements); S written in full.
 cudaError_t launch_hp_split(const HPTask& task, double2* ws, int64_t ws_elems, cudaStream_t s);

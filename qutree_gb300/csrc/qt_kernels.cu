@@ -36,6 +36,17 @@ __device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) { cfma6
 __device__ __forceinline__ void cfmac(double2& acc, double2 a, double2 b) { cfmac64(acc, a, b); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return cadd64(a, b); }
 
+__device__ __forceinline__ void shfl_from(double2& v, int src) {
+  v.x = __shfl_sync(0xffffffffu, v.x, src & 31);
+  v.y = __shfl_sync(0xffffffffu, v.y, src & 31);
+}
+__device__ __forceinline__ void shfl_from(float4& v, int src) {
+  v.x = __shfl_sync(0xffffffffu, v.x, src & 31);
+  v.y = __shfl_sync(0xffffffffu, v.y, src & 31);
+  v.z = __shfl_sync(0xffffffffu, v.z, src & 31);
+  v.w = __shfl_sync(0xffffffffu, v.w, src & 31);
+}
+
 // ---------------------------------------------------------------------------
 // Mode-k product (matvec / matrixTensor).  A slot is (b, j0..j0+3, c): up to
 // four outputs that share the input fiber in[b, :, c].  A thread takes NJ of
@@ -379,13 +390,32 @@ __device__ __forceinline__ void hp_split_tile(const HPTask& t, const int4 tl, ty
     }
 }
 
-template <class P, int R, int C>
-__global__ void __launch_bounds__(kThreads, R * C > 9 ? 2 : 3)
+// The register-tile shapes in three classes (hp_class) of about equal registers (rows x
+// cols 1 x 1..4; 2 x 3, 2 x 4, 3 x 3; 3 x 4, 4 x 4): a stage's tiles of one
+// class share a launch, so that the shapes of uneven bonds run side by side.
+// One launch per shape, one after another with about two blocks per SM each,
+// took 5.1 ms of a sweep of 64 uneven trees (bonds 6..24), 4.0 together.
+template <class P, int CLASS>
+__global__ void __launch_bounds__(kThreads, CLASS == 2 ? 2 : 3)
     k_hp(const HPTask* __restrict__ tasks, const int4* __restrict__ tiles, int64_t tile0,
          typename P::S* __restrict__ ws) {
   const int4 tl = tiles[tile0 + blockIdx.x];
   const HPTask t = tasks[tl.x];
-  hp_split_tile<P, R, C>(t, tl, ws);
+  if (CLASS == 0) {
+    switch (t.cols) {
+      case 1: hp_split_tile<P, 1, 1>(t, tl, ws); break;
+      case 2: hp_split_tile<P, 1, 2>(t, tl, ws); break;
+      case 3: hp_split_tile<P, 1, 3>(t, tl, ws); break;
+      default: hp_split_tile<P, 1, 4>(t, tl, ws);
+    }
+  } else if (CLASS == 1) {
+    if (t.rows == 3) hp_split_tile<P, 3, 3>(t, tl, ws);
+    else if (t.cols == 3) hp_split_tile<P, 2, 3>(t, tl, ws);
+    else hp_split_tile<P, 2, 4>(t, tl, ws);
+  } else {
+    if (t.rows == 3) hp_split_tile<P, 3, 4>(t, tl, ws);
+    else hp_split_tile<P, 4, 4>(t, tl, ws);
+  }
 }
 
 // one task passed by value: block b covers output tile b % ntiles, range b / ntiles
@@ -589,66 +619,80 @@ __global__ void __launch_bounds__(kThreads) k_acc_few(const AccTask* __restrict_
   }
 }
 
-// out = sum_t c_t M_t (d x d), one block per output matrix.
+// out = sum_t c_t M_t (d x d), one element per thread; blockIdx.y is the
+// block of 256 elements.  A chain of `count` dependent sums per element: with
+// one block per matrix (16 elements a thread at d = 64) the ten stages of
+// the 64-mode sweep took 390 us, 122 this way.
 template <class P>
 __global__ void __launch_bounds__(kThreads) k_lin(const LinTask* __restrict__ tasks,
                                                   const LinTerm* __restrict__ terms, int64_t task0) {
   typedef typename P::S S;
   const LinTask t = tasks[task0 + blockIdx.x];
-  const int dd = t.d * t.d;
-  S* out = reinterpret_cast<S*>(t.out);
-  for (int e = threadIdx.x; e < dd; e += kThreads) {
-    typename P::A acc = P::zero();
-    for (int s = 0; s < t.count; ++s) {
-      const LinTerm T = terms[t.first + s];
-      P::cmac(acc, P::coef(T.c), P::ld(reinterpret_cast<const S*>(T.M) + e));
-      P::norm(acc);
-    }
-    out[e] = P::fin(acc);
+  const int e = (int)blockIdx.y * kThreads + threadIdx.x;
+  if (e >= t.d * t.d) return;
+  typename P::A acc = P::zero();
+#pragma unroll 4
+  for (int s = 0; s < t.count; ++s) {
+    const LinTerm T = terms[t.first + s];
+    P::cmac(acc, P::coef(T.c), P::ld(reinterpret_cast<const S*>(T.M) + e));
+    P::norm(acc);
   }
+  reinterpret_cast<S*>(t.out)[e] = P::fin(acc);
 }
 
-// out(i, j) = sum_t sum_k A_t(i, k) op(B_t)(k, j), one output element per
-// thread, 256 per block (tiles of the task list).
+// out(i, j) = sum_t sum_k A_t(i, k) op(B_t)(k, j).  A block owns 8 x 8
+// outputs: warp w column 8 bj + w, lane l row 8 bi + (l & 7), lane group
+// q = l >> 3 the indices k = q mod 4.  So a chain is a quarter of the terms'
+// steps (a node's projected matrix sums all its terms: 150 x 64 steps on the
+// 64-mode tree), and the block reads each 128-byte piece of A and B once for
+// eight outputs.  A tile of the table (256 outputs) stands for up to kMmBlocks
+// blocks; the planner puts the longest sums first.  One output and all four k
+// groups per thread, nodes in address order (the longest sums last): 720 us on
+// the 64-mode sweep; 405 this way.
+constexpr int kMmBlocks = 6;  // >= ceil(d/8)^2 / ceil(d^2/256) for d <= kHpMaxDim
 template <class P>
 __global__ void __launch_bounds__(kThreads) k_mm(const MMTask* __restrict__ tasks, const MMTerm* __restrict__ terms,
                                                  const int2* __restrict__ tiles, int64_t tile0) {
   typedef typename P::S S;
   const int2 tl = tiles[tile0 + blockIdx.x];
   const MMTask t = tasks[tl.x];
-  const int d = t.d;
-  const int e = tl.y + threadIdx.x;
-  if (e >= d * d) return;
-  const int i = e % d, j = e / d;
-  // four independent accumulators over k mod 4 (instruction-level parallelism)
-  typename P::A acc[4] = {P::zero(), P::zero(), P::zero(), P::zero()};
+  const int d = t.d, nb = (d + 7) >> 3, blk = (tl.y >> 8) * kMmBlocks + (int)blockIdx.y;
+  if (blk >= nb * nb) return;
+  const int lane = threadIdx.x & 31, q = lane >> 3;
+  const int oi = 8 * (blk % nb) + (lane & 7), oj = 8 * (blk / nb) + (int)(threadIdx.x >> 5);
+  if (oj >= d) return;  // the whole warp
+  const int i = min(oi, d - 1);
+  typename P::A acc = P::zero();
   const int64_t bs = t.trans_b ? d : 1;  // B element (k, j): B[j + d k] or B[k + d j]
+  const int64_t sa = 4 * (int64_t)d, sb = 4 * bs;
   for (int s = 0; s < t.count; ++s) {
     const MMTerm T = terms[t.first + s];
-    const S* A = reinterpret_cast<const S*>(T.A) + i;
-    const S* B = reinterpret_cast<const S*>(T.B) + (t.trans_b ? j : (int64_t)d * j);
+    const S* A = reinterpret_cast<const S*>(T.A) + i + (int64_t)d * q;
+    const S* B = reinterpret_cast<const S*>(T.B) + (t.trans_b ? oj : (int64_t)d * oj) + bs * q;
     int k = 0;
+#pragma unroll 4
     for (; k + 3 < d; k += 4) {
-      S a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[q] = P::ld(A + (int64_t)d * (k + q));
-        b[q] = P::ld(B + bs * (k + q));
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) P::mac(acc[q], a[q], b[q]);
-      if (k & 4) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) P::norm(acc[q]);
-      }
+      P::mac(acc, P::ld(A), P::ld(B));
+      A += sa;
+      B += sb;
+      if (k & 4) P::norm(acc);
     }
-    for (; k < d; ++k) P::mac(acc[0], P::ld(A + (int64_t)d * k), P::ld(B + bs * k));
-#pragma unroll
-    for (int q = 0; q < 4; ++q) P::norm(acc[q]);
+    if (q == 0)
+      for (; k < d; ++k) {
+        P::mac(acc, P::ld(A), P::ld(B));
+        A += d;
+        B += bs;
+      }
+    P::norm(acc);
   }
+  const S f = P::fin(acc);
 #pragma unroll
-  for (int q = 1; q < 4; ++q) P::add(acc[0], P::fin(acc[q]));
-  reinterpret_cast<S*>(t.out)[e] = P::fin(acc[0]);
+  for (int o = 1; o < 4; ++o) {
+    S v = f;
+    shfl_from(v, lane + 8 * o);
+    if (q == 0) P::add(acc, v);
+  }
+  if (q == 0 && oi < d) reinterpret_cast<S*>(t.out)[oi + d * oj] = P::fin(acc);
 }
 
 // Energy-gradient preparation: M3 = Eout - E rho per node, alpha = 1/S00.
@@ -1363,12 +1407,20 @@ __device__ __forceinline__ double ld_cluster_d(const double* p, uint32_t rank) {
   return v;
 }
 __device__ __forceinline__ double lz_tree(double v, double* red) {
+  // the tree of k_dot; its last five levels within the first warp
   red[threadIdx.x] = v;
   __syncthreads();
-  for (int w = kDotThreads / 2; w > 0; w >>= 1) {
+  for (int w = kDotThreads / 2; w >= 32; w >>= 1) {
     if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
+  if (threadIdx.x < 32) {
+    double r = red[threadIdx.x];
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) r += __shfl_down_sync(0xffffffffu, r, w);
+    if (threadIdx.x == 0) red[0] = r;
+  }
+  __syncthreads();
   const double r = red[0];
   __syncthreads();
   return r;
@@ -1386,6 +1438,7 @@ __global__ void __launch_bounds__(kDotThreads) k_lanczos(LanczosStep t, int cl) 
       double acc = 0.0;
       for (int64_t i = lo + threadIdx.x; i < hi; i += kDotThreads) sum(i, acc);
       const double v = lz_tree(acc, red);
+      if (t.parts == 1) return v;  // (one CTA)
       if (threadIdx.x == 0) part[which][p / cl] = v;
     }
     if (cl > 1) cluster_sync();
@@ -1610,31 +1663,13 @@ cudaError_t probe_fp64_peak(cudaStream_t s, double* tflops) {
   return cudaGetLastError();
 }
 
-template <class P, int R, int C>
-cudaError_t launch_hp_rc(const HPTask* tasks, const int4* tiles, int64_t first, int64_t n,
-                         typename P::S* ws, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_hp<P, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHpSmem);
+template <class P, int CLASS>
+cudaError_t launch_hp_class(const HPTask* tasks, const int4* tiles, int64_t first, int64_t n, typename P::S* ws,
+                            cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(k_hp<P, CLASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHpSmem);
   if (e != cudaSuccess) return e;
-  k_hp<P, R, C><<<(unsigned)n, kThreads, kHpSmem, s>>>(tasks, tiles, first, ws);
+  k_hp<P, CLASS><<<(unsigned)n, kThreads, kHpSmem, s>>>(tasks, tiles, first, ws);
   return cudaSuccess;
-}
-
-// the micro-tile shapes the planner chooses (rows x cols of outputs per thread)
-template <class P>
-cudaError_t launch_hp_shape(int rows, int cols, const HPTask* tasks, const int4* tiles, int64_t first,
-                            int64_t n, typename P::S* ws, cudaStream_t s) {
-  switch (rows * 8 + cols) {
-    case 1 * 8 + 1: return launch_hp_rc<P, 1, 1>(tasks, tiles, first, n, ws, s);
-    case 1 * 8 + 2: return launch_hp_rc<P, 1, 2>(tasks, tiles, first, n, ws, s);
-    case 1 * 8 + 3: return launch_hp_rc<P, 1, 3>(tasks, tiles, first, n, ws, s);
-    case 1 * 8 + 4: return launch_hp_rc<P, 1, 4>(tasks, tiles, first, n, ws, s);
-    case 2 * 8 + 3: return launch_hp_rc<P, 2, 3>(tasks, tiles, first, n, ws, s);
-    case 2 * 8 + 4: return launch_hp_rc<P, 2, 4>(tasks, tiles, first, n, ws, s);
-    case 3 * 8 + 3: return launch_hp_rc<P, 3, 3>(tasks, tiles, first, n, ws, s);
-    case 3 * 8 + 4: return launch_hp_rc<P, 3, 4>(tasks, tiles, first, n, ws, s);
-    case 4 * 8 + 4: return launch_hp_rc<P, 4, 4>(tasks, tiles, first, n, ws, s);
-    default: return cudaErrorInvalidValue;
-  }
 }
 
 template <int R, int C>
@@ -1995,9 +2030,16 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       break;
     case ST_HP: {
       typedef typename P::S S;
-      for (int g = st.seg0; g < st.seg0 + st.nseg; ++g) {
-        const int4 sg = t.hp_segs[g];
-        cudaError_t e = launch_hp_shape<P>(sg.x, sg.y, t.hp, t.hp_tiles, sg.z, sg.w, reinterpret_cast<S*>(t.hp_ws), s);
+      // the segments (one register-tile shape each) lie class by class
+      for (int g = st.seg0; g < st.seg0 + st.nseg;) {
+        const int cls = hp_class(t.hp_segs[g].x, t.hp_segs[g].y);
+        const int64_t first = t.hp_segs[g].z;
+        int64_t n = 0;
+        for (; g < st.seg0 + st.nseg && hp_class(t.hp_segs[g].x, t.hp_segs[g].y) == cls; ++g) n += t.hp_segs[g].w;
+        S* ws = reinterpret_cast<S*>(t.hp_ws);
+        cudaError_t e = cls == 0   ? launch_hp_class<P, 0>(t.hp, t.hp_tiles, first, n, ws, s)
+                        : cls == 1 ? launch_hp_class<P, 1>(t.hp, t.hp_tiles, first, n, ws, s)
+                                   : launch_hp_class<P, 2>(t.hp, t.hp_tiles, first, n, ws, s);
         if (e != cudaSuccess) return e;
       }
       if (st.nhti > 0) {
@@ -2028,10 +2070,12 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       }
       break;
     case ST_LIN:
-      k_lin<P><<<(unsigned)st.n_tasks, kThreads, 0, s>>>(t.lin, t.lin_terms, st.first_task);
+      // max_eig_d bounds every matrix
+      k_lin<P><<<dim3((unsigned)st.n_tasks, (unsigned)((max_eig_d * max_eig_d + kThreads - 1) / kThreads)), kThreads, 0, s>>>(
+          t.lin, t.lin_terms, st.first_task);
       break;
     case ST_MM:
-      k_mm<P><<<(unsigned)st.n_tiles, kThreads, 0, s>>>(t.mm, t.mm_terms, t.mm_tiles, st.first_tile);
+      k_mm<P><<<dim3((unsigned)st.n_tiles, kMmBlocks), kThreads, 0, s>>>(t.mm, t.mm_terms, t.mm_tiles, st.first_tile);
       break;
     case ST_EIG: {
       const int64_t sm = eig_smem_bytes(max_eig_d);

@@ -646,6 +646,18 @@ class Builder {
     int64_t atc_units = 0;
     if (kind == ST_ACC && P.hp_tensor) tile1 = acc_tensor_items(t0, t1, tile0, tile1, atc_units);
     P.oz_bytes = std::max(P.oz_bytes, stage_oz_);
+    // blocks start in table order: the longest sums first, so that none is
+    // left to run alone at the end (nodes lie bottom-up, the largest last)
+    auto longest_first = [&](auto& tiles, auto cost) {
+      std::stable_sort(tiles.begin() + tile0, tiles.begin() + tile1,
+                       [&](const auto& x, const auto& y) { return cost(x.x) > cost(y.x); });
+    };
+    if (kind == ST_MM)
+      longest_first(P.mm_tiles, [&](int t) { return (int64_t)P.mm[t].count * P.mm[t].d; });
+    else if (kind == ST_ACC)
+      longest_first(P.acc_tiles, [&](int t) { return (int64_t)P.acc[t].count * P.acc[t].d; });
+    else if (kind == ST_MP)
+      longest_first(P.mp_tiles, [&](int t) { return P.mp[t].diag ? 1 : P.mp[t].a_in; });
     const double f1 = P.stats.exec_flops;
     Stage s;
     s.flops = f1 - stage_flops_mark;
