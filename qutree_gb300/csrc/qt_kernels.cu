@@ -537,16 +537,17 @@ __global__ void __launch_bounds__(kThreads) k_acc(const AccTask* __restrict__ ta
 
 // The same with NQ = 1 or 2 of a thread's four columns (block (tile, part)),
 // for stages that would leave SMs idle.  A thread sums all terms of a node,
-// a chain of count x d steps: with one column a step is a quarter as long,
-// four times as many warps run, and the loads of four steps are in flight
-// together.  Every output is summed in the order of k_acc.
+// a chain of count x d steps, and with few warps in flight the loads' latency
+// is what a step costs: the steps run in batches of U, the next batch's loads
+// (of the next term after a term's last) in flight under the current one's
+// multiply-adds.  Every output is summed in the order of k_acc.
 template <class P, int NQ>
 __global__ void __launch_bounds__(kThreads) k_acc_few(const AccTask* __restrict__ tasks,
                                                       const AccTerm* __restrict__ terms,
                                                       const int4* __restrict__ tiles, int64_t tile0) {
   typedef typename P::S S;
   typedef typename P::A A;
-  constexpr int U = 4 / NQ;  // steps whose loads are in flight together
+  constexpr int U = 4;
   const int4 tl = tiles[tile0 + blockIdx.x];
   const AccTask t = tasks[tl.x];
   const int r = tl.y + threadIdx.x % kAccRows;
@@ -556,53 +557,77 @@ __global__ void __launch_bounds__(kThreads) k_acc_few(const AccTask* __restrict_
   if (jb >= d) return;  // the whole warp lies past the last column
   const int nq = d - jb < NQ ? d - jb : NQ;  // uniform across the warp
   const int64_t rows = t.rows;
+  const int rc = rv ? r : 0;
   A acc[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) acc[q] = P::zero();
-  for (int s = 0; s < t.count; ++s) {
-    const AccTerm T = terms[t.first + s];
-    const S* X = reinterpret_cast<const S*>(T.X) + r;
+
+  struct Batch {  // steps jp .. of term s; an identity term (H null) is one batch
+    S x[U], h[U][NQ];
+    int jp;
+    bool ident;
+  };
+  int s = 0, jp = 0;  // the next batch to load
+  AccTerm T = {nullptr, nullptr}, Tn = {nullptr, nullptr};
+  if (t.count > 0) T = terms[t.first];
+  if (t.count > 1) Tn = terms[t.first + 1];
+  auto load = [&](Batch& B) {
+    const S* X = reinterpret_cast<const S*>(T.X) + rc;
     const S* H = reinterpret_cast<const S*>(T.H);
-    if (H == nullptr) {
+    B.jp = jp;
+    B.ident = H == nullptr;
+    if (B.ident) {
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const int j = jb + q;
-        if (rv && j < d) P::add(acc[q], P::ld(X + rows * j));
-      }
-      continue;
-    }
-    const S* hrow[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) hrow[q] = H + (q < nq ? jb + q : 0);
-    int jp = 0;
-    for (; jp + U <= d; jp += U) {
-      S x[U], hv[U][NQ];
+      for (int q = 0; q < NQ; ++q) B.h[0][q] = P::ld(X + rows * (jb + (q < nq ? q : 0)));
+      jp = d;
+    } else {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        x[u] = rv ? P::ld(X + rows * (jp + u)) : P::zero();
+        const int k = jp + u < d ? jp + u : d - 1;  // past the end: loaded, not used
+        B.x[u] = P::ld(X + rows * k);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) hv[u][q] = P::ld(hrow[q] + (int64_t)d * (jp + u));
+        for (int q = 0; q < NQ; ++q) B.h[u][q] = P::ld(H + (q < nq ? jb + q : 0) + (int64_t)d * k);
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-          if (q < nq) P::mac(acc[q], hv[u][q], x[u]);
-        if ((jp + u) & 1) {
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) P::norm(acc[q]);
-        }
-      }
+      jp += U;
     }
-    for (; jp < d; ++jp) {
-      const S x = rv ? P::ld(X + rows * jp) : P::zero();
+    if (jp >= d) {
+      jp = 0;
+      ++s;
+      T = Tn;
+      if (s + 1 < t.count) Tn = terms[t.first + s + 1];
+    }
+  };
+  auto sum = [&](const Batch& B) {
+    if (B.ident) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q)
-        if (q < nq) P::mac(acc[q], P::ld(hrow[q] + (int64_t)d * jp), x);
-      if (jp & 1) {
+        if (rv && q < nq) P::add(acc[q], B.h[0][q]);
+      return;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (B.jp + u >= d) break;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (q < nq) P::mac(acc[q], B.h[u][q], B.x[u]);
+      if ((B.jp + u) & 1) {
 #pragma unroll
         for (int q = 0; q < NQ; ++q) P::norm(acc[q]);
       }
+    }
+  };
+  if (t.count > 0) {
+    Batch b0, b1;
+    load(b0);
+    for (;;) {
+      const bool more1 = s < t.count;
+      if (more1) load(b1);
+      sum(b0);
+      if (!more1) break;
+      const bool more0 = s < t.count;
+      if (more0) load(b0);
+      sum(b1);
+      if (!more0) break;
     }
   }
   const double2 alpha64 = t.alpha_ptr ? *t.alpha_ptr : t.alpha;
