@@ -459,14 +459,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_mp_tf(const MPTask* __restric
 // ---------------------------------------------------------------------------
 constexpr int kTcsNStage = kDig * 3 * 64 * 32;  // W side of one 16-k step at np = 64
 
+// Warps of the kernel: four producers; one MMA issuer and three exponent
+// warps; eight of the epilogue.
+constexpr int kTcsThreads = 512, kTcsExWarps = 3, kTcsEpWarps = 8;
+
 enum { TCS_HP = 0, TCS_ACC = 1, TCS_MP = 2 };
 
 struct TcsSmem {
   unsigned char a[2][kOzAStage];
   unsigned char n[2][kTcsNStage];
   Bars bar;
-  uint8_t ex[2][kRows];  // the row exponents of the two units in flight
-  int fx[8][64];         // the unit's column exponents, one copy per epilogue warp
+  int ex[2][kTcsExWarps][kRows];  // largest |X| of the rows of the two units in flight, per exponent warp
+  int fx[8][64];                  // the unit's column exponents, one copy per epilogue warp
 };
 static_assert(sizeof(TcsSmem) <= 232448, "shared memory of the sum-of-products kernel exceeds 227 KB");
 
@@ -849,26 +853,60 @@ __device__ __forceinline__ float4* shfl_ptr(float4* p, int src) {
   return reinterpret_cast<float4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), src));
 }
 
-// the producers' view of row r of an item: its source of X and validity
-struct TcsRow {
-  bool valid;
-  const float4* src;  // HP: B_t; ACC: unused (the term's X)
-  int64_t rg;         // ACC: row of the task
-  int j;              // HP: column of S_t
-};
-
-// Roles (416 threads): warps 0-3 produce X's digits, one thread per row of
-// the tile (each 16-k step in two halves of eight k; first the row's
-// exponent over the unit's k, then the digits step by step, the next half's
-// loads in flight); warp 4 allocates tensor memory and issues the MMAs from
-// one thread; warps 5-12 read the accumulators and update the outputs,
-// warp w reading lanes 32 (w % 4).. (tensor memory's lane quarter of its
-// sub-partition) for half (w - 5) / 4 of the columns.  Every wait is bounded:
-// a wait that runs out sets the status word, and the CTA drains its issued
-// MMAs, frees tensor memory and returns.
-constexpr int kTcsProducers = 128, kTcsEpilogue = 256;
+// Row r of an item: element k of X at src + k stride (mode products and
+// accumulations; hole products: src + b + before a c for k = b + before c), and
+// whether the row exists.  u: the accumulation's term.
 template <int OP>
-__global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
+__device__ __forceinline__ const float4* tcs_row(const TcsArgs& g, int4 itm, int u, int r, int64_t& stride) {
+  if (OP == TCS_HP) {
+    const HpTcGroup& G = g.groups[itm.x];
+    const int mi = r / G.a;
+    if (mi >= G.n) return nullptr;
+    return reinterpret_cast<const float4*>(g.hp[G.member[mi]].B) + (int64_t)G.before * (r - mi * G.a);
+  }
+  const uint32_t rg = (uint32_t)itm.y * kRows + r;  // at most 2^31 rows
+  if (OP == TCS_ACC) {
+    const AccTask& T = g.acc[itm.x];
+    stride = T.rows;
+    return rg < (uint32_t)T.rows ? reinterpret_cast<const float4*>(g.terms[T.first + u].X) + rg : nullptr;
+  }
+  // mode product: row (b, c) of the input, its k-th element at b + before (k + a_in c)
+  const MPTask& t = g.mp[itm.x];
+  stride = t.before;
+  const uint32_t before = (uint32_t)t.before;
+  if (rg >= before * (uint32_t)t.after) return nullptr;
+  const uint32_t c = rg / before;
+  return reinterpret_cast<const float4*>(t.in) + (rg - c * before) + (int64_t)t.before * t.a_in * c;
+}
+
+// the row's largest |X| from the exponent warps' shares: a third of the k each,
+// or, where a row's k are contiguous, every third row
+__device__ __forceinline__ int tcs_row_max(const int (&ex)[kTcsExWarps][kRows], int r, bool along) {
+  return along ? ex[r % kTcsExWarps][r] : max(max(ex[0][r], ex[1][r]), ex[2][r]);
+}
+
+// Roles (512 threads).
+// Warps 0-3 produce X's digits, one thread per row of the tile, each 16-k step
+// in two halves of eight k with the next half's loads in flight.
+// Warp 4 allocates tensor memory and issues the MMAs from one thread; warps
+// 5-7 find the rows' exponents of the units ahead (hole products: a pre-pass
+// does).
+// Warps 8-15 are the epilogue, warp w reading lanes 32 (w % 4).. (tensor
+// memory's lane quarter of its sub-partition) for half (w - 8) / 4 of the
+// columns: it adds a unit's levels, scales, and stores or adds to the outputs.
+// Every wait is bounded (all lanes of a warp give up together): a wait that
+// runs out sets the status word, and the CTA drains its issued MMAs, frees
+// tensor memory and returns.
+// What bounds it, per 128 x 64 unit of 64 k: a 16-k step (42 MMAs, 24 KB of W
+// and 48 KB of X's digits through shared memory) takes 4.9 k cycles, all of it
+// shared-memory bandwidth, and the epilogue 6 to 10 k cycles for each unit that
+// it holds up the next unit's MMAs.  The rows' exponents need all of X before
+// its first digit: in the producers, ahead of every unit, that pass took 9 to
+// 15 k cycles; in warps of its own it runs under the previous unit (a CTA's
+// mode products 22.1 -> 17.2 k cycles a unit; 64-mode wide sweep 41.1 -> 37.2 ms,
+// 64-mode sweep 10.5 -> 10.1 ms, 16-mode 1.72 -> 1.67 ms).
+template <int OP>
+__global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
   extern __shared__ __align__(128) unsigned char tcs_raw[];
   TcsSmem& sm = *reinterpret_cast<TcsSmem*>(tcs_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -878,13 +916,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
 
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&sm.bar.full[s], kTcsProducers);
+      mbar_init(&sm.bar.full[s], 128);
       mbar_init(&sm.bar.empty[s], 1);
-      mbar_init(&sm.bar.exready[s], kTcsProducers);
-      mbar_init(&sm.bar.exfree[s], kTcsEpilogue);
+      mbar_init(&sm.bar.exready[s], kTcsExWarps);
+      mbar_init(&sm.bar.exfree[s], 4 + kTcsEpWarps);
     }
     mbar_init(&sm.bar.tfull, 1);
-    mbar_init(&sm.bar.tempty, kTcsEpilogue);
+    mbar_init(&sm.bar.tempty, kTcsEpWarps);
     mbar_init(&sm.bar.drain, 1);
     mbar_fence_init();
   }
@@ -894,6 +932,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
   fence_after_sync();
   const uint32_t tmem = sm.bar.tmem;
   bool ok = true;
+  auto waited = [&](void* bar, uint32_t parity, int code) {  // whole warp
+    if (__all_sync(0xffffffffu, mbar_wait(bar, parity, kSpin))) return true;
+    set_status(status, code);
+    ok = false;
+    return false;
+  };
 
   if (warp < 4) {
     // ---------------- producers: one per row ----------------
@@ -903,98 +947,64 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
       const int4 itm = tcs_fetch<OP>(g, it);
       const TcsItem I = tcs_item<OP>(g, itm);
       const uint32_t nbytes = (uint32_t)(kDig * 3 * I.np * 32);
-      // row r of the item
-      TcsRow R;
-      int before = 1, a = 1, K = 0;
-      int64_t rows = 0;  // k stride of X (ACC: the task's rows; MP: before)
-      int tfirst = 0;
+      int before = 0, K = 0;
+      int64_t jump = 0;  // hole products: from the end of one run of b to the next
       if (OP == TCS_HP) {
         const HpTcGroup& G = g.groups[itm.x];
         before = G.before;
-        a = G.a;
         K = before * G.after;
-        const int mi = r / a;
-        R.j = r - mi * a;
-        R.valid = mi < G.n;
-        R.src = R.valid ? reinterpret_cast<const float4*>(g.hp[G.member[mi]].B) : nullptr;
-        R.rg = 0;
-      } else if (OP == TCS_ACC) {
-        const AccTask& T = g.acc[itm.x];
-        rows = T.rows;
-        K = T.d;
-        tfirst = T.first;
-        R.rg = (int64_t)itm.y * kRows + r;
-        R.valid = R.rg < rows;
-        R.src = nullptr;
-        R.j = 0;
+        jump = (int64_t)before * (G.a - 1);
       } else {
-        // mode product: row (b, c) of the input, its k-th element at b + before (k + a_in c)
-        const MPTask& t = g.mp[itm.x];
-        const int64_t rg = (int64_t)itm.y * kRows + r;
-        K = t.a_in;
-        rows = t.before;
-        R.valid = rg < (int64_t)t.before * t.after;
-        const int64_t b = R.valid ? rg % t.before : 0, c = R.valid ? rg / t.before : 0;
-        R.src = reinterpret_cast<const float4*>(t.in) + b + (int64_t)t.before * K * c;
-        R.rg = 0;
-        R.j = 0;
+        K = OP == TCS_ACC ? g.acc[itm.x].d : g.mp[itm.x].a_in;
       }
       for (int u = 0; u < I.nunits; ++u, ++un) {
         const int buf = (int)(un & 1);
-        const uint32_t use_par = (un >> 1) & 1;
-        const float4* X = OP != TCS_ACC ? R.src : reinterpret_cast<const float4*>(g.terms[tfirst + u].X) + R.rg;
-        const int kbase = OP == TCS_HP ? (itm.z + u) * I.nks * kChunkK : 0;
-        // the eight values of half hh of step ks: k = kbase + 16 ks + 8 hh + i
-        auto load8 = [&](float4 (&x)[8], int ks, int hh) {
-          const int k0 = kbase + ks * kChunkK + hh * 8;
-          if (OP == TCS_HP) {
-            KWalk w(min(k0, K), before);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              x[i] = (R.valid && k0 + i < K) ? __ldg(X + w.off(R.j, before, a)) : make_float4(0.f, 0.f, 0.f, 0.f);
-              w.next(before);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              x[i] = (R.valid && k0 + i < K) ? __ldg(X + rows * (k0 + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        int64_t stride = 1;
+        const float4* p = tcs_row<OP>(g, itm, u, r, stride);
+        // the row's elements in order: `left` of them, the next one at p
+        int left = 0, b = 0;
+        if (OP == TCS_HP) {
+          const int k0 = (itm.z + u) * I.nks * kChunkK, c = k0 / before;
+          b = k0 - c * before;
+          if (p) {
+            left = K - k0;
+            p += b + (jump + before) * c;
           }
+        } else if (p) {
+          left = K;
+        }
+        auto load8 = [&](float4 (&x)[8]) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            x[i] = i < left ? __ldg(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (OP == TCS_HP) {
+              ++p;
+              if (++b == before) {
+                b = 0;
+                p += jump;
+              }
+            } else {
+              p += stride;
+            }
+          }
+          left -= 8;
         };
-        // the row's largest exponent over the unit's k (hole products: from
-        // the pre-pass), eight loads in flight
+        float4 nx[8];
+        load8(nx);
         int eb;
         if (OP == TCS_HP) {
-          eb = g.groups[itm.x].ex[(size_t)(itm.z + u) * kRows + r];
+          eb = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + u) * kRows + r);
         } else {
-          int mx = 0;
-          if (R.valid)
-            for (int h8 = 0; h8 < 2 * I.nks; ++h8) {
-              float4 x[8];
-              load8(x, h8 >> 1, h8 & 1);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) mx = max(mx, max(fmag(x[i].x), fmag(x[i].z)));
-            }
-          eb = row_exponent(mx);
+          if (!waited(&sm.bar.exready[buf], (un >> 1) & 1, 18)) break;
+          eb = row_exponent(tcs_row_max(sm.ex[buf], r, OP == TCS_MP && stride == 1));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.bar.exfree[buf]);
         }
         const float rowf = row_factor(eb);
-        // the epilogue of the unit two back has read ex of this buffer
-        if (!mbar_wait(&sm.bar.exfree[buf], use_par ^ 1, kSpin)) {
-          set_status(status, 18);
-          ok = false;
-          break;
-        }
-        sm.ex[buf][r] = (uint8_t)eb;
-        mbar_arrive(&sm.bar.exready[buf]);
         const unsigned char* img = tcs_image<OP>(g, itm, u, I);
-        float4 nx[8];
-        load8(nx, 0, 0);
         for (int ks = 0; ks < I.nks; ++ks, ++q) {
           const int s = q & 1;
-          if (!mbar_wait(&sm.bar.empty[s], ((q >> 1) & 1) ^ 1, kSpin)) {
-            set_status(status, 11);
-            ok = false;
-            break;
-          }
+          if (!waited(&sm.bar.empty[s], ((q >> 1) & 1) ^ 1, 11)) break;
           if (tid == 0) {
             // W's digits of this step; the copy completes on full[s] (it
             // finishes within microseconds, before any wait could run out)
@@ -1007,29 +1017,23 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
             float4 x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = nx[i];
-            const int nk = ks + hh;  // the next half: (ks, 1) or (ks + 1, 0)
-            if (nk < I.nks) load8(nx, nk, hh ^ 1);
-            uint32_t wr[kDig][4], wi[kDig][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float d0[kDig], d1[kDig], e0[kDig], e1[kDig];
-              digits_f32(x[2 * i].x, x[2 * i].y, rowf, d0);
-              digits_f32(x[2 * i + 1].x, x[2 * i + 1].y, rowf, d1);
-              digits_f32(x[2 * i].z, x[2 * i].w, rowf, e0);
-              digits_f32(x[2 * i + 1].z, x[2 * i + 1].w, rowf, e1);
-#pragma unroll
-              for (int d = 0; d < kDig; ++d) {
-                wr[d][i] = pack_bf16(d0[d], d1[d]);
-                wi[d][i] = pack_bf16(e0[d], e1[d]);
-              }
-            }
+            if (ks + hh < I.nks) load8(nx);  // the next half: (ks, 1) or (ks + 1, 0)
             const int off = core_off(r, hh, kRows);
 #pragma unroll
-            for (int d = 0; d < kDig; ++d) {
-              *reinterpret_cast<uint4*>(As + (2 * d + 0) * kOzAPlane + off) =
-                  make_uint4(wr[d][0], wr[d][1], wr[d][2], wr[d][3]);
-              *reinterpret_cast<uint4*>(As + (2 * d + 1) * kOzAPlane + off) =
-                  make_uint4(wi[d][0], wi[d][1], wi[d][2], wi[d][3]);
+            for (int part = 0; part < 2; ++part) {
+              uint32_t w[kDig][4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                float d0[kDig], d1[kDig];
+                digits_f32(part ? x[2 * i].z : x[2 * i].x, part ? x[2 * i].w : x[2 * i].y, rowf, d0);
+                digits_f32(part ? x[2 * i + 1].z : x[2 * i + 1].x, part ? x[2 * i + 1].w : x[2 * i + 1].y, rowf, d1);
+#pragma unroll
+                for (int d = 0; d < kDig; ++d) w[d][i] = pack_bf16(d0[d], d1[d]);
+              }
+#pragma unroll
+              for (int d = 0; d < kDig; ++d)
+                *reinterpret_cast<uint4*>(As + (2 * d + part) * kOzAPlane + off) =
+                    make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
             }
           }
           fence_proxy_async();
@@ -1038,74 +1042,161 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         if (!ok) break;
       }
     }
-  } else if (warp == 4) {
-    // ---------------- MMA issue (one thread) ----------------
-    if (lane == 0) {
-      uint32_t q = 0, un = 0;
-      for (int64_t it = my0; it < my1 && ok; ++it) {
-        const int4 itm = tcs_fetch<OP>(g, it);
-        const TcsItem I = tcs_item<OP>(g, itm);
-        const int np = I.np, NL = I.nl;
-        const uint32_t id = idesc_m128(1, 2 * np, false);
-        const uint32_t lboA = (kRows / 8) * 128, lboN = (uint32_t)(3 * np / 8) * 128;
-        const uint64_t pA = kOzAPlane >> 4, pN = (uint64_t)((3 * np * 32) >> 4);
-        const uint64_t p1 = (uint64_t)((np / 8) * 128 >> 4);  // rows np..: [Wr | Wi]
-        for (int u = 0; u < I.nunits && ok; ++u, ++un) {
-          if (!mbar_wait(&sm.bar.tempty, (un & 1) ^ 1, kSpin)) {
-            set_status(status, 14);
-            ok = false;
-            break;
-          }
-          fence_after_sync();
-          for (int ks = 0; ks < I.nks; ++ks, ++q) {
-            const int s = q & 1;
-            if (!mbar_wait(&sm.bar.full[s], (q >> 1) & 1, kSpin)) {
-              set_status(status, 15);
+  } else if (warp < 8) {
+    if (warp == 4) {
+      // ---------------- MMA issue (one thread) ----------------
+      if (lane == 0) {
+        uint32_t q = 0, un = 0;
+        for (int64_t it = my0; it < my1 && ok; ++it) {
+          const int4 itm = tcs_fetch<OP>(g, it);
+          const TcsItem I = tcs_item<OP>(g, itm);
+          const int np = I.np, NL = I.nl;
+          const uint32_t id = idesc_m128(1, 2 * np, false);
+          const uint32_t lboA = (kRows / 8) * 128, lboN = (uint32_t)(3 * np / 8) * 128;
+          const uint64_t pA = kOzAPlane >> 4, pN = (uint64_t)((3 * np * 32) >> 4);
+          const uint64_t p1 = (uint64_t)((np / 8) * 128 >> 4);  // rows np..: [Wr | Wi]
+          for (int u = 0; u < I.nunits && ok; ++u, ++un) {
+            if (!mbar_wait(&sm.bar.tempty, (un & 1) ^ 1, kSpin)) {
+              set_status(status, 14);
               ok = false;
               break;
             }
             fence_after_sync();
-            const uint64_t dA = desc_kmajor(smem_u32(sm.a[s]), lboA, 128);
-            const uint64_t dN = desc_kmajor(smem_u32(sm.n[s]), lboN, 128);
-            const uint32_t first = ks == 0 ? 1u : 0u;
+            for (int ks = 0; ks < I.nks; ++ks, ++q) {
+              const int s = q & 1;
+              if (!mbar_wait(&sm.bar.full[s], (q >> 1) & 1, kSpin)) {
+                set_status(status, 15);
+                ok = false;
+                break;
+              }
+              fence_after_sync();
+              const uint64_t dA = desc_kmajor(smem_u32(sm.a[s]), lboA, 128);
+              const uint64_t dN = desc_kmajor(smem_u32(sm.n[s]), lboN, 128);
+              const uint32_t first = ks == 0 ? 1u : 0u;
 #pragma unroll
-            for (int sd = 0; sd < kDig; ++sd) {
-              const uint64_t ar = dA + (uint64_t)(2 * sd) * pA, ai = ar + pA;
+              for (int sd = 0; sd < kDig; ++sd) {
+                const uint64_t ar = dA + (uint64_t)(2 * sd) * pA, ai = ar + pA;
 #pragma unroll
-              for (int td = 0; td + sd < kDig; ++td) {
-                const int L = sd + td < NL - 1 ? sd + td : NL - 1;
-                const uint64_t nb = dN + (uint64_t)td * pN;
-                const uint32_t d = tmem + (uint32_t)(L * 2 * np);
-                const uint32_t acc = (first && sd == 0 && td == L) ? 0u : 1u;
-                mma_bf16(d, ar, nb + p1, id, acc);  // Xr x [Wr | Wi]
-                mma_bf16(d, ai, nb, id, 1);         // Xi x [-Wi | Wr]
+                for (int td = 0; td + sd < kDig; ++td) {
+                  const int L = sd + td < NL - 1 ? sd + td : NL - 1;
+                  const uint64_t nb = dN + (uint64_t)td * pN;
+                  const uint32_t d = tmem + (uint32_t)(L * 2 * np);
+                  const uint32_t acc = (first && sd == 0 && td == L) ? 0u : 1u;
+                  mma_bf16(d, ar, nb + p1, id, acc);  // Xr x [Wr | Wi]
+                  mma_bf16(d, ai, nb, id, 1);         // Xi x [-Wi | Wr]
+                }
+              }
+              commit(&sm.bar.empty[s]);
+            }
+            if (!ok) break;
+            commit(&sm.bar.tfull);
+          }
+        }
+        commit(&sm.bar.drain);
+        if (!mbar_wait(&sm.bar.drain, 0, kSpin)) set_status(status, 16);
+      }
+    } else if (OP != TCS_HP) {
+      // ---------------- exponents: the rows' largest |X| over the unit's k ----------------
+      // (loads eight at a time in each of the three warps; the records they
+      // need are read once per item, the next term's ahead of its unit)
+      const int xw = warp - 5;
+      uint32_t un = 0;
+      for (int64_t it = my0; it < my1 && ok; ++it) {
+        const int4 itm = tcs_fetch<OP>(g, it);
+        int K, nunits = 1;
+        uint32_t nrows, before = 1;  // at most 2^31 rows
+        int64_t stride;
+        const float4* X;  // the item's tensor (accumulations: the term's)
+        const AccTerm* terms = nullptr;
+        if (OP == TCS_ACC) {
+          const AccTask& T = g.acc[itm.x];
+          K = T.d;
+          nunits = T.count;
+          nrows = (uint32_t)T.rows;
+          stride = T.rows;
+          terms = g.terms + T.first;
+          X = reinterpret_cast<const float4*>(terms[0].X);
+        } else {
+          const MPTask& t = g.mp[itm.x];
+          K = t.a_in;
+          before = (uint32_t)t.before;
+          nrows = before * (uint32_t)t.after;
+          stride = t.before;
+          X = reinterpret_cast<const float4*>(t.in);
+        }
+        const bool along = OP == TCS_MP && before == 1;  // a row's k are contiguous
+        const uint32_t row0 = (uint32_t)itm.y * kRows;
+        for (int u = 0; u < nunits; ++u, ++un) {
+          const int buf = (int)(un & 1);
+          const float4* next = OP == TCS_ACC && u + 1 < nunits ? reinterpret_cast<const float4*>(terms[u + 1].X) : X;
+          // producers and epilogue of the unit two back have read this buffer
+          if (!waited(&sm.bar.exfree[buf], ((un >> 1) & 1) ^ 1, 19)) break;
+          int* ex = sm.ex[buf][xw];
+          if (along) {
+            // every third row, four at a time, the lanes along k
+            for (int r0 = xw; r0 < kRows; r0 += 4 * kTcsExWarps) {
+              int m[4] = {0, 0, 0, 0};
+#pragma unroll 2
+              for (int k = lane; k < K; k += 32)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const uint32_t rg = row0 + r0 + kTcsExWarps * i;
+                  const float4 x = rg < nrows ? __ldg(X + (int64_t)K * rg + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                  m[i] = max(m[i], max(fmag(x.x), fmag(x.z)));
+                }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = r0 + kTcsExWarps * i, v = __reduce_max_sync(0xffffffffu, m[i]);
+                if (lane == i && r < kRows) ex[r] = v;
               }
             }
-            commit(&sm.bar.empty[s]);
+          } else {
+            // a third of the k of every row, the lanes along the rows
+            const int ka = xw * K / kTcsExWarps, kb = (xw + 1) * K / kTcsExWarps;
+            const float4* p[4];
+            int m[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t rg = row0 + 32 * i + lane;
+              int64_t o = rg;
+              if (OP == TCS_MP) {
+                const uint32_t c = rg / before;
+                o = (int64_t)(rg - c * before) + (int64_t)before * K * c;
+              }
+              p[i] = rg < nrows ? X + o + stride * ka : nullptr;
+            }
+#pragma unroll 2
+            for (int k = ka; k < kb; ++k)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float4 x = p[i] ? __ldg(p[i] + stride * (k - ka)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                m[i] = max(m[i], max(fmag(x.x), fmag(x.z)));
+              }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ex[32 * i + lane] = m[i];
           }
-          if (!ok) break;
-          commit(&sm.bar.tfull);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.bar.exready[buf]);
+          X = next;
         }
       }
-      commit(&sm.bar.drain);
-      if (!mbar_wait(&sm.bar.drain, 0, kSpin)) set_status(status, 16);
     }
   } else {
-    // ---------------- epilogue: warps 5..12, lane quarter w % 4, column half (w - 5) / 4 ----------------
-    const int qd = warp & 3, half = (warp - 5) >> 2;
+    // ---------------- epilogue: warps 8..15, lane quarter w % 4, column half (w - 8) / 4 ----------------
+    const int qd = warp & 3, half = (warp - 8) >> 2;
     const int r = 32 * qd + lane;
     const uint32_t lane_addr = tmem + ((uint32_t)(32 * qd) << 16);
-    int* fxw = sm.fx[warp - 5];
+    int* fxw = sm.fx[warp - 8];
     uint32_t un = 0;
     for (int64_t it = my0; it < my1 && ok; ++it) {
       const int4 itm = tcs_fetch<OP>(g, it);
       const TcsItem I = tcs_item<OP>(g, itm);
       const int np = I.np, NL = I.nl;
-      const int c0 = half * (np >> 1), c1 = c0 + (np >> 1);  // this warp's columns
+      const int c0 = half * (np >> 1), w = np >> 1;  // this warp's columns
       // output row r: element n at base[n * stride]
       float4* base = nullptr;
       int64_t stride = 1;
-      bool add_first = false;
+      bool add_first = false, along_k = false;
       if (OP == TCS_HP) {
         const HpTcGroup& G = g.groups[itm.x];
         const int mi = r / G.a, j = r - mi * G.a;
@@ -1127,20 +1218,22 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
           base = reinterpret_cast<float4*>(t.out) + rg % t.before + (int64_t)t.before * t.a_out * (rg / t.before);
         stride = t.before;
         add_first = t.add != 0;
+        along_k = t.before == 1;
       }
-      if (base) base += stride * I.c0;
+      if (base) base += stride * (I.c0 + c0);
+      const int ncols = I.ncols - c0;  // real columns of this warp's half (may be <= 0)
       for (int u = 0; u < I.nunits; ++u, ++un) {
         const int buf = (int)(un & 1);
         const bool store = u == 0 && !add_first;
-        if (!__all_sync(0xffffffffu, mbar_wait(&sm.bar.exready[buf], (un >> 1) & 1, kSpin) &&
-                                         mbar_wait(&sm.bar.tfull, un & 1, kSpin))) {
-          set_status(status, 17);
-          ok = false;
-          break;
+        int er;
+        if (OP == TCS_HP) {
+          er = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + u) * kRows + r);
+        } else {
+          if (!waited(&sm.bar.exready[buf], (un >> 1) & 1, 20)) break;
+          er = row_exponent(tcs_row_max(sm.ex[buf], r, along_k));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.bar.exfree[buf]);
         }
-        fence_after_sync();
-        const int er = (int)sm.ex[buf][r];
-        mbar_arrive(&sm.bar.exfree[buf]);
         const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, u, I) +
                                                       (size_t)I.isteps * kDig * 3 * np * 32);
         const int f0 = __ldg(fxg + lane), f1 = __ldg(fxg + 32 + lane);
@@ -1155,7 +1248,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
         const bool normal = __all_sync(
             0xffffffffu, !base || (er + fmin >= 126 && er + fmax <= 379 && er < 255 && fmax < 255));
         const int erow = (er - 125) << 23;  // + (F << 23): the bits of 2^(E - 126 + F - 126)
-        float4* p = base + stride * c0;
+        if (!waited(&sm.bar.tfull, un & 1, 17)) break;
+        fence_after_sync();
         // outputs contiguous along the columns (stride 1): a lane's 16-byte
         // stores would touch 32 lines; the quads transpose 4 x 4 blocks so
         // that a store covers eight rows of 64 bytes
@@ -1165,8 +1259,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) qp[i] = shfl_ptr(base, (lane & ~3) + i);
         }
-        for (int n0 = c0; n0 < c1; n0 += 4, p += 4 * stride) {
-          const int nc = min(4, I.ncols - n0);  // columns of the block that exist (uniform)
+        float4* p = base;
+        for (int n0 = 0; n0 < w; n0 += 4, p += 4 * stride) {
+          const int nc = min(4, ncols - n0);  // columns of the block that exist (uniform)
           if (nc <= 0) break;
           // the old outputs of these four columns: their loads in flight
           // together, under the tensor-memory reads
@@ -1178,12 +1273,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
           }
           __syncwarp();
           float v[2][4], l[2][4];  // recombined levels: re and im of the four columns
-          tcs_levels(lane_addr + (uint32_t)n0, np, NL, v, l);
+          tcs_levels(lane_addr + (uint32_t)(c0 + n0), np, NL, v, l);
           if (along) {
             float4 o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float f = __int_as_float(erow + fxw[n0 + i]);
+              const float f = __int_as_float(erow + fxw[c0 + n0 + i]);
               o[i] = make_float4(__fmul_rn(v[0][i], f), __fmul_rn(l[0][i], f), __fmul_rn(v[1][i], f),
                                  __fmul_rn(l[1][i], f));
               df_norm(o[i].x, o[i].y);
@@ -1191,7 +1286,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
             }
             quad_transpose(o, lane);
             const int col = n0 + (lane & 3);
-            if (col < I.ncols) {
+            if (col < ncols) {
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 if (qp[i]) qp[i][col] = o[i];
@@ -1202,7 +1297,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
           if (normal) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float f = __int_as_float(erow + fxw[n0 + i]);
+              const float f = __int_as_float(erow + fxw[c0 + n0 + i]);
               float4 o = make_float4(__fmul_rn(v[0][i], f), __fmul_rn(l[0][i], f), __fmul_rn(v[1][i], f),
                                      __fmul_rn(l[1][i], f));
               if (!store) {
@@ -1217,7 +1312,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               if (i >= nc) continue;
-              const int fn = fxw[n0 + i] >> 23;
+              const int fn = (int)((uint32_t)fxw[c0 + n0 + i] >> 23);
               const int sh = (er - 126) + (fn - 126);
               float4 o = make_float4(scale2(v[0][i], sh), scale2(l[0][i], sh), scale2(v[1][i], sh),
                                      scale2(l[1][i], sh));
@@ -1236,7 +1331,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_tcs(TcsArgs g) {
           }
         }
         fence_before_sync();
-        mbar_arrive(&sm.bar.tempty);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.bar.tempty);
       }
     }
   }
@@ -1284,7 +1380,7 @@ cudaError_t launch_tcs(const TcsArgs& g, const int2* img_units, int64_t first_un
   const int smem = (int)sizeof(TcsSmem);
   e = cudaFuncSetAttribute(k_tcs<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k_tcs<OP><<<grid, kThreadsTc, smem, s>>>(g);
+  k_tcs<OP><<<grid, kTcsThreads, smem, s>>>(g);
   return cudaGetLastError();
 }
 
