@@ -23,22 +23,27 @@
 //    that root plus 2^-17 with binary32 step quotients, until a step is
 //    below 2^-30) and the largest cross product of two rows of H - lambda.
 //
-// Execution on this GPU: an FP64 operation has ~32 ns of latency and a
-// division or square root ~0.3 us, whatever the number of active lanes, and
-// the optimiser is one long dependency chain of them (thousands of
-// candidate evaluations per problem, in sequence).  So:
+// Execution on this GPU: an FP64 instruction occupies its sub-partition's unit
+// for 64 cycles, a dependent one follows after 73, a division takes 570 and a
+// square root 620, whatever the number of active lanes, and the optimiser is
+// one long dependency chain of them (about 2000 candidate evaluations of 120
+// FP64 instructions each per problem, in sequence).  So:
 //  * warp 0 (the master) runs the optimiser's scalar chain; every lane holds
-//    the same values, and independent divisions / square roots of the chain
-//    go to different lanes of ONE instruction (results fetched by shuffles)
-//    instead of one after another;
-//  * all four warps run the parallel phases (rotated diagonals of every
-//    matrix at ten candidate rotations, the level-by-level tree sums,
-//    Givens rotations of every matrix, the products of the off-diagonality
-//    measure).  The loops are the same in every warp; the master publishes
-//    each loop decision in shared memory before the barrier that precedes
-//    it, so the barriers match by construction;
+//    the same values, and independent operations of the chain go to different
+//    lanes of ONE instruction (results fetched by shuffles) instead of one
+//    after another.  Comparisons, powers of two and conversions to and from
+//    binary32 work on the bits: an integer instruction takes 4 cycles;
+//  * all four warps evaluate the candidates (rotated diagonals of every matrix
+//    at ten rotations, the tree sums) and run the Givens rotations and the
+//    products of the off-diagonality measure.  During the optimisation the
+//    other warps wait in a loop of their own for the master's next candidates,
+//    two barriers per evaluation;
 //  * the matrices live in shared memory when they fit (else in the task's
 //    global scratch).
+// Eight modes, bonds 7 (20 problems of 2..8 matrices): 19.2 -> 13.0 ms in this
+// kernel, the whole sweep 21.8 -> 15.9 ms alone, against one thread of control
+// for all warps, one FP64 instruction per comparison, pairs of matrices per
+// lane and descriptors decoded at each use.
 // All loops are bounded (at most 25 sweeps, 30 optimiser iterations, 64 step
 // halvings per search, 40 + 100 Newton steps).
 #include <cuda_runtime.h>
@@ -53,6 +58,8 @@ namespace {
 
 constexpr int kWsdThreads = 128;
 constexpr unsigned kFull = 0xffffffffu;
+constexpr double kDelta = 1E-5;  // step of the central differences
+constexpr double kEps = 1E-3;    // the optimiser starts at s = (eps, -eps)
 constexpr int kWsdSmemBudget = 220 * 1024;
 
 __device__ __forceinline__ double2 cm(double2 a, double2 b) {
@@ -68,40 +75,42 @@ __device__ __forceinline__ double cdiv_re(double2 x, double2 w) {
   return (x.x * w.x + x.y * w.y) / (w.x * w.x + w.y * w.y);
 }
 __device__ __forceinline__ void bsync() { __syncthreads(); }
+// the same barrier, reached by the master warp and by the others from different loops
+__device__ __forceinline__ void role_sync() { asm volatile("barrier.sync 1, %0;" ::"n"(kWsdThreads) : "memory"); }
 
 // binary64 -> binary32 by truncation of the significand; zero below 2^-126,
 // infinity above the binary32 range (integer operations only)
 __device__ __forceinline__ float f32_trunc(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-  const int e = (int)((b >> 52) & 0x7ff) - 896;
-  unsigned r;
-  if (e <= 0)
-    r = sign;
-  else if (e >= 255)
-    r = sign | 0x7f800000u;
-  else
-    r = sign | ((unsigned)e << 23) | (unsigned)((b >> 29) & 0x7fffffu);
+  const unsigned hi = (unsigned)__double2hiint(x), sign = hi & 0x80000000u, mag = hi & 0x7fffffffu;
+  // the exponent's low nine bits and the significand, rebiased modulo 2^9
+  unsigned r = (__funnelshift_l((unsigned)__double2loint(x), hi, 3) + 0x40000000u) | sign;
+  if (mag < 0x38100000u) r = sign;
+  if (mag >= 0x47f00000u) r = sign | 0x7f800000u;
   return __uint_as_float(r);
 }
 // binary32 -> binary64, exact for normal numbers; subnormals become zero
 __device__ __forceinline__ double f64_of(float f) {
-  const unsigned r = __float_as_uint(f);
-  const unsigned long long sign = (unsigned long long)(r & 0x80000000u) << 32;
-  const unsigned e = (r >> 23) & 0xffu;
-  unsigned long long b;
-  if (e == 0)
-    b = sign;
-  else if (e == 255)
-    b = sign | 0x7ff0000000000000ull | ((unsigned long long)(r & 0x7fffffu) << 29);
-  else
-    b = sign | ((unsigned long long)(e + 896) << 52) | ((unsigned long long)(r & 0x7fffffu) << 29);
-  return __longlong_as_double((long long)b);
+  const unsigned r = __float_as_uint(f), sign = r & 0x80000000u, mag = r & 0x7fffffffu;
+  unsigned hi = sign | ((mag >> 3) + 0x38000000u), lo = r << 29;
+  if (mag >= 0x7f800000u) hi = sign | 0x7ff00000u | ((mag & 0x7fffffu) >> 3);
+  if (mag < 0x00800000u) {
+    hi = sign;
+    lo = 0;
+  }
+  return __hiloint2double((int)hi, (int)lo);
 }
+
+// a level's operation in one lane: the source lanes x | y << 5 (sign bit: of
+// the addend's flip) and the masks of the factor and the addend.  A lane
+// without an operation keeps its value as S - (+0), the zero from slot 5.
+struct LaneOp {
+  uint32_t src, gm, am;
+};
+constexpr int kEigLevels = 11;
 
 struct Prob {
   int d, n;
-  int H, lgH;  // first level of the matrix tree: H = max(P2 / 2, 1) = 2^lgH, P2 = n padded to a power of two
+  int lgG, m;     // G = 2^lgG lanes per tree over the matrices, m matrices per lane: G m = n padded to a power of two
   int chunk;   // matrices per pass of the off-diagonality measure
   double2* xw;  // n weighted matrices
   double2* xp;  // n plain (shifted) matrices
@@ -110,14 +119,20 @@ struct Prob {
   double2* tM;  // chunk x d^2: X T, then Y Y
   double2* tY;  // chunk x d^2: Y
   double2* blk;   // (n + 1) x 4: (pp, pq, qp, qq) of every matrix and of w at the current pair
-  double2* cand;  // 10 x 2: candidate (c, s)
+  double2* cand0;  // 10 x 2: the first candidates of every pair
+  double2* cand;  // 10 x 2: candidate ((c, |s|^2), s)
   double2* rot;   // the accepted rotation (c, s) of the pair
-  double* sq;     // two tree buffers of 2 x 10 x H
+  double* sq;     // 2 x 10: sums of the squared rotated diagonals per candidate
   double* wd;     // 10 x 2: rotated diagonals of w per candidate
   double* tr;     // chunk x d: diagonal of W Z per matrix
   double* val;    // 2: broadcast values
-  int* ctl;       // 2: loop decisions
-  const uint32_t* lut;  // kEigLevels x 32 lane descriptors
+  int* ctl;       // 1: the master's loop decision (0: done; 1, 2: evaluate cand0, cand)
+  // the master's lanes:
+  LaneOp eig[kEigLevels];    // the eigenproblem's levels
+  double den, zh, zl;        // divisor of the central differences; 1 / den as zh + zl
+  uint32_t diff;             // their terms: lanes of A, B, C, D (5 bits each), the sign of B
+  double dx;                 // the candidate's offset from s in the lane's component
+  double c0, sab0;           // c and |s| of the first candidate
   __device__ double2* X(int k) const { return xw + (int64_t)k * d * d; }
   __device__ double2* Xp(int k) const { return xp + (int64_t)k * d * d; }
 };
@@ -129,12 +144,12 @@ struct Prob {
 // time whether or not it depends on the previous one, so the scalar chain
 // costs one unit slot per instruction.  Independent multiplies, adds and
 // subtracts of one level therefore go into ONE fused multiply-add across
-// the lanes: x*y as fma(x, y, -0), x + y as fma(1, x, y), x - y as
-// fma(1, x, -y) -- each rounds exactly once, like the separate operation
+// the lanes: x*y as fma(x, y, -0), x + y as fma(x, 1, y), x - y as
+// fma(x, 1, -y) -- each rounds exactly once, like the separate operation
 // (the -0 addend keeps the sign of a zero product).  A level's operands are
 // shuffled from a slot vector S (lane l holds value #l); lane descriptors
-// (shared memory, one 32-bit word per lane and level) name the source slots,
-// the operation, |y| and whether the lane keeps its result.
+// (three words per lane and level, in registers) name the source slots and
+// mask the factor and the addend.
 
 // -x and |x| on the sign bit (integer instructions, the IEEE results)
 __device__ __forceinline__ double neg_bits(double x) {
@@ -144,42 +159,52 @@ __device__ __forceinline__ double abs_bits(double x) {
   return __longlong_as_double(__double_as_longlong(x) & 0x7fffffffffffffffll);
 }
 
-enum { OP_MUL = 0, OP_ADD = 1, OP_SUB = 2 };
-constexpr uint32_t lane_desc(int x, int y, int op, int absy = 0) {
-  return (uint32_t)x | ((uint32_t)y << 5) | ((uint32_t)op << 10) | ((uint32_t)absy << 12) | (1u << 13);
+enum { OP_SUB = 0, OP_MUL, OP_ADD, OP_ADDABS };
+constexpr uint32_t lane_desc(int x, int y, int op) { return (uint32_t)x | ((uint32_t)y << 5) | ((uint32_t)op << 10); }
+__device__ __forceinline__ LaneOp lane_op(uint32_t dsc, int lane) {
+  if (dsc == 0) dsc = (uint32_t)lane | (5u << 5);
+  const int op = (int)(dsc >> 10);
+  LaneOp o;
+  o.src = (dsc & 0x3ffu) | (op <= OP_MUL ? 0x80000000u : 0u);
+  o.gm = op == OP_MUL ? 0xffffffffu : 0u;
+  o.am = op == OP_MUL ? 0u : (op == OP_ADDABS ? 0x7fffffffu : 0xffffffffu);
+  return o;
 }
-__device__ __forceinline__ double fma_op(int op, double x, double y) {
-  const double f = op == OP_MUL ? x : 1.0;
-  const double g = op == OP_MUL ? y : x;
-  const double h = op == OP_MUL ? -0.0 : (op == OP_ADD ? y : neg_bits(y));
-  return __fma_rn(f, g, h);
-}
-__device__ __forceinline__ double lane_level(double S, uint32_t dsc) {
-  const double x = __shfl_sync(kFull, S, dsc & 31);
-  double y = __shfl_sync(kFull, S, (dsc >> 5) & 31);
-  if (dsc & (1u << 12)) y = abs_bits(y);
-  const double r = fma_op((dsc >> 10) & 3, x, y);
-  return (dsc >> 13) & 1 ? r : S;
+__device__ __forceinline__ double lane_level(double S, const LaneOp& o) {
+  const double x = __shfl_sync(kFull, S, (int)(o.src & 31));
+  const double y = __shfl_sync(kFull, S, (int)((o.src >> 5) & 31));
+  const uint32_t yh = (uint32_t)__double2hiint(y), yl = (uint32_t)__double2loint(y);
+  const uint32_t gh = (yh & o.gm) | (~o.gm & 0x3ff00000u);            // y or 1
+  const uint32_t hh = (yh & o.am) ^ (o.src & 0x80000000u);            // -0 or +-y or |y|
+  return __fma_rn(x, __hiloint2double((int)gh, (int)(yl & o.gm)), __hiloint2double((int)hh, (int)(yl & ~o.gm)));
 }
 // Comparisons of binary64 values by their bits (integer instructions; the
 // same truth values as the floating-point comparison, NaN included):
-// x < 0; x > 0; x > c and x < c for a constant c > 0
+// x < 0; x > 0; x > c for a constant c > 0
 __device__ __forceinline__ unsigned long long bits_of(double x) { return (unsigned long long)__double_as_longlong(x); }
 __device__ __forceinline__ bool is_negative(double x) {
-  const unsigned long long b = bits_of(x), mag = b & 0x7fffffffffffffffull;
-  return (b >> 63) && mag != 0 && mag <= 0x7ff0000000000000ull;
+  return bits_of(x) - 0x8000000000000001ull <= 0x7fefffffffffffffull;
 }
-__device__ __forceinline__ bool is_positive(double x) {
-  const unsigned long long b = bits_of(x);
-  return !(b >> 63) && b != 0 && b <= 0x7ff0000000000000ull;
-}
+__device__ __forceinline__ bool is_positive(double x) { return bits_of(x) - 1 <= 0x7fefffffffffffffull; }
 __device__ __forceinline__ bool gt_pos(double x, double c) {
-  const unsigned long long b = bits_of(x);
-  return !(b >> 63) && b > bits_of(c) && b <= 0x7ff0000000000000ull;
+  return bits_of(x) - (bits_of(c) + 1) <= 0x7ff0000000000000ull - (bits_of(c) + 1);
 }
-__device__ __forceinline__ bool lt_pos(double x, double c) {
-  const unsigned long long b = bits_of(x);
-  return (b >> 63) ? ((b & 0x7fffffffffffffffull) <= 0x7ff0000000000000ull) : b < bits_of(c);
+// x < y of any two values; x > y of two that are not below zero (sums of squares) or NaN
+__device__ __forceinline__ bool less(double x, double y) {
+  const long long inf = 0x7ff0000000000000ll, mask = 0x7fffffffffffffffll;
+  const long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+  const long long am = a & mask, bm = b & mask;
+  return am <= inf && bm <= inf && (a < 0 ? -am : am) < (b < 0 ? -bm : bm);
+}
+__device__ __forceinline__ bool greater_pos(double x, double y) {
+  const unsigned long long inf = 0x7ff0000000000000ull, a = bits_of(x), b = bits_of(y);
+  return a > b && a <= inf && b <= inf;
+}
+// 2 x: the exponent of a normal number below 2^1023
+__device__ __forceinline__ double twice(double x) {
+  const unsigned h = (unsigned)__double2hiint(x);
+  if ((h & 0x7fffffffu) - 0x00100000u < 0x7fd00000u) return __hiloint2double((int)(h + 0x00100000u), __double2loint(x));
+  return (bits_of(x) << 1) == 0 ? x : x + x;
 }
 // a / 2 and a * 2 for a power of two a in the normal range: the exponent
 __device__ __forceinline__ double half_pow2(double a) { return __longlong_as_double((long long)(bits_of(a) - (1ull << 52))); }
@@ -189,22 +214,21 @@ __device__ __forceinline__ double twice_pow2(double a) { return __longlong_as_do
 // and not an always-executed division
 __device__ __noinline__ double exact_quotient(double p, double dp) { return p / dp; }
 
-// Levels of the 3x3 eigenproblem.  Slots at entry: 0 h00, 1 h01, 2 h11,
+// Levels of the 3x3 eigenproblem (kEigLevels).  Slots at entry: 0 h00, 1 h01, 2 h11,
 // 3 h02, 4 h12, 5 h22 (= 0).
-constexpr int kEigLevels = 11;
 enum { EL_C1 = 0, EL_C2, EL_C3, EL_C4, EL_C5, EL_E1, EL_E2, EL_E3, EL_E4, EL_E5, EL_E6 };
 __constant__ uint32_t c_eig_lut[kEigLevels][32] = {
     // C1: the products of m and det, (h00 + h11), the Gershgorin rows' first sums
     {0, 0, 0, 0, 0, 0, 0, 0,
      lane_desc(0, 2, OP_MUL), lane_desc(1, 1, OP_MUL), lane_desc(0, 5, OP_MUL), lane_desc(3, 3, OP_MUL),
      lane_desc(2, 5, OP_MUL), lane_desc(4, 4, OP_MUL), lane_desc(1, 5, OP_MUL), lane_desc(4, 3, OP_MUL),
-     lane_desc(1, 4, OP_MUL), lane_desc(2, 3, OP_MUL), lane_desc(0, 2, OP_ADD), lane_desc(0, 1, OP_ADD, 1),
-     lane_desc(2, 1, OP_ADD, 1), lane_desc(5, 3, OP_ADD, 1)},
+     lane_desc(1, 4, OP_MUL), lane_desc(2, 3, OP_MUL), lane_desc(0, 2, OP_ADD), lane_desc(0, 1, OP_ADDABS),
+     lane_desc(2, 1, OP_ADDABS), lane_desc(5, 3, OP_ADDABS)},
     // C2: the three terms of m, the inner terms of det, tr, the Gershgorin rows
     {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0,
      lane_desc(8, 9, OP_SUB), lane_desc(10, 11, OP_SUB), lane_desc(12, 13, OP_SUB), lane_desc(14, 15, OP_SUB),
-     lane_desc(16, 17, OP_SUB), lane_desc(18, 5, OP_ADD), lane_desc(19, 3, OP_ADD, 1), lane_desc(20, 4, OP_ADD, 1),
-     lane_desc(21, 4, OP_ADD, 1)},
+     lane_desc(16, 17, OP_SUB), lane_desc(18, 5, OP_ADD), lane_desc(19, 3, OP_ADDABS), lane_desc(20, 4, OP_ADDABS),
+     lane_desc(21, 4, OP_ADDABS)},
     // C3: the outer products of det, the first sum of m, 2 tr
     {0, 0, 0, 0, 0, 0, 0, 0, lane_desc(0, 24, OP_MUL), lane_desc(1, 25, OP_MUL), lane_desc(3, 26, OP_MUL),
      lane_desc(22, 23, OP_ADD), lane_desc(27, 27, OP_ADD)},
@@ -241,90 +265,118 @@ __constant__ uint32_t c_eig_lut[kEigLevels][32] = {
 // h11 = pre3 a^2, h02 = grad0 a, h12 = grad1 a, h22 = 0): the eigenvector of
 // the largest eigenvalue as u0 = v0/v2, u1 = v1/v2 and v0^2 + v1^2 for |v| = 1.
 // Whole warp 0, every lane the same inputs and outputs.
-__device__ void eig3_top(const uint32_t* lut, double p0, double p2, double p3, double g0, double g1, double a,
-                         double* u0, double* u1, double* top2) {
+__device__ void eig3_top(const LaneOp (&lut)[kEigLevels], double p0, double p2, double p3, double g0, double g1,
+                         double a, double* u0, double* u1, double* top2) {
   const int l = threadIdx.x & 31;
-  double S = (l == 0 ? p0 : (l == 1 ? p2 : (l == 2 ? p3 : (l == 3 ? g0 : g1)))) * a;
-  S = S * (l < 3 ? a : 1.0);
-  {  // scale by 2^(1023 - e), e the largest biased exponent: max |entry| in [1, 2)
-    int e = l < 5 ? (int)(((unsigned long long)__double_as_longlong(S) >> 52) & 0x7ff) : 0;
-    e = __reduce_max_sync(kFull, e);
-    if (e >= 1 && e <= 2045) S = S * __longlong_as_double((long long)(2046 - e) << 52);
-  }
-  if (l >= 5) S = 0.0;
-  const double h00 = __shfl_sync(kFull, S, 0), h01 = __shfl_sync(kFull, S, 1), h11 = __shfl_sync(kFull, S, 2);
-  const double h02 = __shfl_sync(kFull, S, 3), h12 = __shfl_sync(kFull, S, 4), h22 = 0.0;
-  // tr = (h00 + h11) + h22; m and det as three terms each; Gershgorin rows
-#pragma unroll
-  for (int k = EL_C1; k <= EL_C5; ++k) S = lane_level(S, lut[k * 32 + l]);
-  const double tr = __shfl_sync(kFull, S, 27), tr2 = __shfl_sync(kFull, S, 12);
-  const double m = __shfl_sync(kFull, S, 14), det = __shfl_sync(kFull, S, 15);
-  double lam_g = __shfl_sync(kFull, S, 28);
-  const double r1 = __shfl_sync(kFull, S, 29), r2 = __shfl_sync(kFull, S, 30);
-  if (r1 > lam_g) lam_g = r1;
-  if (r2 > lam_g) lam_g = r2;
-  // binary32 Newton from the Gershgorin bound: p(l) = -l^3 + tr l^2 - m l + det
-  float fl = f32_trunc(lam_g);
+  double S = l == 0 ? p0 : (l == 1 ? p2 : (l == 2 ? p3 : (l == 3 ? g0 : (l == 4 ? g1 : 0.0))));
   {
-    const float f00 = f32_trunc(h00), f01 = f32_trunc(h01), f02 = f32_trunc(h02);
-    const float f11 = f32_trunc(h11), f12 = f32_trunc(h12), f22 = f32_trunc(h22);
-    const float ftr = f00 + f11 + f22;
-    const float fm = (f00 * f11 - f01 * f01) + (f00 * f22 - f02 * f02) + (f11 * f22 - f12 * f12);
-    const float fdet = f00 * (f11 * f22 - f12 * f12) - f01 * (f01 * f22 - f12 * f02) + f02 * (f01 * f12 - f11 * f02);
-    for (int it = 0; it < 40; ++it) {
-      const float p = ((-fl + ftr) * fl - fm) * fl + fdet;
-      const float dp = (-3.0f * fl + 2.0f * ftr) * fl - fm;
-      if (!(dp < 0.0f)) break;
-      const float nx = fl - p / dp;
-      if (!(nx < fl)) break;
-      fl = nx;
+    // times a^2 or a, then by 2^(1023 - e), e the largest biased exponent, so
+    // that max |entry| is in [1, 2).  a is a power of two <= 1: where no
+    // result leaves the normal range, all of it adds to the exponents
+    const int ex = (int)(bits_of(S) >> 52) & 0x7ff;
+    const bool zero = (bits_of(S) << 1) == 0;
+    const int ea = ((int)(bits_of(a) >> 52) - 1023) * (l < 3 ? 2 : 1);
+    const int e1 = zero ? 0 : ex + ea;
+    const int e = __reduce_max_sync(kFull, e1);
+    if (__all_sync(kFull, zero || (ex >= 1 && ex <= 2045 && e1 >= 1 && e1 + 1023 - e >= 1))) {
+      if (!zero) S = __longlong_as_double(__double_as_longlong(S) + ((long long)(ea + 1023 - e) << 52));
+    } else {
+      S = S * a;
+      S = S * (l < 3 ? a : 1.0);
+      int es = l < 5 ? (int)(bits_of(S) >> 52) & 0x7ff : 0;
+      es = __reduce_max_sync(kFull, es);
+      if (es >= 1 && es <= 2045) S = S * __longlong_as_double((long long)(2046 - es) << 52);
+      if (l >= 5) S = 0.0;
     }
   }
+  const float fS = f32_trunc(S);
+  // tr = (h00 + h11) + h22; m and det as three terms each; Gershgorin rows
+  S = lane_level(S, lut[EL_C1]);
+  // binary32 Newton from the Gershgorin bound: p(l) = -l^3 + tr l^2 - m l + det.
+  // Its preparation and first steps run under the binary64 levels C1 .. C5
+  const float f00 = __shfl_sync(kFull, fS, 0), f01 = __shfl_sync(kFull, fS, 1), f11 = __shfl_sync(kFull, fS, 2);
+  const float f02 = __shfl_sync(kFull, fS, 3), f12 = __shfl_sync(kFull, fS, 4), f22 = 0.0f;
+  const float ftr = f00 + f11 + f22;
+  const float fm = (f00 * f11 - f01 * f01) + (f00 * f22 - f02 * f02) + (f11 * f22 - f12 * f12);
+  const float fdet = f00 * (f11 * f22 - f12 * f12) - f01 * (f01 * f22 - f12 * f02) + f02 * (f01 * f12 - f11 * f02);
+  S = lane_level(S, lut[EL_C2]);
+  const float fg = f32_trunc(S);  // truncation keeps the order of the rows
+  S = lane_level(S, lut[EL_C3]);
+  float fl = __shfl_sync(kFull, fg, 28);
+  const float fr1 = __shfl_sync(kFull, fg, 29), fr2 = __shfl_sync(kFull, fg, 30);
+  if (fr1 > fl) fl = fr1;
+  if (fr2 > fl) fl = fr2;
+  auto newton32 = [&]() {  // one step; false when the iteration ends
+    const float p = ((-fl + ftr) * fl - fm) * fl + fdet;
+    const float dp = (-3.0f * fl + 2.0f * ftr) * fl - fm;
+    if (!(dp < 0.0f)) return false;
+    const float nx = fl - p / dp;
+    if (!(nx < fl)) return false;
+    fl = nx;
+    return true;
+  };
+  bool more = newton32();
+  S = lane_level(S, lut[EL_C4]);
+  if (more) more = newton32();
+  S = lane_level(S, lut[EL_C5]);
+  for (int it = 2; more && it < 40; ++it) more = newton32();
+  const double tr = __shfl_sync(kFull, S, 27), tr2 = __shfl_sync(kFull, S, 12);
+  const double m = __shfl_sync(kFull, S, 14), det = __shfl_sync(kFull, S, 15);
   // binary64 Newton, monotone from above.  p = ((-lam + tr) lam - m) lam + det
   // in lane 0 and p' = (-3 lam + 2 tr) lam - m in lane 1, one instruction
   // per step of both chains; 3 lam in lane 2.
   double lam = f64_of(fl) + 0x1p-17;
-  double p, dp, l3;
+  // (every step takes v as one factor, so that no selection waits for it)
   const double neg_m = neg_bits(m);
+  const double k1 = l == 0 ? -1.0 : (l == 1 ? -3.0 : 3.0);
+  const double a1 = l == 0 ? tr : -0.0, a2 = l == 1 ? tr2 : -0.0;
+  const double a3 = l == 0 ? neg_m : -0.0, a4 = l == 0 ? -0.0 : neg_m;
+  double pv;      // p in lane 0, p' in lane 1
+  unsigned negs;  // bit 0: p < 0, bit 1: p' < 0
   auto pdp = [&]() {
-    double v = __fma_rn(l == 0 ? 1.0 : (l == 1 ? -3.0 : 3.0), l == 0 ? neg_bits(lam) : lam, l == 0 ? tr : -0.0);
-    l3 = __shfl_sync(kFull, v, 2);
-    v = __fma_rn(l == 1 ? 1.0 : v, l == 1 ? v : lam, l == 1 ? tr2 : -0.0);
-    v = __fma_rn(l == 0 ? 1.0 : v, l == 0 ? v : lam, l == 0 ? neg_m : -0.0);
-    v = __fma_rn(l == 0 ? v : 1.0, l == 0 ? lam : v, l == 0 ? -0.0 : neg_m);
-    dp = __shfl_sync(kFull, v, 1);
-    v = __fma_rn(1.0, v, det);
-    p = __shfl_sync(kFull, v, 0);
+    const double even = l == 1 ? 1.0 : lam, odd = l == 0 ? 1.0 : lam, last = l == 0 ? lam : 1.0;
+    const double v1 = __fma_rn(k1, lam, a1);
+    double v = __fma_rn(v1, even, a2);
+    v = __fma_rn(v, odd, a3);
+    v = __fma_rn(v, last, a4);
+    pv = l == 0 ? __fma_rn(v, 1.0, det) : v;
+    negs = __ballot_sync(kFull, is_negative(pv));
+    return v1;  // 3 lam in lane 2
   };
-  pdp();
-  if (!(is_negative(p) && is_negative(dp) && l3 > tr)) {
-    lam = lam_g;
+  const double l3 = __shfl_sync(kFull, pdp(), 2);
+  if (!((negs & 3) == 3 && less(tr, l3))) {
+    lam = __shfl_sync(kFull, S, 28);  // the Gershgorin bound
+    const double r1 = __shfl_sync(kFull, S, 29), r2 = __shfl_sync(kFull, S, 30);
+    if (less(lam, r1)) lam = r1;
+    if (less(lam, r2)) lam = r2;
     pdp();
   }
   for (int it = 0; it < 100; ++it) {
-    if (!is_negative(dp)) break;
-    double step = f64_of(f32_trunc(p) / f32_trunc(dp));
-    if (!(((unsigned long long)__double_as_longlong(step) & 0x7fffffffffffffffull) <= 0x4030000000000000ull))
-      step = exact_quotient(p, dp);  // |step| > 16 or NaN: the binary32 quotient left its range
+    if (!(negs & 2)) break;
+    const float fv = f32_trunc(pv);
+    double step = f64_of(__shfl_sync(kFull, fv, 0) / __shfl_sync(kFull, fv, 1));
+    if (!((bits_of(step) & 0x7fffffffffffffffull) <= 0x4030000000000000ull))
+      // |step| > 16 or NaN: the binary32 quotient left its range
+      step = exact_quotient(__shfl_sync(kFull, pv, 0), __shfl_sync(kFull, pv, 1));
     const double nxt = lam - step;
-    if (!(nxt < lam)) break;
+    if (!(is_positive(step) && bits_of(nxt) != bits_of(lam))) break;  // nxt < lam
     lam = nxt;
     // step > 0 here: compare the bits with those of 2^-30
-    if ((unsigned long long)__double_as_longlong(step) <= 0x3e10000000000000ull) break;
+    if (bits_of(step) <= 0x3e10000000000000ull) break;
     pdp();
   }
   // eigenvector: the largest cross product of two rows of H - lambda
   if (l == 31) S = lam;
 #pragma unroll
-  for (int k = EL_E1; k <= EL_E6; ++k) S = lane_level(S, lut[k * 32 + l]);
+  for (int k = EL_E1; k <= EL_E6; ++k) S = lane_level(S, lut[k]);
   const double n01 = __shfl_sync(kFull, S, 0), n02 = __shfl_sync(kFull, S, 1), n12 = __shfl_sync(kFull, S, 2);
   int sel = 0;
   double nv = n01;
-  if (n02 > nv) {
+  if (greater_pos(n02, nv)) {
     sel = 1;
     nv = n02;
   }
-  if (n12 > nv) sel = 2;
+  if (greater_pos(n12, nv)) sel = 2;
   // u0 = v0 / v2, u1 = v1 / v2, top2 = (v0^2 + v1^2) / |v|^2 in lanes 0, 1, 2
   const double num = __shfl_sync(kFull, S, l == 0 ? 9 + 3 * sel : (l == 1 ? 10 + 3 * sel : 27 + sel));
   const double den = __shfl_sync(kFull, S, l < 2 ? 11 + 3 * sel : sel);
@@ -337,19 +389,25 @@ __device__ void eig3_top(const uint32_t* lut, double p0, double p2, double p3, d
 // weightedJacobiDerivatives from the loss at the nine points (i, j) of the
 // central differences (y[i + 3 j]): lane k takes numerator k as
 // ((A + B) - C) - D (a difference x - y as x + (-y); subtracting +0 keeps
-// every value) and one division gives all five quotients
-__device__ void grad_pre(const double y[9], double delta, double& g0, double& g1, double& p0, double& p2,
-                         double& p3) {
+// every value) and one division by the lane's constant gives all five
+// quotients: q0 = num zh + num zl is within an ulp of num / den, its remainder
+// is exact, and the remainder times zh = fl(1 / den) corrects it to the rounded
+// quotient (Markstein's theorem; four operations instead of the division's
+// nine).  Numbers near the ends of the range take the division.
+// y: lane 1 + (i + 3 j) holds y[i + 3 j], lane 31 zero.
+__device__ void grad_pre(const Prob& P, double y, double& g0, double& g1, double& p0, double& p2, double& p3) {
   const int l = threadIdx.x & 31;
-  const double y4x2 = 2 * y[1 + 3 * 1];
-  const double A = l == 0 || l == 2 ? y[2 + 3 * 1] : (l == 1 || l == 3 ? y[1 + 3 * 2] : y[2 + 3 * 2]);
-  const double B = l == 0 ? neg_bits(y[0 + 3 * 1])
-                           : (l == 1 ? neg_bits(y[1 + 3 * 0]) : (l == 2 ? y[0 + 3 * 1] : (l == 3 ? y[1 + 3 * 0] : y[0 + 3 * 0])));
-  const double C = l < 2 ? 0.0 : (l < 4 ? y4x2 : y[2 + 3 * 0]);
-  const double D = l < 4 ? 0.0 : y[0 + 3 * 2];
+  const double A = __shfl_sync(kFull, y, P.diff & 31);
+  double B = __shfl_sync(kFull, y, (P.diff >> 5) & 31);
+  double C = __shfl_sync(kFull, y, (P.diff >> 10) & 31);
+  const double D = __shfl_sync(kFull, y, (P.diff >> 15) & 31);
+  if (P.diff >> 20) B = neg_bits(B);
+  if (l == 2 || l == 3) C = twice(C);
   const double num = ((A + B) - C) - D;
-  const double den = l < 2 ? 2 * delta : (l < 4 ? delta * delta : 4 * delta * delta);
-  const double r = num / den;
+  const double q0 = __fma_rn(num, P.zh, num * P.zl);
+  double r = __fma_rn(__fma_rn(neg_bits(q0), P.den, num), P.zh, q0);
+  const unsigned e = (unsigned)(bits_of(num) >> 52) & 0x7ffu;
+  if (e < 100 || e > 1900) r = (bits_of(num) << 1) == 0 ? num : exact_quotient(num, P.den);
   g0 = __shfl_sync(kFull, r, 0);
   g1 = __shfl_sync(kFull, r, 1);
   p0 = __shfl_sync(kFull, r, 2);
@@ -357,25 +415,22 @@ __device__ void grad_pre(const double y[9], double delta, double& g0, double& g1
   p2 = __shfl_sync(kFull, r, 4);
 }
 
-// Candidate 0 = (sqrt|arg0|, s) and the nine samples of the central
-// differences around s (weightedJacobiDerivatives) into P.cand, one square
-// root per lane (lanes 0..9); lane 10 takes sqrt|arg10|.  Returns each
-// lane's root.
-__device__ double put_candidates(const Prob& P, double arg0, double sx, double sy, double delta, double arg10) {
-  const int l = threadIdx.x & 31;
-  double x0 = sx, x1 = sy, arg = l == 10 ? arg10 : arg0;
-  if (l >= 1 && l <= 9) {
-    const int q = l - 1, i = q % 3, j = q / 3;
-    // (i - 1) delta and (j - 1) delta: -delta, +0 or delta, exactly
-    x0 = sx + (i == 0 ? -delta : (i == 1 ? 0.0 : delta));
-    x1 = sy + (j == 0 ? -delta : (j == 1 ? 0.0 : delta));
-    const double z = x0 * x0 + x1 * x1;
-    arg = 1 - z;
-  }
-  const double r = sqrt(abs_bits(arg));
-  if (l <= 9) {
-    P.cand[2 * l] = make_double2(r, 0.0);
-    P.cand[2 * l + 1] = make_double2(x0, x1);
+// Candidate 0 = (sqrt|1 - z0|, s) and the nine samples of the central
+// differences around s (weightedJacobiDerivatives) into cand, one square
+// root per lane (lanes 0..9); lane 10 takes sqrt(y0^2 + y1^2).  Returns each
+// lane's root; z: its |x|^2 (lane 10: y0^2 + y1^2).
+__device__ double put_candidates(const Prob& P, double2* cand, double z0, double sx, double sy, double y0, double y1,
+                                 double& z) {
+  const int l = threadIdx.x & 31, k = l & 15;
+  // component 0 of s + ((i - 1) delta, (j - 1) delta) in lane k, component 1 in lane 16 + k; x + -0 keeps every x
+  const double x = (k == 10 ? (l < 16 ? y0 : y1) : (l < 16 ? sx : sy)) + P.dx;
+  const double x2 = x * x;
+  z = x2 + __shfl_xor_sync(kFull, x2, 16);
+  const double arg = 1 - (k == 0 ? z0 : z);
+  const double r = sqrt(k == 10 ? z : abs_bits(arg));
+  if (k <= 9) {
+    if (l < 16) cand[2 * k] = make_double2(r, z);
+    (l < 16 ? cand[2 * k + 1].x : cand[2 * k + 1].y) = x;
   }
   return r;
 }
@@ -384,11 +439,9 @@ __device__ double put_candidates(const Prob& P, double arg0, double sx, double s
 
 // rotatedDiagonals of a cached 2x2 block (pp, pq, qp, qq) of a Hermitian
 // matrix for a real c: a0 = c^2 A_pp + 2c Re(s A_pq) + |s|^2 A_qq and
-// a1 = c^2 A_qq - 2c Re(s A_pq) + |s|^2 A_pp
-__device__ __forceinline__ void rotated_diagonals(const double2* b, double2 c, double2 s, double& a0, double& a1) {
-  const double cc2 = c.x * c.x;
-  const double ss2 = s.x * s.x + s.y * s.y;
-  const double c2 = 2.0 * c.x;
+// a1 = c^2 A_qq - 2c Re(s A_pq) + |s|^2 A_pp (cc2 = c^2, c2 = 2c, ss2 = |s|^2)
+__device__ __forceinline__ void rotated_diagonals(const double2* b, double cc2, double c2, double ss2, double2 s,
+                                                  double& a0, double& a1) {
   const double2 apq = b[1];
   const double t = s.x * apq.x - s.y * apq.y;
   const double ct = c2 * t;
@@ -396,243 +449,234 @@ __device__ __forceinline__ void rotated_diagonals(const double2* b, double2 c, d
   a1 = (cc2 * b[3].x - ct) + ss2 * b[0].x;
 }
 
-// levels 2.. of the pairwise tree over `count` rows of H values per
-// component (level 1 is in buf); returns the buffer holding the sums
-__device__ double* tree_levels(const Prob& P, int count) {
-  const int H = P.H, tid = threadIdx.x;
-  double* buf = P.sq;
-  double* alt = P.sq + 2 * 10 * H;
-  for (int lg = P.lgH; lg > 0; --lg) {  // sizes H, H/2, .., 2 (powers of two)
-    const int half = 1 << (lg - 1);
-    for (int it = tid; it < (2 * count) << (lg - 1); it += kWsdThreads) {
-      const int g = it >> (lg - 1), i = it & (half - 1);  // g = (component, candidate)
-      const int comp = g >= count ? 1 : 0, j = g - comp * count;
-      const double* src = buf + comp * 10 * H + j * H;
-      alt[comp * 10 * H + j * H + i] = src[2 * i] + src[2 * i + 1];
+// The pairwise tree over the matrices, two sums at once: a lane's m (a power
+// of two) consecutive leaves f(0..m-1) ..
+template <class F>
+__device__ __forceinline__ void local_tree(int m, F f, double& s0, double& s1) {
+  f(0, s0, s1);
+  if (m == 1) return;
+  double b0, b1;
+  f(1, b0, b1);
+  s0 = s0 + b0;
+  s1 = s1 + b1;
+  if (m == 2) return;
+  double st0[12], st1[12];  // finished subtrees of 2, 4, 8, .. leaves
+  st0[0] = s0;
+  st1[0] = s1;
+  for (int i = 2; i < m; i += 2) {
+    double a0, a1;
+    f(i, a0, a1);
+    f(i + 1, b0, b1);
+    s0 = a0 + b0;
+    s1 = a1 + b1;
+    int lev = 0;
+    for (int k = i >> 1; k & 1; k >>= 1, ++lev) {
+      s0 = st0[lev] + s0;
+      s1 = st1[lev] + s1;
     }
-    bsync();
-    double* t = buf;
-    buf = alt;
-    alt = t;
+    st0[lev] = s0;
+    st1[lev] = s1;
   }
-  return buf;
+}
+// .. then the G lanes of a group (a power of two up to 32): the group's even
+// lanes return the first sum, the odd ones the second, one addition per level
+// for both.  Whole warp.
+__device__ __forceinline__ double lane_tree(double s0, double s1, int G) {
+  const bool odd = threadIdx.x & 1;
+  const double other = __shfl_xor_sync(kFull, odd ? s0 : s1, 1);
+  if (G == 1) return odd ? other : s0;  // lane 0's two sums in lanes 0 and 1
+  double v = (odd ? s1 : s0) + other;
+  for (int off = 2; off < G; off <<= 1) v = v + __shfl_xor_sync(kFull, v, off);
+  return v;
 }
 
-// weightedJacobiLoc for the `count` candidates in P.cand; xo0, xo1 = xold / w
-// of the pair.  Returns, in warp 0, the loss change of candidate j in lane j
-// and xnum / xden (a division of the caller's, issued with the same
-// instruction) in lane 2 count.  Other warps return 0.
-__device__ double loc_many(const Prob& P, int count, double xo0, double xo1, double xnum, double xden) {
-  const int n = P.n, H = P.H, tid = threadIdx.x;
-  const int items = count * H;
-  // squared rotated diagonals with the first tree level; w's rotated diagonals
-  for (int it = tid; it < items + count; it += kWsdThreads) {
-    if (it < items) {
-      const int j = it >> P.lgH, i = it & (H - 1);
-      const double2 c = P.cand[2 * j], s = P.cand[2 * j + 1];
-      double r0, r1, s0 = 0.0, s1 = 0.0;
-      if (n == 1) {
-        rotated_diagonals(P.blk, c, s, r0, r1);
-        s0 = r0 * r0;
-        s1 = r1 * r1;
-      } else {
-        double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-        if (2 * i < n) {
-          rotated_diagonals(P.blk + 8 * i, c, s, r0, r1);
-          a0 = r0 * r0;
-          a1 = r1 * r1;
+// Ten candidates (all warps): G lanes per candidate add the
+// squared rotated diagonals of the matrices, one more lane per candidate
+// rotates w's.  An FP64 instruction costs the same for one lane as for 32, so
+// up to eight matrices have a lane each, and the tree runs through shuffles.
+// Pairs of matrices per lane with the tree's levels in shared memory, a
+// barrier after each, took 4.6 k cycles per call for eight matrices, this
+// form 1.9 k.  One copy of the code for all warps: the
+// kernel's loop body is larger than the instruction cache next to the warps.
+__device__ __forceinline__ void eval_items(const double2* blk, const double2* cand, double* sq, double* wd, int n, int lgG,
+                                        int m) {
+  const int G = 1 << lgG, lane = threadIdx.x & 31;
+  const int total = 10 * G + 10;
+  for (int it0 = threadIdx.x - lane; it0 < total; it0 += kWsdThreads) {
+    const int it = it0 + lane;
+    const bool isw = it >= 10 * G;
+    const int j = isw ? min(it - 10 * G, 9) : it >> lgG, g = isw ? 0 : it & (G - 1);
+    const double2 c = cand[2 * j], s = cand[2 * j + 1];
+    const double cc2 = c.x * c.x, c2 = twice(c.x), ss2 = c.y;
+    double s0, s1, w0 = 0.0, w1 = 0.0;
+    local_tree(m, [&](int q, double& v0, double& v1) {
+      const int k = isw ? n : g * m + q;
+      v0 = v1 = 0.0;
+      if (isw ? q == 0 : k < n) {
+        double r0, r1;
+        rotated_diagonals(blk + 4 * k, cc2, c2, ss2, s, r0, r1);
+        if (q == 0) {
+          w0 = r0;
+          w1 = r1;
         }
-        if (2 * i + 1 < n) {
-          rotated_diagonals(P.blk + 8 * i + 4, c, s, r0, r1);
-          b0 = r0 * r0;
-          b1 = r1 * r1;
-        }
-        s0 = a0 + b0;
-        s1 = a1 + b1;
+        v0 = r0 * r0;
+        v1 = r1 * r1;
       }
-      P.sq[j * H + i] = s0;
-      P.sq[10 * H + j * H + i] = s1;
-    } else {
-      const int j = it - items;
-      double r0, r1;
-      rotated_diagonals(P.blk + 4 * n, P.cand[2 * j], P.cand[2 * j + 1], r0, r1);
-      P.wd[2 * j] = r0;
-      P.wd[2 * j + 1] = r1;
+    }, s0, s1);
+    const double v = lane_tree(s0, s1, G);
+    if (isw) {
+      if (it < total) {
+        wd[2 * j] = w0;
+        wd[2 * j + 1] = w1;
+      }
+    } else if (G == 1) {
+      sq[j] = s0;
+      sq[10 + j] = s1;
+    } else if (g < 2) {
+      sq[10 * g + j] = v;
     }
   }
-  bsync();
-  const double* sums = tree_levels(P, count);
-  double res = 0.0;
-  if (tid < 32) {  // diff = (xnew0 / w0 - xold0 / w_pp) + (xnew1 / w1 - xold1 / w_qq), one division per lane
-    const int l = tid;
-    double num = xnum, den = xden;
-    if (l < 2 * count) {
-      const int c = l >= count ? 1 : 0, j = l - c * count;
-      num = sums[c * 10 * H + j * H];
-      den = P.wd[2 * j + c];
-    }
-    const double q = num / den;
-    const double t = q - (l < count ? xo0 : xo1);
-    const double t1 = __shfl_sync(kFull, t, (l + count) & 31);
-    double diff = 0;
-    diff += t;
-    diff += t1;
-    res = l < count ? diff : q;
-  }
-  return res;
 }
 
-// calculateWeightedAngles: rational function optimisation of (c, s).  The
-// loss of every new candidate is evaluated together with the nine samples of
-// the central differences around it: if the candidate is accepted they are
-// the next iteration's derivatives, if not the derivatives at the unchanged
-// point are still valid -- the same numbers the reference recomputes.
-// All threads; the rotation is returned in warp 0.
-__device__ void angles(const Prob& P, double xo0, double xo1, double2& c_out, double2& s_out) {
-  const bool master = threadIdx.x < 32;
+// weightedJacobiLoc for the ten candidates in P.cand0 (which 1) or P.cand (2); xo0, xo1 = xold / w
+// of the pair.  Master warp, with the other warps in their loop of
+// rotations().  Returns the loss change of candidate j in lane j and
+// xnum / xden (a division of the caller's, issued with the same instruction)
+// in lane 20.
+__device__ __forceinline__ double loc_many(const Prob& P, int which, double xo0, double xo1, double xnum, double xden) {
+  const int l = threadIdx.x & 31;
+  if (l == 0) P.ctl[0] = which;
+  role_sync();
+  eval_items(P.blk, which == 1 ? P.cand0 : P.cand, P.sq, P.wd, P.n, P.lgG, P.m);
+  role_sync();
+  // diff = (xnew0 / w0 - xold0 / w_pp) + (xnew1 / w1 - xold1 / w_qq), one division per lane
+  double num = xnum, den = xden;
+  if (l < 20) {
+    const int c = l >= 10 ? 1 : 0, j = l - 10 * c;
+    num = P.sq[l];
+    den = P.wd[2 * j + c];
+  }
+  const double q = num / den;
+  double t = q - (l < 10 ? xo0 : xo1);
+  const double t1 = __shfl_sync(kFull, t, (l + 10) & 31);
+  if ((bits_of(t) << 1) == 0) t = 0.0;  // 0 + t: a zero of either sign becomes +0
+  return l < 10 ? t + t1 : q;
+}
+
+// calculateWeightedAngles: rational function optimisation of (c, s), into
+// P.rot.  The loss of every new candidate is evaluated together with the nine
+// samples of the central differences around it: if the candidate is accepted
+// they are the next iteration's derivatives, if not the derivatives at the
+// unchanged point are still valid -- the same numbers the reference
+// recomputes.  Master warp.
+__device__ void angles(const Prob& P, double xo0, double xo1) {
   const int lane = threadIdx.x & 31;
-  const double eps = 1E-3, amin = 1E-12, amax = 1, delta = 1E-5;
+  const double eps = kEps, amin = 1E-12, amax = 1;
   double a = amax, diff_rel = 2 * eps * eps;
-  double c0 = 0, s0 = eps, s1 = -eps, sab = 0, loc_alt = 0;
-  double ycur[9];
-  if (master) {
-    const double r = put_candidates(P, 1 - 2 * eps * eps, s0, s1, delta, s0 * s0 + s1 * s1);
-    c0 = __shfl_sync(kFull, r, 0);
-    sab = __shfl_sync(kFull, r, 10);  // |s|
-  }
-  bsync();
-  {
-    const double res = loc_many(P, 10, xo0, xo1, 0.0, 1.0);
-    if (master) {
-      loc_alt = __shfl_sync(kFull, res, 0);
-#pragma unroll
-      for (int q = 0; q < 9; ++q) ycur[q] = __shfl_sync(kFull, res, 1 + q);
-    }
-  }
-  for (int iter = 0; iter < 30; ++iter) {
-    if (master && lane == 0) P.ctl[0] = (gt_pos(diff_rel, eps * eps) && gt_pos(a, amin)) ? 1 : 0;
-    bsync();
-    if (!P.ctl[0]) break;
-    double g0 = 0, g1 = 0, p0 = 0, p2 = 0, p3 = 0;
-    if (master) grad_pre(ycur, delta, g0, g1, p0, p2, p3);
-    double diff = -1, loc_new = 0, cnew = 0, snew0 = 0, snew1 = 0, zab = 0, top2 = 0;
-    double ynew[9];
-#pragma unroll
-    for (int q = 0; q < 9; ++q) ynew[q] = 0;
-    for (int guard = 0; guard < 64; ++guard) {
-      if (master) {
-        const int go = (gt_pos(a, amin) && is_negative(diff) && gt_pos(diff_rel, eps * eps)) ? 1 : 0;
-        if (go) {
-          double z = 1;
-          for (int g2 = 0; gt_pos(a, amin) && gt_pos(z, 0.5) && g2 < 64; ++g2) {
-            // rfoBuildHessian (src/Core/JacobiRotationFramework.cpp:114-127)
-            double u0, u1;
-            eig3_top(P.lut, p0, p2, p3, g0, g1, a, &u0, &u1, &top2);
-            // ds = a u, snew = s + ds in lanes 0 and 1; zab = sqrt(snew0^2 + snew1^2)
-            double v = a * (lane == 0 ? u0 : u1);
-            v = (lane == 0 ? s0 : s1) + v;
-            snew0 = __shfl_sync(kFull, v, 0);
-            snew1 = __shfl_sync(kFull, v, 1);
-            v = v * v;
-            zab = sqrt(__shfl_sync(kFull, v, 0) + __shfl_sync(kFull, v, 1));
-            z = zab * zab;
-            if (gt_pos(z, 0.5)) a = half_pow2(a);
-          }
-          const double r = put_candidates(P, 1 - z, snew0, snew1, delta, 0.0);
-          cnew = __shfl_sync(kFull, r, 0);
-        }
-        if (lane == 0) P.ctl[1] = go;
-      }
-      bsync();
-      if (!P.ctl[1]) break;
-      const double res = loc_many(P, 10, xo0, xo1, top2, sab * sab + eps * eps);
-      if (master) {
-        loc_new = __shfl_sync(kFull, res, 0);
-#pragma unroll
-        for (int q = 0; q < 9; ++q) ynew[q] = __shfl_sync(kFull, res, 1 + q);
-        diff_rel = __shfl_sync(kFull, res, 20);  // |trafo|^2 / (|s|^2 + eps^2)
-        diff = loc_new - loc_alt;
-        if (is_negative(diff)) {
-          a = half_pow2(a);
-        } else {
-          if (lt_pos(a, amax)) a = twice_pow2(a);
-        }
-      }
-    }
-    if (master && gt_pos(a, amin) && is_positive(diff)) {
-      c0 = cnew;
-      s0 = snew0;
-      s1 = snew1;
-      sab = zab;
+  double c0 = P.c0, s0 = eps, s1 = -eps, sab = P.sab0, loc_alt = 0;
+  double cur = 0;  // loss changes of the current point (lane 0) and its samples (lanes 1..9)
+  double g0 = 0, g1 = 0, p0 = 0, p2 = 0, p3 = 0;
+  double cnew = 0, snew0 = 0, snew1 = 0, zab = 0, top2 = 0, xden = 1;
+  int which = 1, iter = 0, guard = 0;
+  for (;;) {
+    const double res = loc_many(P, which, xo0, xo1, top2, xden);
+    const double loc_new = __shfl_sync(kFull, res, 0);
+    bool search = false;  // another step length at the same point
+    if (which == 1) {
+      which = 2;
+      cur = res;
       loc_alt = loc_new;
-#pragma unroll
-      for (int q = 0; q < 9; ++q) ycur[q] = ynew[q];
+    } else {
+      diff_rel = __shfl_sync(kFull, res, 20);  // |trafo|^2 / (|s|^2 + eps^2)
+      const double diff = loc_new - loc_alt;
+      if (is_negative(diff)) {
+        a = half_pow2(a);
+      } else {
+        if (bits_of(a) < bits_of(amax)) a = twice_pow2(a);  // a > 0
+      }
+      search = ++guard < 64 && gt_pos(a, amin) && is_negative(diff) && gt_pos(diff_rel, eps * eps);
+      if (!search) {
+        ++iter;
+        if (gt_pos(a, amin) && is_positive(diff)) {
+          c0 = cnew;
+          s0 = snew0;
+          s1 = snew1;
+          sab = zab;
+          loc_alt = loc_new;
+          cur = res;
+        }
+      }
     }
+    if (!search) {
+      if (!(iter < 30 && gt_pos(diff_rel, eps * eps) && gt_pos(a, amin))) break;
+      grad_pre(P, lane == 31 ? 0.0 : cur, g0, g1, p0, p2, p3);
+      guard = 0;
+    }
+    double z = 1;
+    for (int g2 = 0; gt_pos(a, amin) && gt_pos(z, 0.5) && g2 < 64; ++g2) {
+      // rfoBuildHessian (src/Core/JacobiRotationFramework.cpp:114-127)
+      double u0, u1;
+      eig3_top(P.eig, p0, p2, p3, g0, g1, a, &u0, &u1, &top2);
+      // ds = a u, snew = s + ds in lanes 0 and 1; zab = sqrt(snew0^2 + snew1^2)
+      double v = a * (lane == 0 ? u0 : u1);
+      v = (lane == 0 ? s0 : s1) + v;
+      snew0 = __shfl_sync(kFull, v, 0);
+      snew1 = __shfl_sync(kFull, v, 1);
+      v = v * v;
+      zab = sqrt(__shfl_sync(kFull, v, 0) + __shfl_sync(kFull, v, 1));
+      z = zab * zab;
+      if (gt_pos(z, 0.5)) a = half_pow2(a);
+    }
+    // lane 10: |s|^2 + eps^2 of the current point
+    double zz;
+    const double r = put_candidates(P, P.cand, z, snew0, snew1, sab, eps, zz);
+    cnew = __shfl_sync(kFull, r, 0);
+    xden = __shfl_sync(kFull, zz, 10);
   }
-  c_out = make_double2(c0, 0.0);
-  s_out = make_double2(s0, s1);
+  if (lane == 0) {
+    P.rot[0] = make_double2(c0, 0.0);
+    P.rot[1] = make_double2(s0, s1);
+    P.ctl[0] = 0;
+  }
+  role_sync();
 }
 
 // weightedJacobiRotations: every pair (i < j) in order; for each, the
 // optimised rotation applied to every weighted matrix, to w and to T
 __device__ void rotations(const Prob& P) {
-  const int d = P.d, n = P.n, H = P.H, tid = threadIdx.x;
-  const bool master = tid < 32;
+  const int d = P.d, n = P.n, tid = threadIdx.x;
   for (int i = 0; i < d - 1; ++i)
     for (int j = i + 1; j < d; ++j) {
-      // the (i, j) blocks of every matrix and of w; the squared current
-      // diagonals with the first level of their tree
-      for (int it = tid; it < n + 1 + H; it += kWsdThreads) {
-        if (it <= n) {
-          const double2* A = it < n ? P.X(it) : P.w;
-          P.blk[4 * it + 0] = A[i + (int64_t)d * i];
-          P.blk[4 * it + 1] = A[i + (int64_t)d * j];
-          P.blk[4 * it + 2] = A[j + (int64_t)d * i];
-          P.blk[4 * it + 3] = A[j + (int64_t)d * j];
-        } else {
-          const int h = it - n - 1;
-          double s0, s1;
-          if (n == 1) {
-            const double x0 = P.X(0)[i + (int64_t)d * i].x, x1 = P.X(0)[j + (int64_t)d * j].x;
-            s0 = x0 * x0;
-            s1 = x1 * x1;
-          } else {
-            double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-            if (2 * h < n) {
-              const double x0 = P.X(2 * h)[i + (int64_t)d * i].x, x1 = P.X(2 * h)[j + (int64_t)d * j].x;
-              a0 = x0 * x0;
-              a1 = x1 * x1;
-            }
-            if (2 * h + 1 < n) {
-              const double x0 = P.X(2 * h + 1)[i + (int64_t)d * i].x, x1 = P.X(2 * h + 1)[j + (int64_t)d * j].x;
-              b0 = x0 * x0;
-              b1 = x1 * x1;
-            }
-            s0 = a0 + b0;
-            s1 = a1 + b1;
+      if (tid < 32) {
+        // xold / w of the pair, lanes 0 and 1; then the optimiser
+        const int p2 = P.m << P.lgG, G = min(p2, 32), m = p2 / G;
+        double s0, s1;
+        local_tree(m, [&](int q, double& v0, double& v1) {
+          const int k = tid * m + q;
+          v0 = v1 = 0.0;
+          if (tid < G && k < n) {
+            const double x0 = P.X(k)[i + (int64_t)d * i].x, x1 = P.X(k)[j + (int64_t)d * j].x;
+            v0 = x0 * x0;
+            v1 = x1 * x1;
           }
-          P.sq[h] = s0;
-          P.sq[10 * H + h] = s1;
+        }, s0, s1);
+        const double r = lane_tree(s0, s1, G) / (tid == 0 ? P.w[i + (int64_t)d * i].x : P.w[j + (int64_t)d * j].x);
+        angles(P, __shfl_sync(kFull, r, 0), __shfl_sync(kFull, r, 1));
+      } else {
+        // the (i, j) blocks of every matrix and of w, then candidates until the master is done
+        for (int e = tid - 32; e < 4 * (n + 1); e += kWsdThreads - 32) {
+          const double2* A = (e >> 2) < n ? P.X(e >> 2) : P.w;
+          P.blk[e] = A[(e & 2 ? j : i) + (int64_t)d * (e & 1 ? j : i)];
+        }
+        for (;;) {
+          role_sync();
+          const int which = P.ctl[0];
+          if (!which) break;
+          eval_items(P.blk, which == 1 ? P.cand0 : P.cand, P.sq, P.wd, n, P.lgG, P.m);
+          role_sync();
         }
       }
-      bsync();
-      const double* sums = tree_levels(P, 1);
-      double xo0 = 0, xo1 = 0;
-      if (master) {  // xold / w of the pair, lanes 0 and 1
-        const int l = tid;
-        const double r = (l == 0 ? sums[0] : sums[10 * H]) / (l == 0 ? P.blk[4 * n + 0].x : P.blk[4 * n + 3].x);
-        xo0 = __shfl_sync(kFull, r, 0);
-        xo1 = __shfl_sync(kFull, r, 1);
-      }
-      double2 c, s;
-      angles(P, xo0, xo1, c, s);
-      if (tid == 0) {
-        P.rot[0] = c;
-        P.rot[1] = s;
-      }
-      bsync();
-      c = P.rot[0];
-      s = P.rot[1];
+      const double2 c = P.rot[0], s = P.rot[1];
       // givensRotation of every matrix and of w, columns i, j; givensTrafoRotation of T
       for (int e = tid; e < (n + 2) * d; e += kWsdThreads) {
         const int mi = e / d, r = e % d;
@@ -728,11 +772,7 @@ __device__ double offdiag(const Prob& P) {
 
 // shared memory of the fixed part of a problem with n matrices of order d
 __host__ __device__ int64_t wsd_fixed_bytes(int n, int d) {
-  int64_t p2 = 1;
-  while (p2 < n) p2 <<= 1;
-  const int64_t H = p2 > 1 ? p2 / 2 : 1;
-  const int64_t b = 16 * (4 * (int64_t)(n + 1) + 20 + 2) + 8 * (40 * H + 20 + (int64_t)n * d + 2) + 16 +
-                    4 * kEigLevels * 32;
+  const int64_t b = 16 * (4 * (int64_t)(n + 1) + 40 + 2) + 8 * (20 + 20 + (int64_t)n * d + 2) + 16;
   return (b + 15) / 16 * 16;
 }
 
@@ -750,22 +790,39 @@ __global__ void __launch_bounds__(kWsdThreads, 1) k_wsd(const WSDTask* __restric
   {
     int p2 = 1;
     while (p2 < n) p2 <<= 1;
-    P.H = p2 > 1 ? p2 / 2 : 1;
-    P.lgH = 0;
-    while ((1 << P.lgH) < P.H) ++P.lgH;
+    const int G = p2 <= 32 ? min(p2, 8) : 32;
+    P.lgG = 31 - __clz(G);
+    P.m = p2 / G;
   }
   P.blk = reinterpret_cast<double2*>(wsd_smem);
-  P.cand = P.blk + 4 * (n + 1);
+  P.cand0 = P.blk + 4 * (n + 1);
+  P.cand = P.cand0 + 20;
   P.rot = P.cand + 20;
   P.sq = reinterpret_cast<double*>(P.rot + 2);
-  P.wd = P.sq + 40 * P.H;
+  P.wd = P.sq + 20;
   P.tr = P.wd + 20;
   P.val = P.tr + (int64_t)n * d;
   P.ctl = reinterpret_cast<int*>(P.val + 2);
   {
-    uint32_t* lut = reinterpret_cast<uint32_t*>(P.ctl + 4);
-    for (int i = tid; i < kEigLevels * 32; i += kWsdThreads) lut[i] = (&c_eig_lut[0][0])[i];
-    P.lut = lut;
+    const int l = tid & 31;
+#pragma unroll
+    for (int k = 0; k < kEigLevels; ++k) P.eig[k] = lane_op(c_eig_lut[k][l], l);
+    // grad_pre's terms: y[i + 3 j] in lane 1 + i + 3 j, lane 31 zero
+    P.den = l < 2 ? 2 * kDelta : (l < 4 ? kDelta * kDelta : 4 * kDelta * kDelta);
+    P.zh = 1.0 / P.den;
+    P.zl = __fma_rn(neg_bits(P.zh), P.den, 1.0) / P.den;
+    const uint32_t A = l == 0 || l == 2 ? 6 : (l == 1 || l == 3 ? 8 : 9);
+    const uint32_t B = l == 0 || l == 2 ? 4 : (l == 1 || l == 3 ? 2 : 1);
+    const uint32_t C = l < 2 ? 31 : (l < 4 ? 5 : 3), D = l < 4 ? 31 : 7;
+    P.diff = A | (B << 5) | (C << 10) | (D << 15) | ((l < 2 ? 1u : 0u) << 20);
+    const int k = l & 15, q = l < 16 ? (k - 1) % 3 : (k - 1) / 3;
+    P.dx = k < 1 || k > 9 ? -0.0 : (q == 0 ? -kDelta : (q == 1 ? 0.0 : kDelta));
+    if (tid < 32) {
+      double z;
+      const double r = put_candidates(P, P.cand0, 2 * kEps * kEps, kEps, -kEps, kEps, -kEps, z);
+      P.c0 = __shfl_sync(kFull, r, 0);
+      P.sab0 = __shfl_sync(kFull, r, 10);
+    }
   }
   // the matrices in shared memory when they fit, else in the task's scratch
   const int64_t fixed = wsd_fixed_bytes(n, d);
