@@ -590,11 +590,18 @@ __device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4
 // pre-pass: the image of W for one unit -- per 16-k step and digit a plane of
 // 3 np rows, -Wi at row n, Wr at np + n, Wi at 2 np + n (rows past the last
 // column zero) -- and the unit's row exponents F_n.  Thread (n, q) takes row
-// n of the steps q, q + 4, ...  HP units (group, chunk): W(i, k) = conj(A[k; i]);
+// n of the 8-k core rows q, q + 8, ...  HP units (group, chunk): W(i, k) = conj(A[k; i]);
 // ACC units (task, term): W(j, k) = alpha H(j, k), alpha I for identity terms;
 // MP units (task): W(j, k) = alpha h(j, k).
+// What bounds it: a unit is one block, and most launches have fewer blocks than
+// SMs, so its time is one thread's chain: the loads, then about 20 instructions
+// per digit pair.  A thread takes 8 k and keeps them from the search for the
+// row's largest element (16 k, loaded twice, by 256 threads: 15 to 19 us a
+// launch; the 16-mode sweep 977 -> 875 us, the 64-mode one 7.80 -> 7.47 ms,
+// bonds above 64 33.1 -> 32.4 ms, three states overlapped).
+constexpr int kTcsImgThreads = 512;
 template <int OP>
-__global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restrict__ units, int64_t first) {
+__global__ void __launch_bounds__(kTcsImgThreads) k_tcs_img(TcsArgs g, const int2* __restrict__ units, int64_t first) {
   int2 u = OP == TCS_MP ? make_int2(g.mp_tasks[first + blockIdx.x], 0) : units[first + blockIdx.x];
   const int n = threadIdx.x & 63, q = threadIdx.x >> 6;
   int np, ncols, c0, steps;  // the unit's column block and image
@@ -627,15 +634,15 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
     steps = tc_steps(k);
     img += (size_t)(OP == TCS_MP ? cb : u.y) * hp_tc_chunk_bytes(np, steps);
   }
-  // the 16 values of row n at step ks
-  auto load16 = [&](int ks, float4 (&v)[16]) {
+  // the eight values of row n in core row hs
+  auto load8 = [&](int hs, float4 (&v)[8]) {
     if (OP == TCS_HP) {
       const HpTcGroup& G = g.groups[u.x];
-      const int K = G.before * G.after, k0 = u.y * hp_tc_kc(G.ap) + ks * kChunkK;
+      const int K = G.before * G.after, k0 = u.y * hp_tc_kc(G.ap) + hs * 8;
       const float4* __restrict__ A = reinterpret_cast<const float4*>(G.A);
       KWalk w(min(k0, K), G.before);
 #pragma unroll
-      for (int kk = 0; kk < 16; ++kk) {
+      for (int kk = 0; kk < 8; ++kk) {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < ncols && k0 + kk < K) {
           x = __ldg(A + w.off(c0 + n, G.before, G.a));
@@ -651,8 +658,8 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
       const bool one = t.alpha.x == 1.0 && t.alpha.y == 0.0;
       const float4* __restrict__ H = reinterpret_cast<const float4*>(t.h);
 #pragma unroll
-      for (int kk = 0; kk < 16; ++kk) {
-        const int k = ks * kChunkK + kk;
+      for (int kk = 0; kk < 8; ++kk) {
+        const int k = hs * 8 + kk;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < ncols && k < t.a_in) {
           x = __ldg(H + c0 + n + (int64_t)t.a_out * k);
@@ -667,8 +674,8 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
       const float4 cf = DF64::coef(alpha);
       const float4* __restrict__ H = reinterpret_cast<const float4*>(tm.H);
 #pragma unroll
-      for (int kk = 0; kk < 16; ++kk) {
-        const int k = ks * kChunkK + kk;
+      for (int kk = 0; kk < 8; ++kk) {
+        const int k = hs * 8 + kk;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < ncols && k < T.d) {
           if (H) x = DF64::mul(cf, __ldg(H + c0 + n + (int64_t)T.d * k));
@@ -681,50 +688,53 @@ __global__ void __launch_bounds__(256) k_tcs_img(TcsArgs g, const int2* __restri
   __shared__ int fx[64];  // largest |W| of a row as an integer, then its exponent
   if (threadIdx.x < 64) fx[threadIdx.x] = 0;
   __syncthreads();
+  // the largest |W| of this thread's core rows, the first one last: its values
+  // stay in registers (up to 64 k a thread has no other)
+  constexpr int kS = kTcsImgThreads / 64;
+  const int last = 2 * steps - 1 - q, nhs = last >= 0 ? last / kS + 1 : 0;
+  float4 v[8];
   int m = 0;
-  for (int ks = q; ks < steps; ks += 4) {
-    float4 v[16];
-    load16(ks, v);
+#pragma unroll 1
+  for (int i = nhs - 1; i >= 0; --i) {
+    load8(q + kS * i, v);
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) m = max(m, max(fmag(v[kk].x), fmag(v[kk].z)));
+    for (int kk = 0; kk < 8; ++kk) m = max(m, max(fmag(v[kk].x), fmag(v[kk].z)));
   }
   atomicMax(&fx[n], m);
   __syncthreads();
-  if (n < np) {
+  if (n < np && nhs > 0) {
     const float f = row_factor(row_exponent(fx[n]));
     const int rows = 3 * np, plane = rows * 32;
-    for (int ks = q; ks < steps; ks += 4) {
-      float4 v[16];
-      load16(ks, v);
-      unsigned char* base = img + (size_t)ks * kDig * plane;
+#pragma unroll 1
+    for (int i = 0;;) {
+      const int hs = q + kS * i, c = hs & 1;
+      unsigned char* base = img + (size_t)(hs >> 1) * kDig * plane;
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {  // the two 8-k core rows of the step
-        uint32_t wr[kDig][4], wi[kDig][4];
+      for (int part = 0; part < 2; ++part) {
+        uint32_t w[kDig][4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-          float d0[kDig], d1[kDig], e0[kDig], e1[kDig];
-          digits_f32(v[8 * c + 2 * p].x, v[8 * c + 2 * p].y, f, d0);
-          digits_f32(v[8 * c + 2 * p + 1].x, v[8 * c + 2 * p + 1].y, f, d1);
-          digits_f32(v[8 * c + 2 * p].z, v[8 * c + 2 * p].w, f, e0);
-          digits_f32(v[8 * c + 2 * p + 1].z, v[8 * c + 2 * p + 1].w, f, e1);
+          float d0[kDig], d1[kDig];
+          digits_f32(part ? v[2 * p].z : v[2 * p].x, part ? v[2 * p].w : v[2 * p].y, f, d0);
+          digits_f32(part ? v[2 * p + 1].z : v[2 * p + 1].x, part ? v[2 * p + 1].w : v[2 * p + 1].y, f, d1);
 #pragma unroll
-          for (int d = 0; d < kDig; ++d) {
-            wr[d][p] = pack_bf16(d0[d], d1[d]);
-            wi[d][p] = pack_bf16(e0[d], e1[d]);
-          }
+          for (int d = 0; d < kDig; ++d) w[d][p] = pack_bf16(d0[d], d1[d]);
         }
 #pragma unroll
         for (int d = 0; d < kDig; ++d) {
           unsigned char* pl = base + (size_t)d * plane;
-          const uint4 re = make_uint4(wr[d][0], wr[d][1], wr[d][2], wr[d][3]);
-          const uint4 im = make_uint4(wi[d][0], wi[d][1], wi[d][2], wi[d][3]);
-          const uint4 nim =
-              make_uint4(im.x ^ 0x80008000u, im.y ^ 0x80008000u, im.z ^ 0x80008000u, im.w ^ 0x80008000u);
-          *reinterpret_cast<uint4*>(pl + core_off(n, c, rows)) = nim;
-          *reinterpret_cast<uint4*>(pl + core_off(np + n, c, rows)) = re;
-          *reinterpret_cast<uint4*>(pl + core_off(2 * np + n, c, rows)) = im;
+          const uint4 x = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+          if (part == 0) {
+            *reinterpret_cast<uint4*>(pl + core_off(np + n, c, rows)) = x;
+          } else {
+            *reinterpret_cast<uint4*>(pl + core_off(n, c, rows)) =
+                make_uint4(x.x ^ 0x80008000u, x.y ^ 0x80008000u, x.z ^ 0x80008000u, x.w ^ 0x80008000u);
+            *reinterpret_cast<uint4*>(pl + core_off(2 * np + n, c, rows)) = x;
+          }
         }
       }
+      if (++i >= nhs) break;
+      load8(q + kS * i, v);
     }
   }
   if (threadIdx.x < 64)
@@ -1372,7 +1382,7 @@ cudaError_t launch_tf(const MPTask* tasks, const int2* tiles, int64_t first_tile
 
 template <int OP>
 cudaError_t launch_tcs(const TcsArgs& g, const int2* img_units, int64_t first_unit, int64_t n_units, cudaStream_t s) {
-  if (n_units > 0) k_tcs_img<OP><<<(unsigned)n_units, 256, 0, s>>>(g, img_units, first_unit);
+  if (n_units > 0) k_tcs_img<OP><<<(unsigned)n_units, kTcsImgThreads, 0, s>>>(g, img_units, first_unit);
   if (OP == TCS_HP) k_hp_ex<<<dim3((unsigned)g.n_items, kRows / 32), 256, 0, s>>>(g);
   unsigned grid = 0;
   cudaError_t e = tc_grid(g.n_items, &grid);
