@@ -907,9 +907,9 @@ __device__ __forceinline__ int tcs_row_max(const int (&ex)[kTcsExWarps][kRows], 
 // Every wait is bounded (all lanes of a warp give up together): a wait that
 // runs out sets the status word, and the CTA drains its issued MMAs, frees
 // tensor memory and returns.
-// What bounds it, per 128 x 64 unit of 64 k: a 16-k step (42 MMAs, 24 KB of W
-// and 48 KB of X's digits through shared memory) takes 4.9 k cycles, all of it
-// shared-memory bandwidth, and the epilogue 6 to 10 k cycles for each unit that
+// What bounds it, per 128 x 64 unit of 64 k: a 16-k step (56 MMAs that read 57 KB
+// of X's and 43 KB of W's digits from shared memory) takes 4.9 k cycles, all of
+// it shared-memory bandwidth, and the epilogue 6 to 10 k cycles for each unit that
 // it holds up the next unit's MMAs.  The rows' exponents need all of X before
 // its first digit: in the producers, ahead of every unit, that pass took 9 to
 // 15 k cycles; in warps of its own it runs under the previous unit (a CTA's
