@@ -166,7 +166,7 @@ def _rho_weighted_err(tree, dpsi, ref, rho):
 # dram__bytes_write.sum over all launches of one sweep of the 64-mode
 # workload, from one ncu capture of that sweep; the summary is committed
 # beside the other profiles and named in TRAFFIC_SOURCE)
-TRAFFIC = {0: 1531.5e6, 1: 3245.5e6, 2: 2104.8e6}
+TRAFFIC = {0: 1525.3e6, 1: 3148.2e6, 2: 2296.4e6}
 TRAFFIC_SOURCE = ("ncu capture of one sweep of the 64-mode workload, k_tcs launches only "
                   "(profiles/launches_sweep_64mode_compressed_df64_tc.md)")
 
