@@ -599,9 +599,11 @@ __device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4
 // row's largest element (16 k, loaded twice, by 256 threads: 15 to 19 us a
 // launch; the 16-mode sweep 977 -> 875 us, the 64-mode one 7.80 -> 7.47 ms,
 // bonds above 64 33.1 -> 32.4 ms, three states overlapped).
+// Launches of more units than SMs gain from two blocks per SM (64 registers, a
+// few spilled; at 88 to 116 one block: 64 modes 7.48 -> 7.40 ms).
 constexpr int kTcsImgThreads = 512;
 template <int OP>
-__global__ void __launch_bounds__(kTcsImgThreads) k_tcs_img(TcsArgs g, const int2* __restrict__ units, int64_t first) {
+__global__ void __launch_bounds__(kTcsImgThreads, 2) k_tcs_img(TcsArgs g, const int2* __restrict__ units, int64_t first) {
   int2 u = OP == TCS_MP ? make_int2(g.mp_tasks[first + blockIdx.x], 0) : units[first + blockIdx.x];
   const int n = threadIdx.x & 63, q = threadIdx.x >> 6;
   int np, ncols, c0, steps;  // the unit's column block and image
