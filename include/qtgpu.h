@@ -82,14 +82,14 @@ extern "C" {
 /* Double-float arithmetic as QT_PREC_DF64, with the mode products, hole
  * products and last-index accumulations of shapes from 32 to 112 on the
  * fifth-generation tensor cores (tcgen05.mma, accumulators in tensor memory;
- * beyond 64 output columns in column blocks of at most 48, accumulations
- * only in the compressed plan's sweep).  Every operand row is scaled by a
+ * beyond 64 output columns in column blocks of at most 48, mode products from
+ * 128 rows on, accumulations only in the compressed plan's sweep).  Every operand row is scaled by a
  * power of two and cut into seven signed digits of at most eight bits by
  * error-free splits, digit products are exact in bf16, each level of digit
  * pairs sums exactly in fp32 as far as tensor memory holds separate level
- * accumulators (all seven for outputs padded to <= 32 columns, five for 48,
- * four for 64, at most five beyond 64 reduction indices or output columns,
- * the last taking the remaining levels), and the levels are
+ * accumulators (all seven for column blocks padded to <= 32, six for 40, five
+ * for 48, four for 56 and 64 and for hole products of 33..64 columns, the last
+ * taking the remaining levels), and the levels are
  * recombined in double-float.  The error is relative to the row maxima of
  * the operands: 2^-49 of the row scale per value, plus the fp32 rounding of
  * the last level accumulator.  Parity tolerance 1e-10 per contraction and

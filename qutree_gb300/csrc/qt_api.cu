@@ -526,6 +526,8 @@ int qt_prepare(qt_ctx* c, int flavour) {
     t.ws = s.ws;
     t.rows = s.rows;
     t.cols = s.cols;
+    t.comp = s.comp;
+    t.pad = 0;
     hp.push_back(t);
   }
   std::vector<qt::HpTcGroup> hp_tc;
@@ -1274,6 +1276,7 @@ int qt_hole_product(qt_ctx* c, void* S, const void* A, const void* B, int64_t be
   t.kchunk = 0;
   t.ws = 0;
   t.rows = t.cols = 4;
+  t.comp = t.pad = 0;
   cudaError_t e = qt::launch_single_hp(t, c->stream, nullptr);
   if (e != cudaSuccess) return cuda_fail(c, e, "qt_hole_product");
   c->launches += 1;
@@ -1829,6 +1832,7 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
     t.kchunk = 0;
     t.ws = 0;
     t.rows = t.cols = 4;
+    t.comp = t.pad = 0;
     // the split by fixed ranges of the reduction, whose order of additions the
     // Krylov sweep's results are sensitive to
     cudaError_t e = qt::launch_hp_split(t, hpws, ws_elems, c->stream);

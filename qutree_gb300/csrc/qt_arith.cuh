@@ -111,6 +111,14 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float bh, float bl)
   hi = s;
   lo = e;
 }
+__device__ __forceinline__ void df_add_comp(float& hi, float& lo, float& c, float bh, float bl) {
+  float s, e, l, e1, e2;
+  df_two_sum(hi, bh, s, e);
+  df_two_sum(lo, bl, l, e1);
+  df_two_sum(l, e, lo, e2);
+  hi = s;
+  c = __fadd_rn(c, __fadd_rn(e1, e2));
+}
 __device__ __forceinline__ float2 df_split(double x) {
   const float h = __double2float_rn(x);
   const float l = __double2float_rn(x - (double)h);
@@ -140,6 +148,12 @@ struct DF64 {
   static __device__ __forceinline__ void add(A& acc, const S& b) {
     df_add(acc.x, acc.y, b.x, b.y);
     df_add(acc.z, acc.w, b.z, b.w);
+  }
+  // the same with the low words' own rounding errors collected in c.x, c.z
+  // (add them to the low words at the end)
+  static __device__ __forceinline__ void add_comp(A& acc, float4& c, const S& b) {
+    df_add_comp(acc.x, acc.y, c.x, b.x, b.y);
+    df_add_comp(acc.z, acc.w, c.z, b.z, b.w);
   }
   static __device__ __forceinline__ C coef(double2 c) {
     const float2 r = df_split(c.x), i = df_split(c.y);

@@ -42,6 +42,7 @@ struct HPTask {
   int kchunk;
   int64_t ws;  // workspace offset (elements) of the partial tiles
   int rows, cols;  // outputs per thread along i and j (1..4)
+  int comp, pad;   // comp: the sum of the partial tiles is compensated (k_hp_sum)
 };
 
 // hole products on the tensor cores (qt_umma.cu, double-float plans): groups
@@ -74,7 +75,7 @@ struct HpTcGroup {
 // (qutree_gb300/autotune.py).  65 keeps a kind off the tensor cores.
 // Shapes beyond 64 output columns (the accumulator tile's most) are cut into
 // column blocks, each an item of its own that produces the row digits again:
-// the 64-mode tree with bonds 32..96 runs its sweep in 36.5 ms this way,
+// the 64-mode tree with bonds 48..96 runs its sweep in 37.3 ms this way,
 // 157 ms with the shapes from 65 on the FP32 pipe.
 constexpr int kTcCols = 64;     // output columns of one accumulator tile
 constexpr int kTcMaxDim = 112;  // seven 16-k steps; the planner's largest bond
@@ -105,8 +106,8 @@ inline bool mp_tc_wide(int a_in, int a_out, int64_t rows, int lo = 32) {
 QT_HD constexpr int hp_tc_kc(int ap) { return ap > 32 ? 2 * kHpTcChunk : kHpTcChunk; }
 // column blocks of n output columns, and the columns of a full one (a multiple
 // of 8; the last block has the rest).  Beyond kTcCols a block has at most 48:
-// five level accumulators, whose last one holds levels 4..6 only (2^-52 of
-// the row scales), below the digits' truncation.
+// six or seven level accumulators up to 40 columns, five for 48 (whose units
+// take half of the k, tcs_halve).
 QT_HD constexpr int tc_blocks(int n) { return n <= kTcCols ? 1 : (n + 47) / 48; }
 QT_HD constexpr int tc_width(int n) { return ((n + tc_blocks(n) - 1) / tc_blocks(n) + 7) & ~7; }
 // 16-k steps of the operand image of a mode product or accumulation over k
@@ -318,6 +319,7 @@ struct Stage {
   int64_t ati0 = 0, nati = 0;  // accumulation stage: its tensor-core items (acc_tc_items)
   int64_t atu0 = 0, natu = 0;  // and the units of its image pre-pass (acc_tc_imgs)
   int64_t atc_units = 0;       // units (terms) of all its items
+  bool tc_wide = false;        // tensor-core work of more than kTcCols columns
   double flops = 0;  // executed flops of the stage
   double bytes = 0;  // algorithmic bytes: operands read once, results written once
 };
@@ -413,6 +415,7 @@ struct Plan {
     int splits = 1, kchunk = 0;
     int64_t ws = 0;
     int rows = 4, cols = 4;
+    int comp = 0;
   };
   struct SAccTerm {
     Ref H;  // buf == -1: identity
@@ -758,7 +761,8 @@ cudaError_t probe_fp64_peak(cudaStream_t s, double* tflops);
 // qualifies when it is not diagonal and a_in, a_out <= 64.  A wait that runs
 // out writes a non-zero code to *status.
 cudaError_t launch_mp_tc(bool oz, const MPTask* tasks, const int2* tiles, int64_t first_tile, int64_t n_tiles,
-                         const int* tc_tasks, int64_t first_task, int64_t n_tasks, int* status, cudaStream_t s);
+                         const int* tc_tasks, int64_t first_task, int64_t n_tasks, bool wide, int* status,
+                         cudaStream_t s);
 constexpr int kMpOzRows = 32;  // the planner's tensor-core tiles: kMpOzSub x kMpOzRows = 128 rows (b, c)
 constexpr int kMpOzSub = 4;
 // bytes per task of the h operand's shared-memory image (written by the
@@ -771,13 +775,13 @@ inline int64_t mp_oz_h_bytes() { return kMpOzImageBytes; }
 // (group, chunk) of the pre-pass that writes A's images
 cudaError_t launch_hp_tc(const HPTask* tasks, const HpTcGroup* groups, const int4* items, int64_t first_item,
                          int64_t n_items, const int2* img_units, int64_t first_unit, int64_t n_units,
-                         double2* ws, int* status, cudaStream_t s);
+                         double2* ws, bool wide, int* status, cudaStream_t s);
 // accumulations on the tensor cores: items (task, 128-row block, units
 // before the item in the stage, 0), one unit per term; image units (task,
 // term) of the pre-pass that writes alpha H_t
 cudaError_t launch_acc_tc(const AccTask* tasks, const AccTerm* terms, const int4* items, int64_t first_item,
                           int64_t n_items, int64_t units, const int2* img_units, int64_t first_unit,
-                          int64_t n_units, int* status, cudaStream_t s);
+                          int64_t n_units, bool wide, int* status, cudaStream_t s);
 // weighted simultaneous diagonalisation, one warp per task (qt_wsd.cu)
 // max_n / max_d bound the tasks' matrix counts and orders (shared memory)
 cudaError_t launch_wsd(const WSDTask* tasks, const WSDTerm* terms, int64_t first, int64_t n, int max_n,

@@ -440,7 +440,10 @@ __global__ void __launch_bounds__(kThreads) k_hp_sum_one(HPTask t, const typenam
 }
 
 // S = sum over the k ranges of the partial tiles, in range order; kHpSumChunks
-// blocks of 256 outputs per task (the loads of four ranges in flight)
+// blocks of 256 outputs per task (the loads of four ranges in flight).  In
+// stages with wide tensor-core products (HPTask::comp) the low words' rounding
+// errors are kept too: a hundred ranges, added without, cost the energy of an
+// 8-mode tree with bonds 80..112 1e-14 -> 5e-14 of its value, with it 4e-15.
 constexpr int kHpSumChunks = 16;
 template <class P>
 __global__ void __launch_bounds__(kThreads) k_hp_sum(const HPTask* __restrict__ tasks, int64_t task0,
@@ -455,6 +458,17 @@ __global__ void __launch_bounds__(kThreads) k_hp_sum(const HPTask* __restrict__ 
   for (int64_t e = (int64_t)(blockIdx.x % kHpSumChunks) * kThreads + threadIdx.x; e < n;
        e += (int64_t)kHpSumChunks * kThreads) {
     A acc = P::zero();
+    if constexpr (std::is_same<P, DF64>::value) {
+      if (t.comp) {
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int z = 0; z < t.splits; ++z) DF64::add_comp(acc, c, ws[t.ws + z * n + e]);
+        acc.y = __fadd_rn(acc.y, c.x);
+        acc.w = __fadd_rn(acc.w, c.z);
+        Sp[e] = P::fin(acc);
+        continue;
+      }
+    }
 #pragma unroll 4
     for (int z = 0; z < t.splits; ++z) P::add(acc, ws[t.ws + z * n + e]);
     Sp[e] = P::fin(acc);
@@ -2049,7 +2063,7 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       }
       if (st.noz > 0) {
         cudaError_t e = launch_mp_tc(std::is_same<P, DF64>::value, t.mp, t.mp_oz_tiles, st.oz0, st.noz,
-                                     t.mp_oz_tasks, st.ozt0, st.nozt, t.status, s);
+                                     t.mp_oz_tasks, st.ozt0, st.nozt, st.tc_wide, t.status, s);
         if (e != cudaSuccess) return e;
       }
       break;
@@ -2070,7 +2084,7 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       if (st.nhti > 0) {
         if (!std::is_same<P, DF64>::value) return cudaErrorInvalidValue;  // the planner emits none
         cudaError_t e = launch_hp_tc(t.hp, t.hp_tc_groups, t.hp_tc_items, st.hti0, st.nhti, t.hp_tc_imgs, st.htu0,
-                                     st.nhtu, reinterpret_cast<double2*>(t.hp_ws), t.status, s);
+                                     st.nhtu, reinterpret_cast<double2*>(t.hp_ws), st.tc_wide, t.status, s);
         if (e != cudaSuccess) return e;
       }
       if (st.aux)
@@ -2090,7 +2104,7 @@ cudaError_t launch_stage_p(const Stage& st, const DevTables& t, double eps, int 
       if (st.nati > 0) {
         if (!std::is_same<P, DF64>::value) return cudaErrorInvalidValue;  // the planner emits none
         cudaError_t e = launch_acc_tc(t.acc, t.acc_terms, t.acc_tc_items, st.ati0, st.nati, st.atc_units,
-                                      t.acc_tc_imgs, st.atu0, st.natu, t.status, s);
+                                      t.acc_tc_imgs, st.atu0, st.natu, st.tc_wide, t.status, s);
         if (e != cudaSuccess) return e;
       }
       break;

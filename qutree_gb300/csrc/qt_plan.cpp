@@ -148,9 +148,13 @@ class Builder {
   Plan& P;
   // Contractions of more than 64 columns on the tensor cores.  The digits'
   // error is relative to a row's largest operand, a double-float
-  // multiply-add's to each product.  The sweep's error does not tell them apart
-  // (bonds 66..96 against the oracle: 2.9e-13, double-float 2.6e-13), but
-  // accumulations that cancel do: (H Phi) rhoinv^T + Phi M2^T with H Phi formed
+  // multiply-add's to each product.  With the levels recombined as in
+  // tcs_levels and the partial tiles as in k_hp_sum they are the more accurate
+  // of the two (8 modes, all bonds 80, 88, 96, 100 or 112, against complex128:
+  // density matrices 2.6e-15..3.4e-15, multiply-adds 4.3e-15..4.8e-15; energies
+  // 2e-15..6e-15, 3e-15..2e-14; gradients 1.3e-13..1.9e-13, 1.6e-13..3.1e-13; the
+  // derivatives, limited by the density inverses, alike), except in
+  // accumulations that cancel: (H Phi) rhoinv^T + Phi M2^T with H Phi formed
   // (the frozen-matrix derivative; reference and grouped plans) gives 2.3e-12
   // instead of 3.3e-13.  Those, and the SCF segments, whose Krylov vectors
   // amplify any change of rounding, keep the FP32 pipe beyond 64.
@@ -188,6 +192,7 @@ class Builder {
   int64_t mats_cursor = 0;
   double stage_flops_mark = 0;
   int64_t stage_oz_ = 0;  // bytes of operand images assigned in the stage being emitted
+  bool stage_wide_ = false;  // it has tensor-core work of more than kTcCols columns
   std::map<std::vector<int>, int64_t> hslot_of_key, cslot_of_key;
 
   double stage_bytes(int kind, int64_t t0, int64_t t1) const {
@@ -510,6 +515,11 @@ class Builder {
       }
     }
     if (P.hp_tensor && hp_tensor_items(t0, t1, tc, ws)) split = true;
+    // with wide tasks on the tensor cores there are many more ranges to add
+    // than with all tasks above: one per chunk of theirs, and of the others
+    // (whose kchunk follows from their own work alone)
+    for (int64_t t = t0; t < t1; ++t) stage_wide_ |= tc[t - t0] && P.hp[t].a > kTcCols;
+    for (int64_t t = t0; t < t1; ++t) P.hp[t].comp = stage_wide_ ? 1 : 0;
     // tiles grouped by micro-tile shape: one launch per shape
     for (int shape = 0; shape < 16; ++shape) {
       const int64_t first = (int64_t)P.hp_tiles.size();
@@ -612,6 +622,7 @@ class Builder {
       Plan::SAcc& a = P.acc[t];
       if (a.count < 1 || !acc_tc_eligible(a.rows, a.d, P.tune.acc) || (a.d > kTcCols && !wide_acc)) continue;
       tc[t - t0] = 1;
+      stage_wide_ |= a.d > kTcCols;
       a.tc_img = stage_oz_;
       const int nb = tc_blocks(a.d);
       stage_oz_ += (int64_t)a.count * nb * hp_tc_chunk_bytes(tc_width(a.d), tc_steps(a.d));
@@ -638,6 +649,7 @@ class Builder {
     const int64_t seg0 = (int64_t)P.hp_segs.size();
     const int64_t hti0 = (int64_t)P.hp_tc_items.size(), htu0 = (int64_t)P.hp_tc_imgs.size();
     stage_oz_ = 0;  // operand images are rewritten by every stage's pre-pass
+    stage_wide_ = false;
     if (kind == ST_HP) split = hp_split(t0, t1, tile0, tile1);
     const int64_t oz0 = (int64_t)P.mp_oz_tiles.size();
     const int64_t ozt0 = (int64_t)P.mp_oz_tasks.size();
@@ -685,6 +697,7 @@ class Builder {
     s.atu0 = atu0;
     s.natu = (int64_t)P.acc_tc_imgs.size() - atu0;
     s.atc_units = atc_units;
+    s.tc_wide = stage_wide_;
     P.stages.push_back(s);
   }
 
@@ -699,6 +712,7 @@ class Builder {
       const bool beyond = wide && P.hp_tensor && mp_tc_wide(m.a_in, m.a_out, rows, P.tune.mp);
       if (m.diag || !(beyond || mp_tc_eligible(m.a_in, m.a_out, P.tune.mp))) continue;
       oz[t - t0] = 1;
+      stage_wide_ |= beyond;
       m.oz_h = stage_oz_;
       // double-float plans: the sum-of-products kernel's image of alpha h;
       // complex64 plans: the split-TF32 image

@@ -542,9 +542,29 @@ __device__ __forceinline__ void tcs_range(const TcsArgs& g, int64_t& i0, int64_t
 // units, 16-k steps per unit and of the operand image
 struct TcsItem {
   int np, ncols, c0, nunits, nks, isteps;
-  int nl;  // level accumulators
+  int nl;     // level accumulators
+  bool wide;  // more than kTcCols columns in all
+  int half;   // 1: every term or chunk is two units, the second from step n0 on
+  int n0;
+  // unit u's term or chunk, its first 16-k step, its steps
+  __device__ __forceinline__ int term(int u) const { return u >> half; }
+  __device__ __forceinline__ int step0(int u) const { return u & half ? n0 : 0; }
+  __device__ __forceinline__ int steps(int u) const { return !half ? nks : u & 1 ? nks - n0 : n0; }
 };
-template <int OP>
+// Bonds beyond 64 whose column blocks are wider than 40 (81..96: 48 columns)
+// have room for five level accumulators only.  The tensor core truncates the
+// sums into the last one, which holds levels 4..6, and the error grows with the
+// number of MMAs on it: these units take half of the k.  Density matrices at
+// bonds 88 and 96 against complex128: 4.8e-15 -> 3.4e-15 (multiply-adds 4.7e-15;
+// six and seven accumulators 2.7e-15).
+template <bool WIDE>
+__device__ __forceinline__ void tcs_halve(TcsItem& v, int n) {
+  v.wide = WIDE && n > kTcCols;
+  v.half = v.wide && v.np > 40 && v.nks > 1 ? 1 : 0;
+  v.n0 = (v.nks + 1) >> 1;
+  v.nunits <<= v.half;
+}
+template <int OP, bool WIDE>
 __device__ __forceinline__ TcsItem tcs_item(const TcsArgs& g, int4 itm) {
   TcsItem v;
   if (OP == TCS_HP) {
@@ -554,9 +574,9 @@ __device__ __forceinline__ TcsItem tcs_item(const TcsArgs& g, int4 itm) {
     v.c0 = G.c0;
     v.nunits = itm.w - itm.z;
     v.nks = v.isteps = hp_tc_kc(G.ap) / kChunkK;
-    // 128-k chunks keep four accumulators (levels 0..2 exact up to 170 k);
-    // column blocks of wide bonds five (levels 0..3 exact up to 128 k)
-    v.nl = v.nks > 4 ? min(G.a > kTcCols ? 5 : 4, levels_for(G.ap)) : levels_for(G.ap);
+    // 128-k chunks of bonds up to 64 keep four accumulators (levels 0..2 exact up to 170 k)
+    v.nl = v.nks > 4 && G.a <= kTcCols ? 4 : levels_for(G.ap);
+    tcs_halve<WIDE>(v, G.a);
     return v;
   }
   int n, k;
@@ -575,16 +595,17 @@ __device__ __forceinline__ TcsItem tcs_item(const TcsArgs& g, int4 itm) {
   v.ncols = min(v.np, n - v.c0);
   v.nks = (k + kChunkK - 1) / kChunkK;
   v.isteps = tc_steps(k);
-  // beyond 64 k (up to 112) five accumulators at most (levels 0..3 exact up to 128 k)
-  v.nl = k > 64 ? min(5, levels_for(v.np)) : levels_for(v.np);
+  v.nl = levels_for(v.np);
+  tcs_halve<WIDE>(v, n);
   return v;
 }
+// operand image of term or chunk u
 template <int OP>
 __device__ __forceinline__ const unsigned char* tcs_image(const TcsArgs& g, int4 itm, int u, const TcsItem& I) {
   const int64_t cb = hp_tc_chunk_bytes(I.np, I.isteps);
   if (OP == TCS_HP) return g.groups[itm.x].img + (size_t)(itm.z + u) * cb;
   if (OP == TCS_MP) return static_cast<const unsigned char*>(g.mp[itm.x].oz_h) + (size_t)itm.w * cb;
-  return static_cast<const unsigned char*>(g.acc[itm.x].tc_img) + (size_t)(u + I.nunits * itm.w) * cb;
+  return static_cast<const unsigned char*>(g.acc[itm.x].tc_img) + (size_t)(u + (I.nunits >> I.half) * itm.w) * cb;
 }
 
 // pre-pass: the image of W for one unit -- per 16-k step and digit a plane of
@@ -812,9 +833,13 @@ __global__ void __launch_bounds__(256) k_hp_ex(TcsArgs g) {
 
 // Four columns of the accumulators (real parts from column 0 of `addr`, the
 // imaginary parts np columns on), their levels added in double-float: levels
-// 0..2 by two-sums, the others (at least one) into the low word.  All threads
-// of the warp.
-__device__ __forceinline__ void tcs_levels(uint32_t addr, int np, int NL, float (&v)[2][4], float (&l)[2][4]) {
+// 0..2 by two-sums, the others (at least one) into the low word.  Beyond 64
+// (wide) level 3 by a two-sum too: in the low word it rounds to 2^-45 of the
+// result, more than the double-float multiply-adds that these shapes replace
+// (bonds 65..112: density matrices 8.6e-15 with it, 5.0e-15 by multiply-adds);
+// up to 64 it would cost the 64-mode sweep 2%.  All threads of the warp.
+__device__ __forceinline__ void tcs_levels(uint32_t addr, int np, int NL, bool wide, float (&v)[2][4],
+                                           float (&l)[2][4]) {
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
     float lv[kDig][4];
@@ -823,6 +848,24 @@ __device__ __forceinline__ void tcs_levels(uint32_t addr, int np, int NL, float 
     for (int L = 0; L < kDig; ++L)
       if (L < 4 || L < NL) tmem_ld4(a + (uint32_t)(L * 2 * np), lv[L]);
     tmem_wait_ld();
+    if (wide) {
+      float rest[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int L = kDig - 1; L >= 4; --L)
+        if (L < NL) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) rest[i] = __fadd_rn(rest[i], lv[L][i]);
+        }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float s, t, e1, e2, e3;
+        df_two_sum(lv[0][i], lv[1][i], s, e1);
+        df_two_sum(s, lv[2][i], t, e2);
+        df_two_sum(t, lv[3][i], v[part][i], e3);
+        l[part][i] = __fadd_rn(__fadd_rn(__fadd_rn(e3, e2), e1), rest[i]);
+      }
+      continue;
+    }
     if (NL > 4) {
 #pragma unroll
       for (int L = 4; L < kDig; ++L)
@@ -917,7 +960,7 @@ __device__ __forceinline__ int tcs_row_max(const int (&ex)[kTcsExWarps][kRows], 
 // 15 k cycles; in warps of its own it runs under the previous unit (a CTA's
 // mode products 22.1 -> 17.2 k cycles a unit; 64-mode wide sweep 41.1 -> 37.2 ms,
 // 64-mode sweep 10.5 -> 10.1 ms, 16-mode 1.72 -> 1.67 ms).
-template <int OP>
+template <int OP, bool WIDE>
 __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
   extern __shared__ __align__(128) unsigned char tcs_raw[];
   TcsSmem& sm = *reinterpret_cast<TcsSmem*>(tcs_raw);
@@ -957,7 +1000,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
     uint32_t q = 0, un = 0;
     for (int64_t it = my0; it < my1 && ok; ++it) {
       const int4 itm = tcs_fetch<OP>(g, it);
-      const TcsItem I = tcs_item<OP>(g, itm);
+      const TcsItem I = tcs_item<OP, WIDE>(g, itm);
       const uint32_t nbytes = (uint32_t)(kDig * 3 * I.np * 32);
       int before = 0, K = 0;
       int64_t jump = 0;  // hole products: from the end of one run of b to the next
@@ -972,18 +1015,20 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
       for (int u = 0; u < I.nunits; ++u, ++un) {
         const int buf = (int)(un & 1);
         int64_t stride = 1;
-        const float4* p = tcs_row<OP>(g, itm, u, r, stride);
+        const int t = I.term(u), s0 = I.step0(u), nks = I.steps(u);
+        const float4* p = tcs_row<OP>(g, itm, t, r, stride);
         // the row's elements in order: `left` of them, the next one at p
         int left = 0, b = 0;
         if (OP == TCS_HP) {
-          const int k0 = (itm.z + u) * I.nks * kChunkK, c = k0 / before;
+          const int k0 = ((itm.z + t) * I.nks + s0) * kChunkK, c = k0 / before;
           b = k0 - c * before;
           if (p) {
             left = K - k0;
             p += b + (jump + before) * c;
           }
         } else if (p) {
-          left = K;
+          left = K - s0 * kChunkK;
+          p += stride * (s0 * kChunkK);
         }
         auto load8 = [&](float4 (&x)[8]) {
 #pragma unroll
@@ -1005,7 +1050,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
         load8(nx);
         int eb;
         if (OP == TCS_HP) {
-          eb = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + u) * kRows + r);
+          eb = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + t) * kRows + r);
         } else {
           if (!waited(&sm.bar.exready[buf], (un >> 1) & 1, 18)) break;
           eb = row_exponent(tcs_row_max(sm.ex[buf], r, OP == TCS_MP && stride == 1));
@@ -1013,8 +1058,8 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
           if (lane == 0) mbar_arrive(&sm.bar.exfree[buf]);
         }
         const float rowf = row_factor(eb);
-        const unsigned char* img = tcs_image<OP>(g, itm, u, I);
-        for (int ks = 0; ks < I.nks; ++ks, ++q) {
+        const unsigned char* img = tcs_image<OP>(g, itm, t, I) + (size_t)s0 * nbytes;
+        for (int ks = 0; ks < nks; ++ks, ++q) {
           const int s = q & 1;
           if (!waited(&sm.bar.empty[s], ((q >> 1) & 1) ^ 1, 11)) break;
           if (tid == 0) {
@@ -1029,7 +1074,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
             float4 x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = nx[i];
-            if (ks + hh < I.nks) load8(nx);  // the next half: (ks, 1) or (ks + 1, 0)
+            if (ks + hh < nks) load8(nx);  // the next half: (ks, 1) or (ks + 1, 0)
             const int off = core_off(r, hh, kRows);
 #pragma unroll
             for (int part = 0; part < 2; ++part) {
@@ -1061,7 +1106,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
         uint32_t q = 0, un = 0;
         for (int64_t it = my0; it < my1 && ok; ++it) {
           const int4 itm = tcs_fetch<OP>(g, it);
-          const TcsItem I = tcs_item<OP>(g, itm);
+          const TcsItem I = tcs_item<OP, WIDE>(g, itm);
           const int np = I.np, NL = I.nl;
           const uint32_t id = idesc_m128(1, 2 * np, false);
           const uint32_t lboA = (kRows / 8) * 128, lboN = (uint32_t)(3 * np / 8) * 128;
@@ -1074,7 +1119,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
               break;
             }
             fence_after_sync();
-            for (int ks = 0; ks < I.nks; ++ks, ++q) {
+            for (int ks = 0, nks = I.steps(u); ks < nks; ++ks, ++q) {
               const int s = q & 1;
               if (!mbar_wait(&sm.bar.full[s], (q >> 1) & 1, kSpin)) {
                 set_status(status, 15);
@@ -1115,7 +1160,8 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
       uint32_t un = 0;
       for (int64_t it = my0; it < my1 && ok; ++it) {
         const int4 itm = tcs_fetch<OP>(g, it);
-        int K, nunits = 1;
+        const TcsItem I = tcs_item<OP, WIDE>(g, itm);
+        int K;
         uint32_t nrows, before = 1;  // at most 2^31 rows
         int64_t stride;
         const float4* X;  // the item's tensor (accumulations: the term's)
@@ -1123,7 +1169,6 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
         if (OP == TCS_ACC) {
           const AccTask& T = g.acc[itm.x];
           K = T.d;
-          nunits = T.count;
           nrows = (uint32_t)T.rows;
           stride = T.rows;
           terms = g.terms + T.first;
@@ -1138,9 +1183,11 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
         }
         const bool along = OP == TCS_MP && before == 1;  // a row's k are contiguous
         const uint32_t row0 = (uint32_t)itm.y * kRows;
-        for (int u = 0; u < nunits; ++u, ++un) {
+        for (int u = 0; u < I.nunits; ++u, ++un) {
           const int buf = (int)(un & 1);
-          const float4* next = OP == TCS_ACC && u + 1 < nunits ? reinterpret_cast<const float4*>(terms[u + 1].X) : X;
+          const int k0 = I.step0(u) * kChunkK, k1 = WIDE ? min(K, k0 + I.steps(u) * kChunkK) : K;
+          const float4* next =
+              OP == TCS_ACC && u + 1 < I.nunits ? reinterpret_cast<const float4*>(terms[I.term(u + 1)].X) : X;
           // producers and epilogue of the unit two back have read this buffer
           if (!waited(&sm.bar.exfree[buf], ((un >> 1) & 1) ^ 1, 19)) break;
           int* ex = sm.ex[buf][xw];
@@ -1149,7 +1196,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
             for (int r0 = xw; r0 < kRows; r0 += 4 * kTcsExWarps) {
               int m[4] = {0, 0, 0, 0};
 #pragma unroll 2
-              for (int k = lane; k < K; k += 32)
+              for (int k = k0 + lane; k < k1; k += 32)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                   const uint32_t rg = row0 + r0 + kTcsExWarps * i;
@@ -1164,7 +1211,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
             }
           } else {
             // a third of the k of every row, the lanes along the rows
-            const int ka = xw * K / kTcsExWarps, kb = (xw + 1) * K / kTcsExWarps;
+            const int ka = k0 + xw * (k1 - k0) / kTcsExWarps, kb = k0 + (xw + 1) * (k1 - k0) / kTcsExWarps;
             const float4* p[4];
             int m[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -1202,7 +1249,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
     uint32_t un = 0;
     for (int64_t it = my0; it < my1 && ok; ++it) {
       const int4 itm = tcs_fetch<OP>(g, it);
-      const TcsItem I = tcs_item<OP>(g, itm);
+      const TcsItem I = tcs_item<OP, WIDE>(g, itm);
       const int np = I.np, NL = I.nl;
       const int c0 = half * (np >> 1), w = np >> 1;  // this warp's columns
       // output row r: element n at base[n * stride]
@@ -1239,14 +1286,14 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
         const bool store = u == 0 && !add_first;
         int er;
         if (OP == TCS_HP) {
-          er = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + u) * kRows + r);
+          er = __ldg(g.groups[itm.x].ex + (size_t)(itm.z + I.term(u)) * kRows + r);
         } else {
           if (!waited(&sm.bar.exready[buf], (un >> 1) & 1, 20)) break;
           er = row_exponent(tcs_row_max(sm.ex[buf], r, along_k));
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.bar.exfree[buf]);
         }
-        const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, u, I) +
+        const int* fxg = reinterpret_cast<const int*>(tcs_image<OP>(g, itm, I.term(u), I) +
                                                       (size_t)I.isteps * kDig * 3 * np * 32);
         const int f0 = __ldg(fxg + lane), f1 = __ldg(fxg + 32 + lane);
         __syncwarp();
@@ -1285,7 +1332,7 @@ __global__ void __launch_bounds__(kTcsThreads, 1) k_tcs(TcsArgs g) {
           }
           __syncwarp();
           float v[2][4], l[2][4];  // recombined levels: re and im of the four columns
-          tcs_levels(lane_addr + (uint32_t)(c0 + n0), np, NL, v, l);
+          tcs_levels(lane_addr + (uint32_t)(c0 + n0), np, NL, I.wide, v, l);
           if (along) {
             float4 o[4];
 #pragma unroll
@@ -1382,17 +1429,20 @@ cudaError_t launch_tf(const MPTask* tasks, const int2* tiles, int64_t first_tile
   return cudaGetLastError();
 }
 
+// wide: some item has more than kTcCols columns
 template <int OP>
-cudaError_t launch_tcs(const TcsArgs& g, const int2* img_units, int64_t first_unit, int64_t n_units, cudaStream_t s) {
+cudaError_t launch_tcs(const TcsArgs& g, const int2* img_units, int64_t first_unit, int64_t n_units, bool wide,
+                       cudaStream_t s) {
   if (n_units > 0) k_tcs_img<OP><<<(unsigned)n_units, kTcsImgThreads, 0, s>>>(g, img_units, first_unit);
   if (OP == TCS_HP) k_hp_ex<<<dim3((unsigned)g.n_items, kRows / 32), 256, 0, s>>>(g);
   unsigned grid = 0;
   cudaError_t e = tc_grid(g.n_items, &grid);
   if (e != cudaSuccess) return e;
   const int smem = (int)sizeof(TcsSmem);
-  e = cudaFuncSetAttribute(k_tcs<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const auto kernel = wide ? k_tcs<OP, true> : k_tcs<OP, false>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k_tcs<OP><<<grid, kTcsThreads, smem, s>>>(g);
+  kernel<<<grid, kTcsThreads, smem, s>>>(g);
   return cudaGetLastError();
 }
 
@@ -1400,7 +1450,7 @@ cudaError_t launch_tcs(const TcsArgs& g, const int2* img_units, int64_t first_un
 
 cudaError_t launch_hp_tc(const HPTask* tasks, const HpTcGroup* groups, const int4* items, int64_t first_item,
                          int64_t n_items, const int2* img_units, int64_t first_unit, int64_t n_units,
-                         double2* ws, int* status, cudaStream_t s) {
+                         double2* ws, bool wide, int* status, cudaStream_t s) {
   if (n_items <= 0) return cudaSuccess;
   TcsArgs g{};
   g.hp = tasks;
@@ -1410,11 +1460,11 @@ cudaError_t launch_hp_tc(const HPTask* tasks, const HpTcGroup* groups, const int
   g.item0 = first_item;
   g.n_items = n_items;
   g.status = status;
-  return launch_tcs<TCS_HP>(g, img_units, first_unit, n_units, s);
+  return launch_tcs<TCS_HP>(g, img_units, first_unit, n_units, wide, s);
 }
 
 cudaError_t launch_mp_tcs(const MPTask* tasks, const int2* tiles, int64_t first_tile, int64_t n_tiles,
-                          const int* tc_tasks, int64_t first_task, int64_t n_tasks, int* status, cudaStream_t s) {
+                          const int* tc_tasks, int64_t first_task, int64_t n_tasks, bool wide, int* status, cudaStream_t s) {
   if (n_tiles <= 0) return cudaSuccess;
   TcsArgs g{};
   g.mp = tasks;
@@ -1423,12 +1473,12 @@ cudaError_t launch_mp_tcs(const MPTask* tasks, const int2* tiles, int64_t first_
   g.item0 = first_tile;
   g.n_items = n_tiles;
   g.status = status;
-  return launch_tcs<TCS_MP>(g, nullptr, first_task, n_tasks, s);
+  return launch_tcs<TCS_MP>(g, nullptr, first_task, n_tasks, wide, s);
 }
 
 cudaError_t launch_acc_tc(const AccTask* tasks, const AccTerm* terms, const int4* items, int64_t first_item,
                           int64_t n_items, int64_t units, const int2* img_units, int64_t first_unit,
-                          int64_t n_units, int* status, cudaStream_t s) {
+                          int64_t n_units, bool wide, int* status, cudaStream_t s) {
   if (n_items <= 0) return cudaSuccess;
   TcsArgs g{};
   g.acc = tasks;
@@ -1438,13 +1488,13 @@ cudaError_t launch_acc_tc(const AccTask* tasks, const AccTerm* terms, const int4
   g.n_items = n_items;
   g.units = units;
   g.status = status;
-  return launch_tcs<TCS_ACC>(g, img_units, first_unit, n_units, s);
+  return launch_tcs<TCS_ACC>(g, img_units, first_unit, n_units, wide, s);
 }
 
 cudaError_t launch_mp_tc(bool oz, const MPTask* tasks, const int2* tiles, int64_t first_tile, int64_t n_tiles,
-                         const int* tc_tasks, int64_t first_task, int64_t n_tasks, int* status, cudaStream_t s) {
+                         const int* tc_tasks, int64_t first_task, int64_t n_tasks, bool wide, int* status, cudaStream_t s) {
   if (n_tiles <= 0) return cudaSuccess;
-  if (oz) return launch_mp_tcs(tasks, tiles, first_tile, n_tiles, tc_tasks, first_task, n_tasks, status, s);
+  if (oz) return launch_mp_tcs(tasks, tiles, first_tile, n_tiles, tc_tasks, first_task, n_tasks, wide, status, s);
   if (n_tasks > 0) k_mp_tf_h<<<(unsigned)n_tasks, 256, 0, s>>>(tasks, tc_tasks, first_task);
   return launch_tf(tasks, tiles, first_tile, n_tiles, status, s);
 }
