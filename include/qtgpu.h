@@ -83,8 +83,10 @@ extern "C" {
  * products and last-index accumulations of shapes from 32 to 112 on the
  * fifth-generation tensor cores (tcgen05.mma, accumulators in tensor memory;
  * beyond 64 output columns in column blocks of at most 48, mode products from
- * 128 rows on, accumulations only in the compressed plan's sweep).  Every operand row is scaled by a
- * power of two and cut into seven signed digits of at most eight bits by
+ * 128 rows on, accumulations only in the compressed plan's sweep; their operand
+ * images and partial tiles take up to an eighth of the scratch budget, and
+ * qt_prepare plans without them where the device has no memory for them).
+ * Every operand row is scaled by a power of two and cut into seven signed digits of at most eight bits by
  * error-free splits, digit products are exact in bf16, each level of digit
  * pairs sums exactly in fp32 as far as tensor memory holds separate level
  * accumulators (all seven for column blocks padded to <= 32, six for 40, five

@@ -435,38 +435,47 @@ int qt_prepare(qt_ctx* c, int flavour) {
     long v = std::atol(s);
     if (v > 0) budget = (int64_t)v * (1 << 20) / 16;
   }
-  std::string msg = qt::build_plan(c->plan, c->nodes, c->ops, c->sop,
-                                   flavour | (scf ? 0x2000 : 0) | (tensor_mp ? 0x8000 : 0), prec, budget, grad,
-                                   cdvr ? &c->cdvr : nullptr, c->tune);
-  if (!msg.empty()) return fail(c, QT_ERR_SHAPE, "qt_prepare: " + msg);
   Plan& P = c->plan;
-  c->buf_elems[qt::B_PSI] = P.psi_arena;
-  c->buf_elems[qt::B_HPHI] = P.psi_arena;
-  c->buf_elems[qt::B_DPSI] = P.psi_arena;
-  c->buf_elems[qt::B_MATS] = P.mats_size;
-  c->buf_elems[qt::B_OPS] = (int64_t)c->ops.data.size() / 2;
-  c->buf_elems[qt::B_SCR] = std::max<int64_t>(P.scratch_size, 16);
-  c->buf_elems[qt::B_PARAM] = 16;
-  c->buf_elems[qt::B_PSI64] = prec >= 1 ? P.psi_arena : 0;
-  c->buf_elems[qt::B_DPSI64] = prec >= 1 ? P.psi_arena : 0;
-  c->buf_elems[qt::B_GRAD] = grad ? P.psi_arena : 0;
-  c->buf_elems[qt::B_GRAD64] = (grad && prec >= 1) ? P.psi_arena : 0;
-  c->buf_elems[qt::B_KEEP] = P.keep_size;
-  c->buf_elems[qt::B_HPW] = P.hpw_size;
-  c->buf_elems[qt::B_KRY] = P.kry_size;
-  c->buf_elems[qt::B_CDVR] = P.cdvr ? P.cdvr_size : 0;
-  c->buf_elems[qt::B_OZ] = (P.oz_bytes + 15) / 16;
+  qt::TcTune tune = c->tune;
   int64_t arena = 0;
-  for (int i = 0; i < qt::B_NBUF; ++i) {
-    if ((i == qt::B_PSI64 || i == qt::B_DPSI64 || i == qt::B_GRAD64) && prec == 0) continue;  // aliases
-    if ((i == qt::B_GRAD || i == qt::B_GRAD64) && !grad) continue;
-    int64_t n = std::max<int64_t>(c->buf_elems[i], 16);
-    cudaError_t e = dev_malloc((void**)&c->buf[i], n * sizeof(double2));
-    if (e != cudaSuccess) {
-      release_arena(c);
-      return fail(c, QT_ERR_ALLOC, std::string("qt_prepare: device allocation failed: ") + cudaGetErrorString(e));
+  for (;;) {
+    std::string msg = qt::build_plan(P, c->nodes, c->ops, c->sop,
+                                     flavour | (scf ? 0x2000 : 0) | (tensor_mp ? 0x8000 : 0), prec, budget, grad,
+                                     cdvr ? &c->cdvr : nullptr, tune);
+    if (!msg.empty()) return fail(c, QT_ERR_SHAPE, "qt_prepare: " + msg);
+    c->buf_elems[qt::B_PSI] = P.psi_arena;
+    c->buf_elems[qt::B_HPHI] = P.psi_arena;
+    c->buf_elems[qt::B_DPSI] = P.psi_arena;
+    c->buf_elems[qt::B_MATS] = P.mats_size;
+    c->buf_elems[qt::B_OPS] = (int64_t)c->ops.data.size() / 2;
+    c->buf_elems[qt::B_SCR] = std::max<int64_t>(P.scratch_size, 16);
+    c->buf_elems[qt::B_PARAM] = 16;
+    c->buf_elems[qt::B_PSI64] = prec >= 1 ? P.psi_arena : 0;
+    c->buf_elems[qt::B_DPSI64] = prec >= 1 ? P.psi_arena : 0;
+    c->buf_elems[qt::B_GRAD] = grad ? P.psi_arena : 0;
+    c->buf_elems[qt::B_GRAD64] = (grad && prec >= 1) ? P.psi_arena : 0;
+    c->buf_elems[qt::B_KEEP] = P.keep_size;
+    c->buf_elems[qt::B_HPW] = P.hpw_size;
+    c->buf_elems[qt::B_KRY] = P.kry_size;
+    c->buf_elems[qt::B_CDVR] = P.cdvr ? P.cdvr_size : 0;
+    c->buf_elems[qt::B_OZ] = (P.oz_bytes + 15) / 16;
+    cudaError_t e = cudaSuccess;
+    arena = 0;
+    for (int i = 0; i < qt::B_NBUF && e == cudaSuccess; ++i) {
+      if ((i == qt::B_PSI64 || i == qt::B_DPSI64 || i == qt::B_GRAD64) && prec == 0) continue;  // aliases
+      if ((i == qt::B_GRAD || i == qt::B_GRAD64) && !grad) continue;
+      int64_t n = std::max<int64_t>(c->buf_elems[i], 16);
+      e = dev_malloc((void**)&c->buf[i], n * sizeof(double2));
+      arena += n * 16;
     }
-    arena += n * 16;
+    if (e == cudaSuccess) break;
+    release_arena(c);
+    cudaGetLastError();  // the allocation's error is reported here, not by the next launch
+    // once more without the wide shapes' images and partial tiles
+    const bool again = tune.wide && std::any_of(P.stages.begin(), P.stages.end(), [](const qt::Stage& st) { return st.tc_wide; });
+    if (!again)
+      return fail(c, QT_ERR_ALLOC, std::string("qt_prepare: device allocation failed: ") + cudaGetErrorString(e));
+    tune.wide = false;
   }
   if (prec == 0) {
     c->buf[qt::B_PSI64] = c->buf[qt::B_PSI];

@@ -81,7 +81,13 @@ constexpr int kTcCols = 64;     // output columns of one accumulator tile
 constexpr int kTcMaxDim = 112;  // seven 16-k steps; the planner's largest bond
 struct TcTune {
   int mp = 32, hp = 32, acc = 32;
+  bool wide = true;  // shapes beyond kTcCols too (qt_prepare plans without them when device memory runs out)
 };
+// Operand images and partial tiles of wide shapes cost memory that the FP32
+// pipe does not need (64 modes, bonds 112, 256 couplings: 4.1 + 2.5 GB): a stage
+// whose wide tasks need more than this part of the scratch budget is cut into
+// several (that plan: 79 stages -> 153, 0.85 GB; bonds 48..96: 79 -> 82).
+constexpr int kTcWideShare = 8;
 // hole product: lo <= a and at least two 64-k chunks of reduction
 inline bool hp_tc_eligible(int before, int a, int after, int lo = 32) {
   return a >= lo && lo <= kTcCols && a <= kTcMaxDim && (int64_t)before * after >= 2 * kHpTcChunk;

@@ -90,6 +90,7 @@ class Builder {
   void set_cdvr(const CdvrDesc* d) { cdvr = d; }
 
   void run() {
+    wide = P.tune.wide;
     geometry();
     activity();
     layout();
@@ -102,7 +103,7 @@ class Builder {
     stage_inverse();
     if (scf && !compressed) throw std::runtime_error("the SCF sweep needs the compressed plan");
     if (compressed) {
-      wide_acc = true;
+      wide_acc = wide;
       comp_layout();
       comp_represent();
       comp_meanfield();
@@ -487,8 +488,8 @@ class Builder {
     std::vector<char> tc(t1 - t0, 0);
     if (P.hp_tensor)
       for (int64_t t = t0; t < t1; ++t)
-        tc[t - t0] = hp_tc_eligible(P.hp[t].before, P.hp[t].a, P.hp[t].after, P.tune.hp) &&
-                     (wide || P.hp[t].a <= kTcCols);
+        tc[t - t0] = P.hp[t].a > kTcCols ? wide_hp(P.hp[t])
+                                        : hp_tc_eligible(P.hp[t].before, P.hp[t].a, P.hp[t].after, P.tune.hp);
     double work = 0;
     for (int64_t t = t0; t < t1; ++t)
       if (!tc[t - t0]) work += (double)ntiles(P.hp[t]) * P.hp[t].before * P.hp[t].after;
@@ -548,7 +549,7 @@ class Builder {
     for (int64_t t = t0; t < t1; ++t) {
       if (!tc[t - t0]) continue;
       const Plan::SHP& h = P.hp[t];
-      // one group per column block (a > 64: two, with one member each)
+      // one group per column block (a > 64: two or three, with one member each)
       for (int cb = 0; cb < tc_blocks(h.a); ++cb) {
         const auto key = std::make_tuple(h.A.buf, h.A.off, h.before, h.a, h.after, cb);
         auto it = open.find(key);
@@ -620,7 +621,7 @@ class Builder {
     units = 0;
     for (int64_t t = t0; t < t1; ++t) {
       Plan::SAcc& a = P.acc[t];
-      if (a.count < 1 || !acc_tc_eligible(a.rows, a.d, P.tune.acc) || (a.d > kTcCols && !wide_acc)) continue;
+      if (a.d > kTcCols ? !wide_accum(a) : a.count < 1 || !acc_tc_eligible(a.rows, a.d, P.tune.acc)) continue;
       tc[t - t0] = 1;
       stage_wide_ |= a.d > kTcCols;
       a.tc_img = stage_oz_;
@@ -642,9 +643,71 @@ class Builder {
     return w;
   }
 
+  // whether a task of more than kTcCols columns takes the tensor cores
+  bool wide_mp(const Plan::SMP& m) const {
+    return wide && P.hp_tensor && !m.diag && mp_tc_wide(m.a_in, m.a_out, (int64_t)m.before * m.after, P.tune.mp);
+  }
+  bool wide_hp(const Plan::SHP& h) const {
+    return wide && P.hp_tensor && h.a > kTcCols && hp_tc_eligible(h.before, h.a, h.after, P.tune.hp);
+  }
+  bool wide_accum(const Plan::SAcc& a) const {
+    return wide_acc && P.hp_tensor && a.count > 0 && a.d > kTcCols && acc_tc_eligible(a.rows, a.d, P.tune.acc);
+  }
+
+  // First task of [t0, t1) at which the operand images and partial tiles of the
+  // wide tensor-core tasks before it exceed their share of the scratch budget
+  // (at least t0 + 1; t1: all fit)
+  int64_t memory_cut(int kind, int64_t t0, int64_t t1) const {
+    if (kind != ST_MP && kind != ST_HP && kind != ST_ACC) return t1;
+    const int64_t limit = budget * 16 / kTcWideShare;
+    std::set<std::tuple<int, int64_t, int, int, int>> images;  // hole products share A's
+    int64_t used = 0;
+    for (int64_t t = t0; t < t1; ++t) {
+      if (kind == ST_MP && wide_mp(P.mp[t])) {
+        const auto& m = P.mp[t];
+        used += tc_blocks(m.a_out) * hp_tc_chunk_bytes(tc_width(m.a_out), tc_steps(m.a_in));
+      } else if (kind == ST_ACC && wide_accum(P.acc[t])) {
+        const auto& a = P.acc[t];
+        used += (int64_t)a.count * tc_blocks(a.d) * hp_tc_chunk_bytes(tc_width(a.d), tc_steps(a.d));
+      } else if (kind == ST_HP && wide_hp(P.hp[t])) {
+        const auto& h = P.hp[t];
+        const int kc = hp_tc_kc(tc_width(h.a));
+        const int64_t chunks = ((int64_t)h.before * h.after + kc - 1) / kc;
+        used += chunks * (16 * (int64_t)h.a * h.a + 128 * tc_blocks(h.a));
+        if (images.insert(std::make_tuple(h.A.buf, h.A.off, h.before, h.a, h.after)).second)
+          used += tc_blocks(h.a) * chunks * hp_tc_chunk_bytes(tc_width(h.a), kc / 16);
+      }
+      if (used > limit && t > t0) return t;
+    }
+    return t1;
+  }
+
+  // one stage, or several where memory_cut says so (its tasks are independent)
   void emit_stage(int kind, int64_t t0, int64_t t1, int64_t tile0, int64_t tile1,
                   const char* name) {
     if (t1 <= t0) return;
+    const double flops = P.stats.exec_flops - stage_flops_mark, bytes = stage_bytes(kind, t0, t1);
+    stage_flops_mark = P.stats.exec_flops;
+    while (t0 < t1) {
+      const int64_t cut = memory_cut(kind, t0, t1);
+      int64_t mid = tile1;
+      if (cut < t1 && kind != ST_HP) {  // (hole products get their tiles in hp_split)
+        auto first_of = [&](const auto& tiles) {
+          return std::lower_bound(tiles.begin() + tile0, tiles.begin() + tile1, cut,
+                                  [](const auto& tile, int64_t t) { return tile.x < t; }) -
+                 tiles.begin();
+        };
+        mid = kind == ST_MP ? first_of(P.mp_tiles) : first_of(P.acc_tiles);
+      }
+      const double part = stage_bytes(kind, t0, cut);
+      emit_one(kind, t0, cut, tile0, mid, name, part == bytes ? flops : flops * (part / bytes), part);
+      t0 = cut;
+      tile0 = kind == ST_HP ? (int64_t)P.hp_tiles.size() : mid;
+    }
+  }
+
+  void emit_one(int kind, int64_t t0, int64_t t1, int64_t tile0, int64_t tile1, const char* name,
+                double flops, double bytes) {
     bool split = false;
     const int64_t seg0 = (int64_t)P.hp_segs.size();
     const int64_t hti0 = (int64_t)P.hp_tc_items.size(), htu0 = (int64_t)P.hp_tc_imgs.size();
@@ -670,11 +733,9 @@ class Builder {
       longest_first(P.acc_tiles, [&](int t) { return (int64_t)P.acc[t].count * P.acc[t].d; });
     else if (kind == ST_MP)
       longest_first(P.mp_tiles, [&](int t) { return P.mp[t].diag ? 1 : P.mp[t].a_in; });
-    const double f1 = P.stats.exec_flops;
     Stage s;
-    s.flops = f1 - stage_flops_mark;
-    s.bytes = stage_bytes(kind, t0, t1);
-    stage_flops_mark = f1;
+    s.flops = flops;
+    s.bytes = bytes;
     s.kind = kind;
     s.first_task = t0;
     s.n_tasks = t1 - t0;
@@ -709,7 +770,7 @@ class Builder {
     for (int64_t t = t0; t < t1; ++t) {
       auto& m = P.mp[t];
       const int64_t rows = (int64_t)m.before * m.after;
-      const bool beyond = wide && P.hp_tensor && mp_tc_wide(m.a_in, m.a_out, rows, P.tune.mp);
+      const bool beyond = wide_mp(m);
       if (m.diag || !(beyond || mp_tc_eligible(m.a_in, m.a_out, P.tune.mp))) continue;
       oz[t - t0] = 1;
       stage_wide_ |= beyond;
