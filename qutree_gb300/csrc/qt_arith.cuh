@@ -195,15 +195,23 @@ struct DF64 {
   }
   typedef float2 R;
   static __device__ __forceinline__ bool positive(const S& x) { return x.x > 0.f; }
-  // 1 / (hi + lo) on the FP32 pipe: r0 = fl(1 / hi), e = 1 - (hi + lo) r0
-  // (about 2^-24, its own rounding 2^-48), r = r0 + r0 (e + e^2)
+  // 1 / (hi + lo) on the FP32 pipe, to the rounding of a split binary64
+  // quotient (2^-49): r0 = fl(1 / hi); 1 - hi r0 is a binary32 number, so that
+  // e = 1 - (hi + lo) r0 is known to two words (eh, el); r = r0 + r0 (e + e^2)
+  // with the products' and sums' low parts kept
   static __device__ __forceinline__ R rrecip(const S& x) {
     const float r0 = __frcp_rn(x.x);
-    float e = __fmaf_rn(-x.x, r0, 1.f);
-    e = __fmaf_rn(-x.y, r0, e);
-    const float c = __fmul_rn(r0, __fmaf_rn(e, e, e));
+    const float p = __fmul_rn(-x.y, r0), pl = __fmaf_rn(-x.y, r0, -p);
+    float eh, el;
+    df_two_sum(__fmaf_rn(-x.x, r0, 1.f), p, eh, el);
+    el = __fadd_rn(el, pl);
+    const float c = __fmul_rn(r0, eh), cl = __fmaf_rn(r0, eh, -c);
+    const float tail = __fmaf_rn(r0, __fmaf_rn(eh, eh, el), cl);
     R r;
-    df_quick_two_sum(r0, c, r.x, r.y);
+    float ch, ct, s, l;
+    df_quick_two_sum(c, tail, ch, ct);
+    df_quick_two_sum(r0, ch, s, l);
+    df_quick_two_sum(s, __fadd_rn(l, ct), r.x, r.y);
     return r;
   }
   static __device__ __forceinline__ S conj_scale(const S& x, R r) {
