@@ -26,7 +26,9 @@ using qt::Ref;
 // What the host reads after every sweep, in page-locked memory: copies there
 // queue behind the sweep, and one wait covers them all (pageable copies wait
 // one by one: derivative and expectation of 8 modes, host to host, 204 us
-// instead of 178)
+// instead of 178).  Allocated by the first qt_prepare, which allocates device
+// memory anyway: page-locked allocations wait for the device and are refused
+// under a global-mode capture, and a context for the primitives alone needs none.
 struct HostWords {
   static constexpr int kTrees = 128;
   int status;
@@ -36,7 +38,7 @@ struct HostWords {
 struct qt_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
-  HostWords* host = nullptr;
+  HostWords* host = nullptr;  // from the first qt_prepare on
   std::string err;
   bool have_tree = false, have_sop = false, prepared = false, have_psi = false, swept = false;
   bool built = false;  // matrices of the current plan computed (qt_build / qt_derivative)
@@ -227,9 +229,7 @@ int qt_ctx_create(qt_ctx** out, int device) {
                     cudaGetErrorString(scope.err));
   }
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&c->host), sizeof(HostWords));
   if (e != cudaSuccess) {
-    if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return fail(nullptr, QT_ERR_CUDA, std::string("qt_ctx_create: ") + cudaGetErrorString(e));
   }
@@ -254,13 +254,13 @@ namespace {
 // queued ahead of the caller's wait for the stream and looked at after it
 // (cleared once reported)
 int queue_status(qt_ctx* c) {
-  c->host->status = 0;
+  if (c->host) c->host->status = 0;
   if (!c->prepared || !c->tables.status) return QT_OK;
   QT_CUDA(c, cudaMemcpyAsync(&c->host->status, c->tables.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   return QT_OK;
 }
 int check_status(qt_ctx* c) {
-  const int st = c->host->status;
+  const int st = c->host ? c->host->status : 0;
   if (st == 0) return QT_OK;
   QT_CUDA(c, cudaMemsetAsync(c->tables.status, 0, sizeof(int), c->stream));
   return fail(c, QT_ERR_TIMEOUT, "a tensor-core kernel gave up waiting (code " + std::to_string(st) +
@@ -430,6 +430,7 @@ int qt_prepare(qt_ctx* c, int flavour) {
     return fail(c, QT_ERR_ARG, "unknown plan flavour");
   QT_DEVICE(c);
   release_arena(c);
+  if (!c->host) QT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host), sizeof(HostWords)));
   int64_t budget = (int64_t)1 << 28;  // scratch elements (4 GiB)
   if (const char* s = std::getenv("QT_SCRATCH_MIB")) {
     long v = std::atol(s);
