@@ -32,6 +32,7 @@ using qt::Ref;
 struct HostWords {
   static constexpr int kTrees = 128;
   int status;
+  int lanczos_stop;  // written by k_lanczos: the Lanczos space has ended
   double2 energy[2 * kTrees];
 };
 
@@ -1751,6 +1752,17 @@ struct DevFree {
     if (p) cudaFree(p);
   }
 };
+struct Event {
+  cudaEvent_t e = nullptr;
+  ~Event() {
+    if (e) cudaEventDestroy(e);
+  }
+};
+// Products of H whose launches the host queues before it knows whether the
+// Lanczos space has ended: one where a product takes less than a wait and the
+// launches behind it (about 100 us, at 1 TFLOP/s), none beyond, so that an
+// invariant space costs at most one product that short
+constexpr double kLanczosAheadFlops = 1e8;
 
 }  // namespace
 
@@ -1866,6 +1878,8 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
     c->launches += 1;
     return QT_OK;
   };
+  Event step_done[2];
+  for (Event& ev : step_done) QT_CUDA(c, cudaEventCreateWithFlags(&ev.e, cudaEventDisableTiming));
   int rc;
   if (df && (rc = to_arith(psi_ar, psi, P.psi_packed)) != QT_OK) return rc;
   // initial build: buildSCF(node, parent) for every non-top node, bottom-up
@@ -1880,8 +1894,13 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
       const int64_t N = g.N;
       cd* pa = psi + g.aoff;
       int size = (int)std::min<int64_t>(n_krylov, N);
-      // Lanczos on the effective Hamiltonian (solveKrylovSpace): the whole
-      // recursion is enqueued, its scalars come back with one wait
+      // Lanczos on the effective Hamiltonian (solveKrylovSpace): the host is at
+      // most `ahead` products ahead of the end of the space, the scalars come
+      // back with one copy
+      double product_flops = 0;
+      for (int64_t q = P.scf_apply_b[a]; q < P.scf_apply_e[a]; ++q) product_flops += P.stages[q].flops;
+      const int ahead = product_flops <= kLanczosAheadFlops ? 1 : 0;
+      c->host->lanczos_stop = 0;
       std::vector<double> al, be;
       double* dres = reinterpret_cast<double*>(dscal);
       qt::LanczosStep lz;
@@ -1892,7 +1911,12 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
       lz.kout = kout;
       lz.res = dres;
       lz.breakdown = kLanczosBreakdown;
+      lz.host_stop = &c->host->lanczos_stop;
       for (int l = -1; l < size; ++l) {
+        if (l - 1 - ahead >= 0) {  // the latest step whose outcome must be known
+          QT_CUDA(c, cudaEventSynchronize(step_done[(l - 1 - ahead) & 1].e));
+          if (*static_cast<volatile int*>(&c->host->lanczos_stop)) break;
+        }
         lz.l = l;
         lz.last = l + 1 == size ? 1 : 0;
         lz.v = l < 0 ? pa : V(l);
@@ -1902,6 +1926,7 @@ int qt_scf(qt_ctx* c, int n_iter, int n_krylov, int n_itp, double beta, double* 
         cudaError_t e = qt::launch_lanczos(lz, c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "qt_scf Lanczos step");
         c->launches += 1;
+        if (l >= 0) QT_CUDA(c, cudaEventRecord(step_done[l & 1].e, c->stream));
       }
       double hres[qt::kLzScalars];
       QT_CUDA(c, cudaMemcpyAsync(hres, dres, sizeof(hres), cudaMemcpyDeviceToHost, c->stream));

@@ -752,6 +752,7 @@ struct LanczosStep {
   void* kin;
   const void* kout;
   double* res;
+  int* host_stop;       // page-locked: set when the space has ended
   double breakdown;
 };
 cudaError_t launch_lanczos(const LanczosStep& step, cudaStream_t s);

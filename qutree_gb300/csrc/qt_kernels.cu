@@ -1436,7 +1436,8 @@ __global__ void __launch_bounds__(kThreads) k_convert(void* __restrict__ dst, co
 // tree, then a tree over the slices), slices shared out over the CTAs, the
 // partial sums read through distributed shared memory.  One launch in place
 // of eight with two waits of the host between them; per step 80 us of an
-// 8-mode tree's ~110 went there.
+// 8-mode tree's ~110 went there.  The host learns of the end through
+// host_stop and queues no further products.
 __device__ __forceinline__ double ld_cluster_d(const double* p, uint32_t rank) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
   uint32_t ra;
@@ -1546,7 +1547,10 @@ __global__ void __launch_bounds__(kDotThreads) k_lanczos(LanczosStep t, int cl) 
       const bool stop = nrm <= t.breakdown * scale;
       if (writer) {
         t.res[kLzBeta + t.l] = s == s ? nrm : s;  // fmax drops a NaN
-        if (stop) t.res[kLzStop] = t.l + 1;
+        if (stop) {
+          t.res[kLzStop] = t.l + 1;
+          *t.host_stop = 1;
+        }
       }
       if (!stop) {
         const double c = 1.0 / nrm;
