@@ -988,6 +988,34 @@ __device__ void herm_jacobi(double2* A, double2* U, int d, double2* rot, double2
   }
 }
 
+// Whether the Hermitian matrix with lower triangle U (global memory,
+// overwritten) has a Cholesky factorisation; uniform over the block.
+__device__ bool cholesky_succeeds(double2* U, int d) {
+  for (int k = 0; k < d; ++k) {
+    const double dk = U[k + (int64_t)d * k].x;
+    if (!(dk > 0.0)) return false;
+    const double l = sqrt(dk);
+    __syncthreads();
+    for (int i = k + threadIdx.x; i < d; i += kThreads) {
+      const double2 v = U[i + (int64_t)d * k];
+      U[i + (int64_t)d * k] = make_double2(v.x / l, v.y / l);
+    }
+    __syncthreads();
+    // trailing update of the lower triangle: U(i,j) -= L(i,k) conj(L(j,k))
+    const int rem = d - k - 1;
+    for (int e = threadIdx.x; e < rem * rem; e += kThreads) {
+      const int i = k + 1 + e % rem, j = k + 1 + e / rem;
+      if (j > i) continue;
+      const double2 li = U[i + (int64_t)d * k], lj = U[j + (int64_t)d * k];
+      double2 u = U[i + (int64_t)d * j];
+      cfma(u, make_double2(-li.x, -li.y), make_double2(lj.x, -lj.y));
+      U[i + (int64_t)d * j] = u;
+    }
+    __syncthreads();
+  }
+  return true;
+}
+
 __device__ __forceinline__ void eig_body(const EigTask& t, double eps) {
   extern __shared__ double2 smem[];
   const int d = t.d;
@@ -1010,9 +1038,14 @@ __device__ __forceinline__ void eig_body(const EigTask& t, double eps) {
     __syncthreads();
   };
   load(A);
-  // First path.  The smallest eigenvalue is at least 1 / |rho^-1|_F; if that
-  // exceeds 40 eps, eps*exp(-w/eps) changes 1/w by less than 2e-19 relative and
-  // the regularised inverse is the plain inverse.
+  // If every eigenvalue w exceeds 40 eps, eps*exp(-w/eps) changes 1/w by less
+  // than 2e-19 relative and the regularised inverse is the plain inverse.  Two
+  // certificates, the second only where the first leaves the question open:
+  //  * |rho^-1|_F <= 1 / (40 eps), since w >= 1 / |rho^-1|_F;
+  //  * a Cholesky factorisation of rho - 100 eps I (backward error about
+  //    d 2^-53 |rho|, far below 50 eps for eps = 1e-10 and normalised states).
+  //    With |rho^-1|_F > sqrt(d) / (100 eps) some w is below 100 eps: it would
+  //    fail (rank-deficient densities, which need the eigenvalues anyway).
   __shared__ double2 col_s[2 * kHpMaxDim];
   if (herm_sweep_inverse<F64>(A, d, col_s)) {
     double n2 = 0.0;
@@ -1028,8 +1061,15 @@ __device__ __forceinline__ void eig_body(const EigTask& t, double eps) {
       if (threadIdx.x < s) red_off[threadIdx.x] += red_off[threadIdx.x + s];
       __syncthreads();
     }
-    const double lim = 1.0 / (40.0 * eps);
-    if (red_off[0] <= lim * lim) {
+    const double lim = 1.0 / (40.0 * eps), open = 1.0 / (100.0 * eps);
+    bool plain = red_off[0] <= lim * lim;
+    if (!plain && red_off[0] <= d * (open * open)) {
+      load(U);
+      for (int i = threadIdx.x; i < d; i += kThreads) U[i + (int64_t)d * i].x -= 100.0 * eps;
+      __syncthreads();
+      plain = cholesky_succeeds(U, d);
+    }
+    if (plain) {
       for (int e = threadIdx.x; e < d * d; e += kThreads) {
         const int i = e % d, j = e / d;
         const double2 x = i >= j ? A[e] : A[j + d * i];
@@ -1040,83 +1080,6 @@ __device__ __forceinline__ void eig_body(const EigTask& t, double eps) {
   }
   __syncthreads();
   load(A);
-  for (int e = threadIdx.x; e < d * d; e += kThreads) {
-    // shifted copy for the positive-definiteness certificate below
-    U[e] = (e % d == e / d) ? make_double2(A[e].x - 100.0 * eps, 0.0) : A[e];
-  }
-  __syncthreads();
-  // Second path.  If every eigenvalue exceeds 50*eps, eps*exp(-w/eps) changes
-  // 1/w by less than 4e-24 relative, so the regularised inverse is the plain
-  // inverse.  A Cholesky factorisation of rho - 100*eps*I that succeeds
-  // certifies that bound (its backward error, ~d*2^-53*|rho|, is far below
-  // 50*eps for eps = 1e-10 and normalised states); then rho^-1 comes from a
-  // Gauss-Jordan inversion (no pivoting needed for a positive definite
-  // matrix) in O(d^3) instead of a Jacobi eigensolver.
-  __shared__ int not_pd;
-  __shared__ double2 piv_s;
-  if (threadIdx.x == 0) not_pd = 0;
-  __syncthreads();
-  for (int k = 0; k < d; ++k) {
-    const double dk = U[k + (int64_t)d * k].x;
-    if (!(dk > 0.0)) {
-      if (threadIdx.x == 0) not_pd = 1;
-      break;  // uniform: every thread reads the same value
-    }
-    const double l = sqrt(dk);
-    __syncthreads();
-    for (int i = k + threadIdx.x; i < d; i += kThreads) {
-      double2 v = U[i + (int64_t)d * k];
-      U[i + (int64_t)d * k] = make_double2(v.x / l, v.y / l);
-    }
-    __syncthreads();
-    // trailing update of the lower triangle: U(i,j) -= L(i,k) conj(L(j,k))
-    const int rem = d - k - 1;
-    for (int e = threadIdx.x; e < rem * rem; e += kThreads) {
-      const int i = k + 1 + e % rem, j = k + 1 + e / rem;
-      if (j > i) continue;
-      const double2 li = U[i + (int64_t)d * k], lj = U[j + (int64_t)d * k];
-      double2 u = U[i + (int64_t)d * j];
-      cfma(u, make_double2(-li.x, -li.y), make_double2(lj.x, -lj.y));
-      U[i + (int64_t)d * j] = u;
-    }
-    __syncthreads();
-  }
-  __syncthreads();
-  if (!not_pd) {
-    double2* X = t.rhoinv;
-    for (int e = threadIdx.x; e < d * d; e += kThreads)
-      X[e] = make_double2((e % d) == (e / d) ? 1.0 : 0.0, 0.0);
-    __syncthreads();
-    for (int col = 0; col < d; ++col) {
-      if (threadIdx.x == 0) {
-        const double2 v = A[col + d * col];
-        const double den = v.x * v.x + v.y * v.y;
-        piv_s = make_double2(v.x / den, -v.y / den);
-      }
-      __syncthreads();
-      const double2 pinv = piv_s;
-      for (int j = threadIdx.x; j < d; j += kThreads) {
-        A[col + d * j] = cmul(A[col + d * j], pinv);
-        X[col + (int64_t)d * j] = cmul(X[col + (int64_t)d * j], pinv);
-      }
-      __syncthreads();
-      // column col of A before elimination (fw reused as the factor column)
-      for (int r = threadIdx.x; r < d; r += kThreads) fw[r] = A[r + d * col];
-      __syncthreads();
-      for (int e = threadIdx.x; e < d * d; e += kThreads) {
-        const int r = e % d, j = e / d;
-        if (r == col) continue;
-        const double2 f = fw[r];
-        double2 a = A[e], x = X[e];
-        cfma(a, make_double2(-f.x, -f.y), A[col + d * j]);
-        cfma(x, make_double2(-f.x, -f.y), X[col + (int64_t)d * j]);
-        A[e] = a;
-        X[e] = x;
-      }
-      __syncthreads();
-    }
-    return;
-  }
   herm_jacobi(A, U, d, rot, ph, pq, red_off, red_diag);
   for (int i = threadIdx.x; i < d; i += kThreads) {
     const double w = A[i + d * i].x;

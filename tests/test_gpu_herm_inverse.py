@@ -83,3 +83,30 @@ def test_projector_of_non_orthonormal_nodes(bond, prec, tol):
             a, b = a @ r.T, b @ r.T
         num, den = max(num, np.abs(a - b).max()), max(den, np.abs(b).max())
     assert num <= 10 * tol * den
+
+
+@pytest.mark.parametrize("d", [17, 64, 112])
+@pytest.mark.parametrize("low,rest", [(110.0, 250.0), (60.0, 90.0), (90.0, 260.0)])
+def test_density_inverse_between_the_certificates(d, low, rest):
+    """All eigenvalues within a few hundred eps: the Frobenius norm of the
+    inverse alone does not decide.  The spectrum lies above 100 eps (the
+    factorisation certifies it), below (no factorisation is tried at d = 112),
+    or has one eigenvalue below (it is tried and fails)."""
+    eps = 1e-8
+    rng = np.random.default_rng(d)
+    w = eps * rng.uniform(0.5 * (low + rest), rest, d)
+    w[0] = eps * low
+    m = hermitian(rng, w)
+    lam, u = np.linalg.eigh(m)
+    want = (u / (lam + eps * np.exp(-lam / eps))) @ u.conj().T
+    ctx = qtgpu.Context(0)
+    try:
+        a, b = ctx.to_device(m.ravel(order="F")), ctx.to_device(np.zeros(d * d, complex))
+        ctx.rho_inverse_noalloc(b, a, 1, d, eps)
+        got = ctx.from_device(b, (d * d,)).reshape((d, d), order="F")
+        ctx.free(a)
+        ctx.free(b)
+    finally:
+        ctx.close()
+    cond = lam[-1] / lam[0]
+    assert rel_err(got, want) <= 8 * d * cond * 2.0 ** -53 + 64 * 2.0 ** -53 * cond
