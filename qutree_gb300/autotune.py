@@ -1,21 +1,25 @@
 """Autotuner of the tensor-core bounds (qt_set_tc_thresholds).
 
 For every contraction kind (mode products, hole products, last-index
-accumulations) and every size a in 16..64 (steps of 8) it times, on the
+accumulations) and every size a in 16..64 (steps of 8), 72 and 96 it times, on the
 device, the double-float compressed sweep of a probe problem whose
 contractions all have size a -- a balanced tree of 64 modes with a-point
 leaves and bonds a, a coupled-oscillator SOP with 256 random couplings --
 once with that kind on the tensor cores (bound a) and once on the FP32
 pipe (bound 65), the other two kinds on the FP32 pipe in both.  A kind's bound is the smallest size from
-which the tensor cores win at every larger size (by at least 3%); 65 when
-they never do.  The bounds are cached per device (name and SM count) as
-JSON; HamiltonianRepresentation(..., tc_thresholds="auto") reads them.
+which the tensor cores win at every larger size (by at least 3%), 64 when
+that is beyond 64 (65 would keep the shapes beyond 64 off the tensor cores
+too), and 65 when they lose at the largest.  The bounds are cached per device
+(name and SM count) as JSON, with a digest of the library's sources: bounds
+measured with other kernels are not read.
+HamiltonianRepresentation(..., tc_thresholds="auto") reads them.
 
     python -m qutree_gb300.autotune [--device 0] [--sizes 16,24,...]
 """
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
 import time
@@ -26,7 +30,7 @@ from . import qtgpu
 from .model import balanced_tree, coupled_oscillators, random_wavefunction
 
 KINDS = ("mp", "hp", "acc")
-SIZES = (16, 24, 32, 40, 48, 56, 64)
+SIZES = (16, 24, 32, 40, 48, 56, 64, 72, 96)
 DEFAULT = {"mp": 32, "hp": 32, "acc": 32}
 
 
@@ -36,19 +40,42 @@ def _device_key(device: int) -> str:
     return f"{p.name.replace(' ', '_')}-sm{p.multi_processor_count}"
 
 
+def _kernels() -> str:
+    """Digest of the sources the kernels and the planner are built from."""
+    csrc = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
+    digest = hashlib.sha256()
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name), "rb") as f:
+            digest.update(name.encode() + b"\0" + f.read())
+    return digest.hexdigest()[:16]
+
+
 def cache_path(device: int = 0) -> str:
     root = os.environ.get("QT_AUTOTUNE_DIR", os.path.join(os.path.expanduser("~"), ".cache", "qtgpu"))
     return os.path.join(root, f"tc_bounds-{_device_key(device)}.json")
 
 
 def cached(device: int = 0):
-    """(mp, hp, acc) bounds cached for this device, or the built-in ones."""
+    """(mp, hp, acc) bounds cached for this device by these kernels, or the
+    built-in ones."""
     try:
         with open(cache_path(device)) as f:
-            b = json.load(f)["bounds"]
-        return tuple(int(b[k]) for k in KINDS)
-    except (OSError, KeyError, ValueError):
-        return tuple(DEFAULT[k] for k in KINDS)
+            rec = json.load(f)
+        if rec["kernels"] == _kernels():
+            return tuple(int(rec["bounds"][k]) for k in KINDS)
+    except (OSError, KeyError, ValueError, TypeError):
+        pass
+    return tuple(DEFAULT[k] for k in KINDS)
+
+
+def choose(timings: dict, margin: float = 0.03) -> int:
+    """The bound of one kind from {size: {"tensor_cores_ms", "fp32_pipe_ms"}}."""
+    bound = 65
+    for a in sorted(timings, reverse=True):  # the smallest size from which the tensor cores always win
+        if timings[a]["tensor_cores_ms"] > (1.0 - margin) * timings[a]["fp32_pipe_ms"]:
+            break
+        bound = min(a, 64)
+    return bound
 
 
 def probe_problem(a: int, modes: int = 64, seed: int = 5):
@@ -88,20 +115,11 @@ def tune(device: int = 0, sizes=SIZES, write: bool = True, margin: float = 0.03)
         off = _time_sweeps(tree, sop, psi, (65, 65, 65), device)
         for i, k in enumerate(KINDS):
             bounds = [65, 65, 65]
-            bounds[i] = a
+            bounds[i] = min(a, 64)
             on = _time_sweeps(tree, sop, psi, tuple(bounds), device)
             timings[k][a] = {"tensor_cores_ms": on, "fp32_pipe_ms": off}
-    chosen = {}
-    for k in KINDS:
-        bound = 65
-        for a in sorted(sizes, reverse=True):  # the smallest size from which the tensor cores always win
-            t = timings[k][a]
-            if t["tensor_cores_ms"] <= (1.0 - margin) * t["fp32_pipe_ms"]:
-                bound = a
-            else:
-                break
-        chosen[k] = bound
-    rec = {"device": _device_key(device), "bounds": chosen,
+    chosen = {k: choose(timings[k], margin) for k in KINDS}
+    rec = {"device": _device_key(device), "kernels": _kernels(), "bounds": chosen,
            "probe": "balanced tree of 64 modes, leaves and bonds a, coupled oscillators; compressed "
                     "double-float sweep, one kind on the tensor cores against none",
            "timings_ms": {k: {str(a): v for a, v in d.items()} for k, d in timings.items()},
