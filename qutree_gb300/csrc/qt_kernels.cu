@@ -2324,15 +2324,16 @@ cudaError_t launch_rho_inverse_static(const double2* rho, double2* rhoinv, int n
 //
 // A cluster of CTAs owns a node, each CTA a contiguous block of its rows (in
 // shared memory when they fit, else in place).  Step j is one pass over the
-// rows for all dot products with x = A[j:m, j] (columns k > j: to update
-// them; k < j: the Gram matrix of the reflectors), one exchange of the CTAs'
-// partial sums through distributed shared memory, and the update:
-//   w_k = v^H a_k = x^H a_k - conj(alpha) a_jk,   a_k -= tau v w_k,
-// where |x|^2 is the sum for k = j, and row j comes from its CTA.  Then
+// rows below j for all dot products with x = A[j+1:m, j] (columns k > j: to
+// update them; k < j: the Gram matrix of the reflectors), one exchange of the
+// CTAs' partial sums through distributed shared memory, and the update:
+//   w_k = v^H a_k = x^H a_k + conj(v_0) a_jk,   a_k -= tau v w_k,
+// where |x|^2 is the sum for k = j, and row j comes from its CTA; tau = 2 / |v|^2
+// of the v that is stored.  Then
 // Q = [I; 0] - V M with the compact form M = T V_top^H, (T^-1)_il = v_i^H v_l
 // for i < l and 1 / tau_i on the diagonal, solved by back substitution
-// (columns shared out over the CTAs), and one product per row.  No atomics,
-// fixed orders of addition.
+// (columns shared out over the CTAs), and one product per row, the identity
+// added last.  No atomics, fixed orders of addition.
 //
 // Bound: the FP64 pipe, 10 m n^2 DFMA over the cluster's SMs, and per step a
 // chain of about 3 us (sums, exchange, square root, divisions).  One block per
@@ -2374,14 +2375,14 @@ __global__ void __launch_bounds__(kThreads) k_house_qr(const QRTask* __restrict_
   __syncthreads();
   for (int j = 0; j < steps; ++j) {
     const int par = j & 1, lo = max(0, j - r0);  // first row of the block at or below row j
-    // partial x^H a_k over the block's rows >= j
+    // partial x^H a_k over the block's rows > j
     {
       const int k = tid % n, c = tid / n;
       double2 acc = cz();
       if (c < ch) {
         const double2* x = X + ld * j;
         const double2* a = X + ld * k;
-        for (int i = lo + c; i < nr; i += ch) cfmac(acc, x[i], a[i]);
+        for (int i = max(0, j + 1 - r0) + c; i < nr; i += ch) cfmac(acc, x[i], a[i]);
         red[tid] = acc;
       }
       for (int h = ch / 2; h > 0; h /= 2) {
@@ -2415,37 +2416,39 @@ __global__ void __launch_bounds__(kThreads) k_house_qr(const QRTask* __restrict_
         row = rowj[par * n + tid];
       }
     }
-    if (tid == j) red[kThreads - 1] = red[j];  // |x|^2 (the slot is free: n <= kHpMaxDim)
+    if (tid == j) red[kThreads - 1] = red[j];  // |x|^2 below x_0 (the slot is free: n <= kHpMaxDim)
     if (tid == j) tw[j] = row;                     // x_0
     __syncthreads();
     if (tid < 32) {  // the scalars, roots and divisions in separate lanes
-      const double nrm2 = red[kThreads - 1].x;
+      const double below = red[kThreads - 1].x;
       const double2 x0 = tw[j];
       const double a2 = x0.x * x0.x + x0.y * x0.y;
-      const double rt = sqrt(tid == 0 ? nrm2 : a2);
+      const double rt = sqrt(tid == 0 ? below + a2 : a2);
       const double nrm = __shfl_sync(0xffffffffu, rt, 0), ax0 = __shfl_sync(0xffffffffu, rt, 1);
-      const double den = nrm2 + ax0 * nrm;  // |v|^2 / 2
-      const double q = tid == 0 ? 1.0 / den : x0.x / ax0;
-      const double qy = x0.y / ax0;
-      if (tid == 0) s_tau[j] = den > 0.0 ? q : 0.0;
-      if (tid == 1) {
-        const double2 ph = ax0 > 0.0 ? make_double2(q, qy) : make_double2(1.0, 0.0);
-        s_alpha[j] = make_double2(-ph.x * nrm, -ph.y * nrm);
+      const double q = (tid == 0 ? x0.x : x0.y) / ax0;
+      double2 ph = make_double2(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
+      if (!(ax0 > 0.0)) ph = make_double2(1.0, 0.0);
+      const double2 al = make_double2(-ph.x * nrm, -ph.y * nrm);
+      const double2 v0 = make_double2(x0.x - al.x, x0.y - al.y);
+      const double vn2 = below + (v0.x * v0.x + v0.y * v0.y);
+      if (tid == 0) {
+        s_tau[j] = vn2 > 0.0 ? 2.0 / vn2 : 0.0;
+        s_alpha[j] = al;
       }
     }
     __syncthreads();
     const double tau = s_tau[j];
-    const double2 al = s_alpha[j];
+    const double2 al = s_alpha[j], x0 = tw[j];
+    const double2 v0 = make_double2(x0.x - al.x, x0.y - al.y);
     if (tid < n && tid != j) {
-      double2 w = red[tid];  // - conj(alpha) a_jk
-      w.x = fma(-al.x, row.x, fma(-al.y, row.y, w.x));
-      w.y = fma(-al.x, row.y, fma(al.y, row.x, w.y));
+      double2 w = red[tid];
+      cfmac(w, v0, row);
       if (tid > j)
         tw[tid] = make_double2(tau * w.x, tau * w.y);
       else if (rank == 0)
         t.R[j + (int64_t)n * tid] = make_double2(w.x, -w.y);  // v_k^H v_j, parked below R's diagonal
     }
-    if (j >= r0 && j < r0 + nr && tid == j) X[(j - r0) + ld * j] = make_double2(row.x - al.x, row.y - al.y);
+    if (j >= r0 && j < r0 + nr && tid == j) X[(j - r0) + ld * j] = v0;
     __syncthreads();
     const int nk = n - 1 - j;
     if (nk > 0) {
@@ -2521,13 +2524,14 @@ __global__ void __launch_bounds__(kThreads) k_house_qr(const QRTask* __restrict_
     }
     for (int e = tid; e < nb * n; e += kThreads) {
       const int i = e % nb, k = e / nb, row = r0 + b0 + i;
-      double2 acc = make_double2(row == k ? 1.0 : 0.0, 0.0);
+      double2 acc = cz();
       const int last = min(row, steps - 1);  // v_l is zero above row l
 #pragma unroll 4
       for (int l = 0; l <= last; ++l) {
         const double2 x = v[i + lv * l];
         cfma(acc, make_double2(-x.x, -x.y), t.Qs[l + (int64_t)steps * k]);
       }
+      if (row == k) acc.x += 1.0;
       t.A[row + (int64_t)m * k] = acc;
     }
     __syncthreads();
