@@ -110,3 +110,39 @@ def test_density_inverse_between_the_certificates(d, low, rest):
         ctx.close()
     cond = lam[-1] / lam[0]
     assert rel_err(got, want) <= 8 * d * cond * 2.0 ** -53 + 64 * 2.0 ** -53 * cond
+
+
+@pytest.mark.parametrize("decades", [2, 3, 4])
+@pytest.mark.parametrize("prec,unit", [(qtgpu.QT_PREC_F64, 2.0 ** -53), (qtgpu.QT_PREC_DF64, 2.0 ** -47)])
+def test_projector_of_nearly_dependent_columns(decades, prec, unit):
+    """Node tensors whose columns span `decades` orders of magnitude in all
+    directions: cond(S) is the square.  The bound is that of the inverse
+    alone, 8 d cond(S) units."""
+    tree = balanced_tree(4, 40, 17)
+    sop = coupled_oscillators(tree, n_pairs=None, coupling=0.2, quartic=0.1, rng=np.random.default_rng(1), omega=1.0)
+    psi = random_wavefunction(tree, 3)
+    rng = np.random.default_rng(4)
+    tensors = []
+    for n, t in zip(tree.nodes, psi.tensors):
+        d = n.d_up
+        a, b = (np.linalg.qr(rng.standard_normal((d, d)) + 1j * rng.standard_normal((d, d)))[0] for _ in range(2))
+        g = (a * 10.0 ** (-decades * np.arange(d) / max(1, d - 1))) @ b
+        tensors.append(t if n.is_top else np.asfortranarray(np.tensordot(t, g, axes=([-1], [0]))))
+    flat = TensorTree(tree, tensors).flat()
+    ref = O.derivative(tree, sop, flat)
+    h = qtgpu.HamiltonianRepresentation(sop, tree, flavour=qtgpu.QT_PLAN_COMPRESSED | prec)
+    try:
+        got = qtgpu.Derivative(h, flat)
+    finally:
+        h.close()
+    off, ro = tree.offsets(), 0
+    num = den = 0.0
+    for n in tree.nodes:  # weighted back by rho, as in the other sweep tests
+        d = n.d_up
+        r = ref.rho[ro:ro + d * d].reshape((d, d), order="F")
+        ro += d * d
+        a, b = (x[off[n.address]:off[n.address + 1]].reshape((-1, d), order="F") for x in (got, ref.dpsi))
+        if not n.is_top:
+            a, b = a @ r.T, b @ r.T
+        num, den = max(num, np.abs(a - b).max()), max(den, np.abs(b).max())
+    assert num <= 8 * 17 * 10.0 ** (2 * decades) * unit * den

@@ -20,3 +20,12 @@ def test_lanczos_edges(leaf, bond, n_krylov, prec, tol):
     tree = balanced_tree(4, leaf, bond)
     sop = coupled_oscillators(tree, n_pairs=None, coupling=0.2, quartic=0.1, rng=np.random.default_rng(2), omega=1.0)
     _check(tree, sop, random_wavefunction(tree, 2), tol=tol, prec=prec, n_iter=1, n_krylov=n_krylov)
+
+
+@pytest.mark.parametrize("prec,tol", [(qtgpu.QT_PREC_F64, 1e-11), (qtgpu.QT_PREC_DF64, 1e-10)])
+def test_lanczos_more_slices_than_ctas(prec, tol):
+    """Inner nodes of 74088 elements: ten slices on a cluster of eight CTAs, two
+    of which own two."""
+    tree = balanced_tree(4, 43, 42)
+    sop = coupled_oscillators(tree, n_pairs=None, coupling=0.2, quartic=0.1, rng=np.random.default_rng(2), omega=1.0)
+    _check(tree, sop, random_wavefunction(tree, 2), tol=tol, prec=prec, n_iter=1, n_krylov=2)
