@@ -658,7 +658,7 @@ class Builder {
   // wide tensor-core tasks before it exceed their share of the scratch budget
   // (at least t0 + 1; t1: all fit)
   int64_t memory_cut(int kind, int64_t t0, int64_t t1) const {
-    if (kind != ST_MP && kind != ST_HP && kind != ST_ACC) return t1;
+    if (!P.hp_tensor || !wide || (kind != ST_MP && kind != ST_HP && kind != ST_ACC)) return t1;
     const int64_t limit = budget * 16 / kTcWideShare;
     std::set<std::tuple<int, int64_t, int, int, int>> images;  // hole products share A's
     int64_t used = 0;
@@ -688,6 +688,7 @@ class Builder {
     if (t1 <= t0) return;
     const double flops = P.stats.exec_flops - stage_flops_mark, bytes = stage_bytes(kind, t0, t1);
     stage_flops_mark = P.stats.exec_flops;
+    const int64_t first = t0;
     while (t0 < t1) {
       const int64_t cut = memory_cut(kind, t0, t1);
       int64_t mid = tile1;
@@ -699,7 +700,7 @@ class Builder {
         };
         mid = kind == ST_MP ? first_of(P.mp_tiles) : first_of(P.acc_tiles);
       }
-      const double part = stage_bytes(kind, t0, cut);
+      const double part = t0 == first && cut == t1 ? bytes : stage_bytes(kind, t0, cut);
       emit_one(kind, t0, cut, tile0, mid, name, part == bytes ? flops : flops * (part / bytes), part);
       t0 = cut;
       tile0 = kind == ST_HP ? (int64_t)P.hp_tiles.size() : mid;
