@@ -432,17 +432,22 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_mp_tf(const MPTask* __restric
 
 // ---------------------------------------------------------------------------
 // Sums of products on the tensor cores (double-float plans): the hole
-// products and the last-index accumulations.  Both compute, per output row
-// m and column n,
+// products, the last-index accumulations and the mode products.  All compute,
+// per output row m and column n,
 //   D(m, n) = sum over units u of  sum_k X_u(m, k) W_u(n, k)     (complex)
-// in units of at most 64 k, every unit with its own power-of-two scales per
+// in units of at most 128 k, every unit with its own power-of-two scales per
 // row of X_u (E_m) and per row of W_u (F_n):
 //  * hole products S_t(i, j) = sum_k conj(A[k; i]) B_t[k; j]: the rows m are
 //    the (task t, j) of a group of tasks that share A (X = B_t), n = i and
-//    W = conj(A); the units are the 64-k chunks of the reduction;
+//    W = conj(A); the units are the chunks of the reduction, 64 k up to 32
+//    columns, else 128;
 //  * accumulations out[r, j] (+)= alpha sum_t sum_j' H_t(j, j') X_t[r, j']:
 //    rows m = r (a block of 128), n = j, one unit per term t with X = X_t
-//    and W = alpha H_t (alpha I for identity terms).
+//    and W = alpha H_t (alpha I for identity terms), up to 112 k;
+//  * mode products C[b, j, c] = alpha sum_a h(j, a) B[b, a, c]: rows m = (b, c)
+//    (a block of 128), n = j, one unit of up to 112 k.
+// Beyond 64 columns an item is one column block (tc_blocks), and 48-column
+// blocks take a unit in two halves (tcs_halve).
 // The accumulator tile has 2 np columns, the real parts for n < np and the
 // imaginary parts after them, so
 //   Re D = Xr Wr - Xi Wi,   Im D = Xr Wi + Xi Wr
@@ -450,12 +455,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_mp_tf(const MPTask* __restric
 // Xi x [-Wi | Wr].  W's image, written by a pre-pass per unit, stores the
 // rows [-Wi | Wr | Wi] (np each) once per 16-k step and digit; the two
 // operands are its rows np.. and 0.. .  The producers cut X's digits; the
-// image steps arrive by bulk copies on the same barrier.  A unit's level
-// sums are exact in fp32 (at most 7 pairs x 2 x 64 products of |digit
-// products| <= 2^14 units per level); the epilogue recombines them in
-// double-float, scales by 2^(E_m + F_n) and adds them to the output in
-// double-float (a work item's first unit stores, or adds to the old output
-// where the accumulation asks for it).
+// image steps arrive by bulk copies on the same barrier.  A level's sum is
+// exact in fp32 where it has an accumulator of its own: digit 0 is at most
+// 128 units, 1 and 2 at most 64, 3 at most 80, the others 128, so that 2 x 128
+// products per pair stay below 2^24 units in levels 0..4, and 2 x 112 in 5 and
+// 6.  With fewer than seven accumulators (levels_for; four for 128-k chunks up
+// to 64 columns) the last one takes the remaining levels and is rounded.  The
+// epilogue recombines the levels in double-float, scales by 2^(E_m + F_n) and
+// adds them to the output in double-float (a work item's first unit stores, or
+// adds to the old output where the accumulation asks for it).
 // ---------------------------------------------------------------------------
 constexpr int kTcsNStage = kDig * 3 * 64 * 32;  // W side of one 16-k step at np = 64
 
@@ -483,7 +491,7 @@ struct TcsArgs {
   const MPTask* mp;          // mode products: tasks, tiles (task, 128-row block) and the pre-pass's tasks
   const int2* mp_tiles;
   const int* mp_tasks;
-  const int4* items;         // HP (group, range z, first chunk, end chunk); ACC (task, block, units before, 0)
+  const int4* items;         // HP (group, range z, first chunk, end chunk); ACC (task, block, units before, column block)
   int64_t item0, n_items;
   int64_t units;             // ACC: units of all items (weighted split over the CTAs)
   int* status;
